@@ -29,6 +29,16 @@ namespace {
 // ---------------------------------------------------------------------------------------
 // (a) projection
 // ---------------------------------------------------------------------------------------
+// A block's camera in shared memory, by arithmetic.
+template <int MODE>
+struct CameraOf {
+    using type = RpcFast;
+};
+template <>
+struct CameraOf<VS_PROJ_EXACT> {
+    using type = RpcExact;
+};
+
 template <int MODE>
 __global__ void __launch_bounds__(256) rpc_project_kernel(const VsRpcCamera *__restrict__ cams,
                                                           const double *__restrict__ lat,
@@ -37,33 +47,27 @@ __global__ void __launch_bounds__(256) rpc_project_kernel(const VsRpcCamera *__r
                                                           long long stride, double *__restrict__ col,
                                                           double *__restrict__ row,
                                                           uint8_t *__restrict__ keep) {
-    __shared__ VsRpcCamera cam;
-    __shared__ RpcFast fast;
+    constexpr bool kExact = MODE == VS_PROJ_EXACT;
+    __shared__ typename CameraOf<MODE>::type cam;
     const int c = blockIdx.y;
-    {
-        const double *src = reinterpret_cast<const double *>(cams + c);
-        double *dst = reinterpret_cast<double *>(&cam);
-        for (int i = threadIdx.x; i < static_cast<int>(sizeof(VsRpcCamera) / 8); i += blockDim.x) dst[i] = src[i];
-    }
-    __syncthreads();
-    if (MODE == VS_PROJ_FAST && threadIdx.x == 0) prepare_fast(cam, fast);
-    __syncthreads();
+    if constexpr (kExact) load_exact(cams + c, cam);
+    else prepare_fast(cams[c], cam);
     const double *la = lat + c * stride, *lo = lon + c * stride, *al = alt + c * stride;
     double *oc = col + c * n, *orow = row + c * n;
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
          i += static_cast<long long>(gridDim.x) * blockDim.x) {
         double cc, rr;
         bool k;
-        if (MODE == VS_PROJ_EXACT) {
+        if constexpr (kExact) {
             project_exact(cam, __ldcs(la + i), __ldcs(lo + i), __ldcs(al + i), cc, rr);
-            k = cc >= 0.0 && rr >= 0.0 && cc < cam.width && rr < cam.height;
+            k = cc >= 0.0 && rr >= 0.0 && cc < cam.cam.width && rr < cam.cam.height;
         } else {
             df dc, dr;
-            project_fast(fast, split_double(__ldcs(la + i)), split_double(__ldcs(lo + i)),
+            project_fast(cam, split_double(__ldcs(la + i)), split_double(__ldcs(lo + i)),
                          split_double(__ldcs(al + i)), dc, dr);
             cc = df_to_double(dc);
             rr = df_to_double(dr);
-            k = df_ge0(dc) && df_ge0(dr) && df_lt(dc, fast.width) && df_lt(dr, fast.height);
+            k = df_ge0(dc) && df_ge0(dr) && df_lt(dc, cam.width) && df_lt(dr, cam.height);
         }
         __stcs(oc + i, cc);
         __stcs(orow + i, rr);
@@ -329,17 +333,16 @@ __global__ void __launch_bounds__(kMomThreads, 6) moments_kernel(
     store_block_moments(m, count, partial + (static_cast<long long>(v) * gridDim.x + blockIdx.x) * kSlots, red);
 }
 
-// Double-float form of every view's camera, prepared once per call (one thread per view)
-// rather than by the first thread of every projection block.
-__global__ void prepare_views_kernel(const VsRpcCamera *__restrict__ cams, int n_views, RpcFast *__restrict__ fast,
-                                     float *__restrict__ wh) {
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= n_views) return;
-    RpcFast f;
-    prepare_fast(cams[v], f);
-    fast[v] = f;
-    wh[2 * v] = f.width;
-    wh[2 * v + 1] = f.height;
+// Double-float form of every view's camera, prepared once per call (one block per view)
+// rather than by every projection block.
+__global__ void __launch_bounds__(64) prepare_views_kernel(const VsRpcCamera *__restrict__ cams,
+                                                           RpcFast *__restrict__ fast, float *__restrict__ wh) {
+    const int v = blockIdx.x;
+    prepare_fast(cams[v], fast[v]);
+    if (threadIdx.x == 0) {
+        wh[2 * v] = fast[v].width;
+        wh[2 * v + 1] = fast[v].height;
+    }
 }
 
 // Projection pass of the fused camera path: (col, row) of every grid point through view
@@ -351,18 +354,17 @@ __global__ void __launch_bounds__(256) project_view_kernel(const VsRpcCamera *__
                                                            const double *__restrict__ lon,
                                                            const double *__restrict__ alt, long long n,
                                                            long long stride, float4 *__restrict__ colrow) {
-    __shared__ VsRpcCamera cam;
-    __shared__ RpcFast fast;
+    constexpr bool kExact = MODE == VS_PROJ_EXACT;
+    __shared__ typename CameraOf<MODE>::type cam;
     const int v = blockIdx.y;
-    {
-        const unsigned *src = MODE == VS_PROJ_EXACT ? reinterpret_cast<const unsigned *>(cams + v)
-                                                    : reinterpret_cast<const unsigned *>(fasts + v);
-        unsigned *dst = MODE == VS_PROJ_EXACT ? reinterpret_cast<unsigned *>(&cam) : reinterpret_cast<unsigned *>(&fast);
-        const int words = MODE == VS_PROJ_EXACT ? static_cast<int>(sizeof(VsRpcCamera) / 4)
-                                                : static_cast<int>(sizeof(RpcFast) / 4);
-        for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
+    if constexpr (kExact) {
+        load_exact(cams + v, cam);
+    } else {
+        const unsigned *src = reinterpret_cast<const unsigned *>(fasts + v);
+        unsigned *dst = reinterpret_cast<unsigned *>(&cam);
+        for (int i = threadIdx.x; i < static_cast<int>(sizeof(RpcFast) / 4); i += blockDim.x) dst[i] = src[i];
+        __syncthreads();
     }
-    __syncthreads();
     const long long off = v * stride;
     const long long step = static_cast<long long>(gridDim.x) * blockDim.x;
     // the next point's coordinates (raw 64-bit patterns) are loaded before the current
@@ -385,13 +387,13 @@ __global__ void __launch_bounds__(256) project_view_kernel(const VsRpcCamera *__
             b2 = __ldcs(al + i + step);
         }
         df dc, dr;
-        if (MODE == VS_PROJ_EXACT) {
+        if constexpr (kExact) {
             double cc, rr;
             project_exact(cam, __longlong_as_double(a0), __longlong_as_double(a1), __longlong_as_double(a2), cc, rr);
             dc = split_double(cc);
             dr = split_double(rr);
         } else {
-            project_fast(fast, split_double(__longlong_as_double(a0)), split_double(__longlong_as_double(a1)),
+            project_fast(cam, split_double(__longlong_as_double(a0)), split_double(__longlong_as_double(a1)),
                          split_double(__longlong_as_double(a2)), dc, dr);
         }
         colrow[static_cast<long long>(v) * n + i] = make_float4(dc.hi, dc.lo, dr.hi, dr.lo);
@@ -1126,10 +1128,16 @@ extern "C" int vs_rpc_project(const VsRpcCamera *cams, int n_cams, const double 
     VS_REQUIRE(mode == VS_PROJ_EXACT || mode == VS_PROJ_FAST, "vs_rpc_project: bad mode %d", mode);
     if (n == 0) return VS_OK;
     VS_REQUIRE(cams && lat && lon && alt && col && row, "vs_rpc_project: null pointer");
-    const int threads = 256;
-    long long want = ceil_div(n, threads);
-    unsigned gx = static_cast<unsigned>(std::min<long long>(want, std::max(1LL, sm_count() * 8LL / n_cams + 1)));
-    dim3 grid(gx, n_cams);
+    // The exact form is bound by each SM's FP64 pipe, so few points are spread over all SMs:
+    // 1999 points in blocks of 256 took 26 us on 8 SMs, in blocks of 32 on 63 SMs 14 us.
+    const int sms = sm_count();
+    const long long points = n * n_cams;
+    const int threads = points >= 512LL * sms ? 256 : (points >= 128LL * sms ? 64 : 32);
+    const long long want = ceil_div(n, threads);
+    const long long cap = std::max(1LL, sms * (2048LL / threads) / n_cams + 1);
+    // even shares: every thread of a full grid takes as many points as any other, +-1
+    const long long rounds = ceil_div(want, cap);
+    const dim3 grid(static_cast<unsigned>(ceil_div(want, rounds)), n_cams);
     cudaStream_t st = as_stream(stream);
     if (mode == VS_PROJ_EXACT)
         rpc_project_kernel<VS_PROJ_EXACT><<<grid, threads, 0, st>>>(cams, lat, lon, alt, n, point_stride, col, row, keep);
@@ -1237,7 +1245,7 @@ extern "C" int vs_camera_approx_perspective(const VsRpcCamera *cams, int n_views
     int s = launch_norm(x, y, z, point_stride, nullptr, nullptr, nullptr, cams, n_views, n, f, st);
     if (s != VS_OK) return s;
     const int blocks = mom_blocks(n);
-    prepare_views_kernel<<<static_cast<unsigned>(ceil_div(n_views, 64)), 64, 0, st>>>(cams, n_views, f.fast, f.wh);
+    prepare_views_kernel<<<n_views, 64, 0, st>>>(cams, f.fast, f.wh);
     VS_LAUNCH_CHECK("prepare_views_kernel");
     if (n > 0) {
         const unsigned pg = static_cast<unsigned>(std::min<long long>(ceil_div(n, 256), sm_count() * 8LL / n_views + 8));
