@@ -4,11 +4,18 @@
 // normalised frame) it projects the point and two finite-difference neighbours (steps 2,
 // then 0.1), moves lon/lat by the projections of the image residual on the two difference
 // vectors, and stops when EVERY point reprojects within sqrt(1e-18) of its target.  A
-// point's result therefore depends on its camera's global iteration count, so the device
-// keeps each point's state in the workspace and the host runs the per-camera global loop:
-// one update launch per iteration for the cameras still running, each block counting its
-// unconverged points.  Every FP64 operation is the reference's (no contraction into FMA),
-// so the results are bit-identical.
+// point's result therefore depends on its camera's global iteration count.  Every FP64
+// operation is the reference's (no contraction into FMA), so the results are bit-identical.
+//
+// The global count is found without a host round trip per iteration.  It is at least the
+// largest over the points of the first iteration at which that point has converged, so
+//   1. inverse_first_kernel iterates each warp's points, in registers, until every one of them has
+//      converged once, keeps their state and posts that iteration (a maximum per camera);
+//   2. inverse_advance_kernel takes every point on to the posted maximum, writes the results
+//      and counts the points that have left convergence again.
+// No such point: done, with one host synchronisation.  Otherwise the camera goes on one iteration at
+// a time (inverse_advance_kernel, target + 1).  Every point runs each iteration once either way.
+#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
@@ -17,27 +24,93 @@
 namespace vs {
 namespace {
 
-constexpr int kInvThreads = 256;
+// The kernels are bound by the FP64 pipe (19 sums and a share of the quotients per polynomial),
+// which every SM has its own of: small blocks spread the points evenly over the SMs (90,001
+// points: blocks of 64 hold every SM to within 8% of the mean load, blocks of 256 to 30%), and
+// registers for 12 of them on an SM (90,001 points, 7 iterations: 511 us; for 8 or fewer
+// 600 us, for 16 520 us).  The whole call took 1088 us with the products on the FP64 pipe and a
+// host synchronisation per iteration, 485 us now.
+constexpr int kInvThreads = 64;
 constexpr int kStateFields = 11;   // lon lat x0 y0 x1 y1 x2 y2 c_col c_row c_alt
 
 struct InvState {
     double *f[kStateFields];
+    int *k;                        // iterations done
 };
 
-__device__ __forceinline__ double rfm(const double *num, const double *den, double lat, double lon, double alt) {
-    return __ddiv_rn(poly_exact(num, lat, lon, alt), poly_exact(den, lat, lon, alt));
+// The three projections of an iteration share the products of the coordinates they share (the
+// same values: the compiler computes each once), 364 of 540 per iteration.
+struct Factor3 {
+    Factor a, b, c;
+};
+struct Prod3 {
+    Prod a, b, c;
+};
+struct Double3 {
+    double a, b, c;
+};
+__device__ __forceinline__ Prod3 operator*(const RpcCoef &k, const Factor3 &f) { return {k * f.a, k * f.b, k * f.c}; }
+__device__ __forceinline__ Prod3 operator*(const Prod3 &p, const Factor3 &f) {
+    return {p.a * f.a, p.b * f.b, p.c * f.c};
+}
+__device__ __forceinline__ Double3 value(const Prod3 &p) { return {value(p.a), value(p.b), value(p.c)}; }
+__device__ __forceinline__ Double3 sum(const Double3 &p, const Double3 &q) {
+    return {da(p.a, q.a), da(p.b, q.b), da(p.c, q.c)};
+}
+
+// poly_factors at three points.
+__device__ __forceinline__ Double3 poly_factors3(const RpcCoef *c, const Factor3 &x, const Factor3 &y,
+                                                 const Factor3 &z) {
+    const double c0 = value(c[0]);
+    Double3 out{c0, c0, c0};
+    out = sum(out, sum(sum(value(c[1] * y), value(c[2] * x)), value(c[3] * z)));
+    out = sum(out, sum(sum(value(c[4] * y * x), value(c[5] * y * z)), value(c[6] * x * z)));
+    out = sum(out, sum(sum(value(c[7] * y * y), value(c[8] * x * x)), value(c[9] * z * z)));
+    out = sum(out, value(c[10] * x * y * z));
+    out = sum(out, value(c[11] * y * y * y));
+    out = sum(out, sum(sum(value(c[12] * y * x * x), value(c[13] * y * z * z)),
+                     value(c[14] * y * y * x)));
+    out = sum(out, value(c[15] * x * x * x));
+    out = sum(out, sum(sum(value(c[16] * x * z * z), value(c[17] * y * y * z)),
+                     value(c[18] * x * x * z)));
+    out = sum(out, value(c[19] * z * z * z));
+    return out;
+}
+
+__device__ __forceinline__ Double3 poly3(const RpcExact &s, int q, bool fast, const Factor3 &fx, const Factor3 &fy,
+                                         const Factor3 &fz, const Double3 &x, const Double3 &y, double z) {
+    if (fast) return poly_factors3(s.coef + 20 * q, fx, fy, fz);
+    const double *c = s.cam.row_num + 20 * q;      // the camera's polynomials follow one another
+    return {poly_exact(c, x.a, y.a, z), poly_exact(c, x.b, y.b, z), poly_exact(c, x.c, y.c, z)};
 }
 
 // the reference's three projections: at (lat, lon), (lat, lon + eps), (lat + eps, lon)
-__device__ __forceinline__ void frames(const VsRpcCamera &c, double lat, double lon, double alt, double eps,
+__device__ __forceinline__ void frames(const RpcExact &s, double lat, double lon, double alt, double eps,
                                        double (&o)[6]) {
     const double lon_e = __dadd_rn(lon, eps), lat_e = __dadd_rn(lat, eps);
-    o[0] = rfm(c.col_num, c.col_den, lat, lon, alt);
-    o[1] = rfm(c.row_num, c.row_den, lat, lon, alt);
-    o[2] = rfm(c.col_num, c.col_den, lat, lon_e, alt);
-    o[3] = rfm(c.row_num, c.row_den, lat, lon_e, alt);
-    o[4] = rfm(c.col_num, c.col_den, lat_e, lon, alt);
-    o[5] = rfm(c.row_num, c.row_den, lat_e, lon, alt);
+    const Double3 x{lat, lat, lat_e}, y{lon, lon_e, lon};
+    const bool fast = s.moderate && moderate(lat) && moderate(lat_e) && moderate(lon) && moderate(lon_e) && moderate(alt);
+    const Factor3 fx{factor_of(lat), factor_of(lat), factor_of(lat_e)}, fy{factor_of(lon), factor_of(lon_e), factor_of(lon)};
+    const Factor3 fz{factor_of(alt), factor_of(alt), factor_of(alt)};
+#pragma unroll 1
+    for (int axis = 0; axis < 2; ++axis) {         // rows, then columns
+        Double3 num{0.0, 0.0, 0.0}, den{0.0, 0.0, 0.0};
+#pragma unroll 1
+        for (int d = 0; d < 2; ++d) {
+            num = den;
+            den = poly3(s, 2 * axis + d, fast, fx, fy, fz, x, y, alt);
+        }
+        const double q0 = __ddiv_rn(num.a, den.a), q1 = __ddiv_rn(num.b, den.b), q2 = __ddiv_rn(num.c, den.c);
+        if (axis == 0) {
+            o[1] = q0;
+            o[3] = q1;
+            o[5] = q2;
+        } else {
+            o[0] = q0;
+            o[2] = q1;
+            o[4] = q2;
+        }
+    }
 }
 
 // (x0 - c_col)^2 + (y0 - c_row)^2 < 1e-18 (false for NaN)
@@ -46,106 +119,121 @@ __device__ __forceinline__ bool converged(double x0, double y0, double cc, doubl
     return __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)) < 1e-18;
 }
 
-__device__ __forceinline__ void count_block(bool unconverged, int *count) {
-    __shared__ int s;
-    if (threadIdx.x == 0) s = 0;
-    __syncthreads();
-    const unsigned b = __ballot_sync(0xffffffffu, unconverged);
-    if ((threadIdx.x & 31) == 0 && b) atomicAdd(&s, __popc(b));
-    __syncthreads();
-    if (threadIdx.x == 0 && s) atomicAdd(count, s);
+// One point: its position, projections and target in the normalised frame.
+struct InvPoint {
+    double lon, lat, o[6], cc, cr, ca;
+};
+
+// Iteration k (0-based) of one point.
+__device__ __forceinline__ void inverse_iteration(const RpcExact &s, int k, InvPoint &p) {
+    const double e1x = __dsub_rn(p.o[2], p.o[0]), e1y = __dsub_rn(p.o[3], p.o[1]);
+    const double e2x = __dsub_rn(p.o[4], p.o[0]), e2y = __dsub_rn(p.o[5], p.o[1]);
+    const double ux = __dsub_rn(p.cc, p.o[0]), uy = __dsub_rn(p.cr, p.o[1]);
+    const double a1 = __ddiv_rn(__dadd_rn(__dmul_rn(ux, e1x), __dmul_rn(uy, e1y)),
+                                __dadd_rn(__dmul_rn(e1x, e1x), __dmul_rn(e1y, e1y)));
+    const double a2 = __ddiv_rn(__dadd_rn(__dmul_rn(ux, e2x), __dmul_rn(uy, e2y)),
+                                __dadd_rn(__dmul_rn(e2x, e2x), __dmul_rn(e2y, e2y)));
+    const double eps = k == 0 ? 2.0 : 0.1;
+    p.lon = __dadd_rn(p.lon, __dmul_rn(a1, eps));
+    p.lat = __dadd_rn(p.lat, __dmul_rn(a2, eps));
+    frames(s, p.lat, p.lon, p.ca, 0.1, p.o);
 }
 
-// grid (points, cameras)
-__global__ void __launch_bounds__(kInvThreads) inverse_init_kernel(
+__device__ __forceinline__ void save_point(const InvState &st, long long s, const InvPoint &p, int k) {
+    st.f[0][s] = p.lon;
+    st.f[1][s] = p.lat;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) st.f[2 + q][s] = p.o[q];
+    st.f[8][s] = p.cc;
+    st.f[9][s] = p.cr;
+    st.f[10][s] = p.ca;
+    st.k[s] = k;
+}
+
+// grid (points, cameras).  target[c]: the largest posted iteration; failed[c]: a point of the
+// camera has not converged within max_iter iterations.
+__global__ void __launch_bounds__(kInvThreads, 12) inverse_first_kernel(
     const VsRpcCamera *__restrict__ cams, const double *__restrict__ col, const double *__restrict__ row,
-    const double *__restrict__ alt, long long n, long long stride, InvState st, int *__restrict__ count) {
+    const double *__restrict__ alt, long long n, long long stride, int max_iter, InvState st, int *__restrict__ target,
+    int *__restrict__ failed) {
+    __shared__ RpcExact cam;
     const int c = blockIdx.y;
+    load_exact(cams + c, cam);
     const long long i = blockIdx.x * static_cast<long long>(kInvThreads) + threadIdx.x;
-    bool unc = false;
-    if (i < n) {
-        const VsRpcCamera &cam = cams[c];
-        const long long p = c * stride + i, s = c * n + i;
-        const double cc = __ddiv_rn(__dsub_rn(col[p], cam.col_off), cam.col_scale);
-        const double cr = __ddiv_rn(__dsub_rn(row[p], cam.row_off), cam.row_scale);
-        const double ca = __ddiv_rn(__dsub_rn(alt[p], cam.alt_off), cam.alt_scale);
-        double o[6];
-        frames(cam, -1.0, -1.0, ca, 2.0, o);
-        st.f[0][s] = -1.0;
-        st.f[1][s] = -1.0;
-#pragma unroll
-        for (int k = 0; k < 6; ++k) st.f[2 + k][s] = o[k];
-        st.f[8][s] = cc;
-        st.f[9][s] = cr;
-        st.f[10][s] = ca;
-        unc = !converged(o[0], o[1], cc, cr);
+    const bool in = i < n;
+    InvPoint p;
+    {
+        const long long g = c * stride + (in ? i : n - 1);      // idle lanes follow the last point
+        p.cc = __ddiv_rn(__dsub_rn(col[g], cam.cam.col_off), cam.cam.col_scale);
+        p.cr = __ddiv_rn(__dsub_rn(row[g], cam.cam.row_off), cam.cam.row_scale);
+        p.ca = __ddiv_rn(__dsub_rn(alt[g], cam.cam.alt_off), cam.cam.alt_scale);
     }
-    count_block(unc, count + c);
+    p.lon = p.lat = -1.0;
+    frames(cam, -1.0, -1.0, p.ca, 2.0, p.o);
+    bool done = converged(p.o[0], p.o[1], p.cc, p.cr);
+    int k = 0;
+    while (k < max_iter && !__all_sync(0xffffffffu, done)) {
+        inverse_iteration(cam, k, p);
+        ++k;
+        done |= converged(p.o[0], p.o[1], p.cc, p.cr);
+    }
+    if (in) save_point(st, c * n + i, p, k);
+    if ((threadIdx.x & 31) == 0) atomicMax(target + c, k);
+    if (!done) atomicOr(failed + c, 1);
 }
 
-// One global iteration for the cameras with iter[c] >= 0 (iter[c] = iterations done).
-__global__ void __launch_bounds__(kInvThreads) inverse_step_kernel(const VsRpcCamera *__restrict__ cams,
-                                                                   const int *__restrict__ iter, long long n,
-                                                                   InvState st, int *__restrict__ count) {
+// Takes the points of the cameras with run[c] != 0 on to iteration target[c], writes their
+// results and counts those that do not reproject within the bound there.
+__global__ void __launch_bounds__(kInvThreads, 12) inverse_advance_kernel(
+    const VsRpcCamera *__restrict__ cams, const double *__restrict__ alt, long long n, long long stride, int normalized,
+    InvState st, const int *__restrict__ target, const int *__restrict__ run, double *__restrict__ lon_out,
+    double *__restrict__ lat_out, double *__restrict__ alt_out, int *__restrict__ count) {
+    __shared__ RpcExact cam;
     const int c = blockIdx.y;
-    const int k = iter[c];
-    if (k < 0) return;
+    if (run && !run[c]) return;
+    load_exact(cams + c, cam);
+    const int to = target[c];
     const long long i = blockIdx.x * static_cast<long long>(kInvThreads) + threadIdx.x;
-    bool unc = false;
+    bool unconverged = false;
     if (i < n) {
-        const VsRpcCamera &cam = cams[c];
         const long long s = c * n + i;
-        double lon = st.f[0][s], lat = st.f[1][s];
-        const double x0 = st.f[2][s], y0 = st.f[3][s], x1 = st.f[4][s], y1 = st.f[5][s], x2 = st.f[6][s],
-                     y2 = st.f[7][s];
-        const double cc = st.f[8][s], cr = st.f[9][s], ca = st.f[10][s];
-        const double e1x = __dsub_rn(x1, x0), e1y = __dsub_rn(y1, y0);
-        const double e2x = __dsub_rn(x2, x0), e2y = __dsub_rn(y2, y0);
-        const double ux = __dsub_rn(cc, x0), uy = __dsub_rn(cr, y0);
-        const double a1 = __ddiv_rn(__dadd_rn(__dmul_rn(ux, e1x), __dmul_rn(uy, e1y)),
-                                    __dadd_rn(__dmul_rn(e1x, e1x), __dmul_rn(e1y, e1y)));
-        const double a2 = __ddiv_rn(__dadd_rn(__dmul_rn(ux, e2x), __dmul_rn(uy, e2y)),
-                                    __dadd_rn(__dmul_rn(e2x, e2x), __dmul_rn(e2y, e2y)));
-        const double eps = k == 0 ? 2.0 : 0.1;
-        lon = __dadd_rn(lon, __dmul_rn(a1, eps));
-        lat = __dadd_rn(lat, __dmul_rn(a2, eps));
-        double o[6];
-        frames(cam, lat, lon, ca, 0.1, o);
-        st.f[0][s] = lon;
-        st.f[1][s] = lat;
+        InvPoint p;
+        p.lon = st.f[0][s];
+        p.lat = st.f[1][s];
 #pragma unroll
-        for (int q = 0; q < 6; ++q) st.f[2 + q][s] = o[q];
-        unc = !converged(o[0], o[1], cc, cr);
+        for (int q = 0; q < 6; ++q) p.o[q] = st.f[2 + q][s];
+        p.cc = st.f[8][s];
+        p.cr = st.f[9][s];
+        p.ca = st.f[10][s];
+        const int from = st.k[s];
+        for (int k = from; k < to; ++k) inverse_iteration(cam, k, p);
+        if (from < to) save_point(st, s, p, to);
+        unconverged = !converged(p.o[0], p.o[1], p.cc, p.cr);
+        if (normalized) {
+            lon_out[s] = p.lon;
+            lat_out[s] = p.lat;
+            if (alt_out) alt_out[s] = p.ca;
+        } else {
+            lon_out[s] = __dadd_rn(__dmul_rn(p.lon, cam.cam.lon_scale), cam.cam.lon_off);
+            lat_out[s] = __dadd_rn(__dmul_rn(p.lat, cam.cam.lat_scale), cam.cam.lat_off);
+            if (alt_out) alt_out[s] = alt[c * stride + i];
+        }
     }
-    count_block(unc, count + c);
+    const unsigned b = __ballot_sync(0xffffffffu, unconverged);
+    if ((threadIdx.x & 31) == 0 && b) atomicAdd(count + c, __popc(b));
 }
 
-__global__ void inverse_final_kernel(const VsRpcCamera *__restrict__ cams, const double *__restrict__ alt,
-                                     long long n, long long stride, int normalized, InvState st,
-                                     double *__restrict__ lon_out, double *__restrict__ lat_out,
-                                     double *__restrict__ alt_out) {
-    const int c = blockIdx.y;
-    const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-    if (i >= n) return;
-    const VsRpcCamera &cam = cams[c];
-    const long long s = c * n + i;
-    const double lon = st.f[0][s], lat = st.f[1][s];
-    if (normalized) {
-        lon_out[s] = lon;
-        lat_out[s] = lat;
-        if (alt_out) alt_out[s] = st.f[10][s];
-    } else {
-        lon_out[s] = __dadd_rn(__dmul_rn(lon, cam.lon_scale), cam.lon_off);
-        lat_out[s] = __dadd_rn(__dmul_rn(lat, cam.lat_scale), cam.lat_off);
-        if (alt_out) alt_out[s] = alt[c * stride + i];
-    }
-}
+// Per camera: targets, failure flags, unconverged counts, and which cameras go on.
+struct InvCounters {
+    int *target, *failed, *count, *run;
+};
 
-InvState carve_inverse(Carver &cv, int n_cams, long long n, int *&count, int *&iter) {
+InvState carve_inverse(Carver &cv, int n_cams, long long n, InvCounters &k) {
     InvState st;
     for (auto &f : st.f) f = cv.take<double>(static_cast<size_t>(n_cams) * n);
-    count = cv.take<int>(n_cams);
-    iter = cv.take<int>(n_cams);
+    st.k = cv.take<int>(static_cast<size_t>(n_cams) * n);
+    int *base = cv.take<int>(4 * static_cast<size_t>(n_cams));
+    k = {base, base + n_cams, base + 2 * static_cast<size_t>(n_cams), base + 3 * static_cast<size_t>(n_cams)};
     return st;
 }
 
@@ -157,8 +245,8 @@ using namespace vs;
 extern "C" size_t vs_rpc_inverse_project_workspace_size(int n_cams, int64_t n) {
     if (n_cams <= 0 || n < 0) return 0;
     Carver cv(nullptr);
-    int *a, *b;
-    carve_inverse(cv, n_cams, n, a, b);
+    InvCounters k;
+    carve_inverse(cv, n_cams, n, k);
     return cv.used + 256;
 }
 
@@ -175,7 +263,6 @@ extern "C" int vs_rpc_inverse_project(const VsRpcCamera *cams, int n_cams, const
         set_error("vs_rpc_inverse_project: workspace %zu < %zu bytes", workspace_bytes, need);
         return VS_ERR_WORKSPACE;
     }
-    std::vector<int> it(n_cams, 0), cnt(n_cams, 0);
     if (n == 0) {
         if (iterations)
             for (int c = 0; c < n_cams; ++c) iterations[c] = 0;
@@ -183,56 +270,48 @@ extern "C" int vs_rpc_inverse_project(const VsRpcCamera *cams, int n_cams, const
     }
     cudaStream_t st = as_stream(stream);
     Carver cv(workspace);
-    int *d_count = nullptr, *d_iter = nullptr;
-    const InvState state = carve_inverse(cv, n_cams, n, d_count, d_iter);
+    InvCounters d;
+    const InvState state = carve_inverse(cv, n_cams, n, d);
     const dim3 grid(static_cast<unsigned>(ceil_div(n, kInvThreads)), static_cast<unsigned>(n_cams));
-    auto fetch = [&]() -> int {
-        if (cudaMemcpyAsync(cnt.data(), d_count, sizeof(int) * n_cams, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-            cudaStreamSynchronize(st) != cudaSuccess) {
-            set_error("vs_rpc_inverse_project: %s", cudaGetErrorString(cudaGetLastError()));
-            return VS_ERR_CUDA;
-        }
-        return VS_OK;
+    std::vector<int> h(3 * static_cast<size_t>(n_cams));      // targets, failures, counts
+    const size_t bytes = sizeof(int) * n_cams;
+    auto cuda_ok = [](cudaError_t e) {
+        if (e != cudaSuccess) set_error("vs_rpc_inverse_project: %s", cudaGetErrorString(e));
+        return e == cudaSuccess;
     };
-    if (cudaMemsetAsync(d_count, 0, sizeof(int) * n_cams, st) != cudaSuccess) {
-        set_error("vs_rpc_inverse_project: cudaMemsetAsync failed");
-        return VS_ERR_CUDA;
-    }
-    inverse_init_kernel<<<grid, kInvThreads, 0, st>>>(cams, col, row, alt, n, point_stride, state, d_count);
-    VS_LAUNCH_CHECK("inverse_init_kernel");
-    int s = fetch();
-    if (s != VS_OK) return s;
-    // per camera: iterations done, or -1 once all of its points have converged
-    std::vector<int> state_iter(n_cams);
-    for (int c = 0; c < n_cams; ++c) state_iter[c] = cnt[c] > 0 ? 0 : -1;
+    if (!cuda_ok(cudaMemsetAsync(d.target, 0, 3 * bytes, st))) return VS_ERR_CUDA;
+    inverse_first_kernel<<<grid, kInvThreads, 0, st>>>(cams, col, row, alt, n, point_stride, max_iter, state, d.target,
+                                                       d.failed);
+    VS_LAUNCH_CHECK("inverse_first_kernel");
+    const int *run = nullptr;
+    std::vector<int> go(n_cams);
     for (;;) {
+        inverse_advance_kernel<<<grid, kInvThreads, 0, st>>>(cams, alt, n, point_stride, normalized, state, d.target, run,
+                                                             lon, lat, alt_out, d.count);
+        VS_LAUNCH_CHECK("inverse_advance_kernel");
+        if (!cuda_ok(cudaMemcpyAsync(h.data(), d.target, 3 * bytes, cudaMemcpyDeviceToHost, st)) ||
+            !cuda_ok(cudaStreamSynchronize(st)))
+            return VS_ERR_CUDA;
+        const int *target = h.data(), *failed = target + n_cams, *count = failed + n_cams;
         bool any = false;
-        for (int c = 0; c < n_cams; ++c) any |= state_iter[c] >= 0;
-        if (!any) break;
-        for (int c = 0; c < n_cams; ++c)
-            if (state_iter[c] >= max_iter) {
+        for (int c = 0; c < n_cams; ++c) {
+            go[c] = count[c] > 0;
+            any |= go[c] != 0;
+            if (failed[c] || (go[c] && target[c] >= max_iter)) {
                 set_error("vs_rpc_inverse_project: camera %d did not converge in %d iterations", c, max_iter);
                 return VS_ERR_DEGENERATE;
             }
-        if (cudaMemcpyAsync(d_iter, state_iter.data(), sizeof(int) * n_cams, cudaMemcpyHostToDevice, st) !=
-                cudaSuccess ||
-            cudaMemsetAsync(d_count, 0, sizeof(int) * n_cams, st) != cudaSuccess) {
-            set_error("vs_rpc_inverse_project: upload failed");
+        }
+        if (!any) break;
+        // points that left the bound again at the common iteration: their cameras go on by one
+        for (int c = 0; c < n_cams; ++c) h[c] += go[c];
+        if (!cuda_ok(cudaMemcpyAsync(d.target, h.data(), bytes, cudaMemcpyHostToDevice, st)) ||
+            !cuda_ok(cudaMemcpyAsync(d.run, go.data(), bytes, cudaMemcpyHostToDevice, st)) ||
+            !cuda_ok(cudaMemsetAsync(d.count, 0, bytes, st)))
             return VS_ERR_CUDA;
-        }
-        inverse_step_kernel<<<grid, kInvThreads, 0, st>>>(cams, d_iter, n, state, d_count);
-        VS_LAUNCH_CHECK("inverse_step_kernel");
-        if ((s = fetch()) != VS_OK) return s;
-        for (int c = 0; c < n_cams; ++c) {
-            if (state_iter[c] < 0) continue;
-            ++it[c];
-            state_iter[c] = cnt[c] > 0 ? state_iter[c] + 1 : -1;
-        }
+        run = d.run;
     }
-    inverse_final_kernel<<<grid, kInvThreads, 0, st>>>(cams, alt, n, point_stride, normalized, state, lon, lat,
-                                                        alt_out);
-    VS_LAUNCH_CHECK("inverse_final_kernel");
     if (iterations)
-        for (int c = 0; c < n_cams; ++c) iterations[c] = it[c];
+        for (int c = 0; c < n_cams; ++c) iterations[c] = h[c];
     return VS_OK;
 }
