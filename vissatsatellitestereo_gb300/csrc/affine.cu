@@ -33,20 +33,22 @@ __global__ void aff_box_init_kernel(unsigned long long *box, int n_views) {
     if (i < n_views * 6) box[i] = (i % 6) < 3 ? ~0ull : 0ull;   // mins, then maxs
 }
 
-// min/max per axis over a strided sample of each view's points (grid y = view)
+// min/max per axis over a strided sample of each view's points (grid y = view).  Integer
+// tests and keys only: an FP64 compare costs ~20 cycles of the narrow pipe per warp.
 __global__ void aff_box_kernel(const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ z,
                                long long stride, long long n, long long step, unsigned long long *__restrict__ box) {
     const int v = blockIdx.y;
     const double *src[3] = {x + v * stride, y + v * stride, z + v * stride};
+    const unsigned long long limit = 0x7e37e43c8800759cull;     // bits of 1e300: larger, inf and NaN are skipped
     unsigned long long mn[3] = {~0ull, ~0ull, ~0ull}, mx[3] = {0ull, 0ull, 0ull};
     for (long long k = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; k * step < n;
          k += static_cast<long long>(gridDim.x) * blockDim.x) {
         const long long i = k * step;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            const double val = src[a][i];
-            if (val == val && fabs(val) < 1e300) {
-                const unsigned long long kk = dkey(val);
+            const long long val = reinterpret_cast<const long long *>(src[a])[i];
+            if (static_cast<unsigned long long>(val & 0x7fffffffffffffffll) < limit) {
+                const unsigned long long kk = dkey(__longlong_as_double(val));
                 mn[a] = min(mn[a], kk);
                 mx[a] = max(mx[a], kk);
             }
@@ -65,12 +67,15 @@ __global__ void aff_box_kernel(const double *__restrict__ x, const double *__res
     }
 }
 
-__global__ void aff_norm_kernel(const unsigned long long *__restrict__ box, int n_views, AffNorm *__restrict__ norm) {
+// shared: all views have one point set, whose box is the first one
+__global__ void aff_norm_kernel(const unsigned long long *__restrict__ box, int n_views, int shared,
+                                AffNorm *__restrict__ norm) {
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= n_views) return;
+    const int b = shared ? 0 : v;
     AffNorm nm;
     for (int a = 0; a < 3; ++a) {
-        const unsigned long long lo = box[v * 6 + a], hi = box[v * 6 + 3 + a];
+        const unsigned long long lo = box[b * 6 + a], hi = box[b * 6 + 3 + a];
         double c = 0.0, s = 1.0;
         if (lo <= hi && hi != 0ull) {
             const double l = double_from_key(lo), h = double_from_key(hi);
@@ -134,17 +139,37 @@ __global__ void __launch_bounds__(kAffThreads) aff_moments_kernel(
     }
 }
 
-// One thread per view: sum the block partials in order, Cholesky-solve both systems,
-// map back to raw coordinates.  P row-major [2][4]; params (optional) [w, h, P].
-__global__ void aff_solve_kernel(const double *__restrict__ partial, int blocks, int n_views,
-                                 const AffNorm *__restrict__ norm, const VsRpcCamera *__restrict__ cams,
-                                 double *__restrict__ P, double *__restrict__ params, int32_t *__restrict__ status) {
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= n_views) return;
-    double m[kAffSums];
-    for (int k = 0; k < kAffSums; ++k) m[k] = 0.0;
-    for (int b = 0; b < blocks; ++b)
-        for (int k = 0; k < kAffSums; ++k) m[k] += partial[(static_cast<long long>(v) * blocks + b) * kAffSums + k];
+// One block per view: the block partials summed in kAffChains interleaved chains per sum (one
+// thread walking all of them took 73 us for 53 blocks), then Cholesky and the two right-hand
+// sides on one lane each, mapped back to raw coordinates.  P row-major [2][4]; params
+// (optional) [w, h, P].
+constexpr int kAffChains = 14;
+constexpr int kAffSolveThreads = 256;
+static_assert(kAffChains * kAffSums <= kAffSolveThreads, "one thread per chain");
+
+__global__ void __launch_bounds__(kAffSolveThreads) aff_solve_kernel(
+    const double *__restrict__ partial, int blocks, const AffNorm *__restrict__ norm,
+    const VsRpcCamera *__restrict__ cams, double *__restrict__ P, double *__restrict__ params,
+    int32_t *__restrict__ status) {
+    __shared__ double chains[kAffChains][kAffSums];
+    __shared__ double m[kAffSums];
+    const int v = blockIdx.x;
+    const int slot = threadIdx.x % kAffSums, chain = threadIdx.x / kAffSums;
+    if (chain < kAffChains) {
+        double s = 0.0;
+        const double *p = partial + static_cast<long long>(v) * blocks * kAffSums + slot;
+        for (int b = chain; b < blocks; b += kAffChains) s += p[static_cast<long long>(b) * kAffSums];
+        chains[chain][slot] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x < kAffSums) {
+        double s = 0.0;
+        for (int k = 0; k < kAffChains; ++k) s += chains[k][threadIdx.x];
+        m[threadIdx.x] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x >= 2) return;
+    const int rhs = threadIdx.x;           // 0: columns, 1: rows
     double G[4][4];
     int q = 0;
     for (int a = 0; a < 4; ++a)
@@ -169,39 +194,36 @@ __global__ void aff_solve_kernel(const double *__restrict__ partial, int blocks,
         }
     }
     const AffNorm nm = norm[v];
-    double out[8];
-    for (int rhs = 0; rhs < 2; ++rhs) {
-        double a[4];
-        if (ok) {
-            double t[4];
-            for (int i = 0; i < 4; ++i) {
-                double s = m[10 + 4 * rhs + i];
-                for (int k = 0; k < i; ++k) s -= L[i][k] * t[k];
-                t[i] = s / L[i][i];
-            }
-            for (int i = 3; i >= 0; --i) {
-                double s = t[i];
-                for (int k = i + 1; k < 4; ++k) s -= L[k][i] * a[k];
-                a[i] = s / L[i][i];
-            }
-        } else {
-            for (int i = 0; i < 4; ++i) a[i] = __longlong_as_double(0x7ff8000000000000ll);
+    double a[4];
+    if (ok) {
+        double t[4];
+        for (int i = 0; i < 4; ++i) {
+            double s = m[10 + 4 * rhs + i];
+            for (int k = 0; k < i; ++k) s -= L[i][k] * t[k];
+            t[i] = s / L[i][i];
         }
-        // value = a0 (x - c0) s0 + a1 (y - c1) s1 + a2 (z - c2) s2 + a3
-        double off = a[3];
-        for (int k = 0; k < 3; ++k) {
-            out[4 * rhs + k] = a[k] * nm.s[k];
-            off -= a[k] * nm.s[k] * nm.c[k];
+        for (int i = 3; i >= 0; --i) {
+            double s = t[i];
+            for (int k = i + 1; k < 4; ++k) s -= L[k][i] * a[k];
+            a[i] = s / L[i][i];
         }
-        out[4 * rhs + 3] = off;
+    } else {
+        for (int i = 0; i < 4; ++i) a[i] = __longlong_as_double(0x7ff8000000000000ll);
     }
-    for (int k = 0; k < 8; ++k) P[v * 8 + k] = out[k];
+    // value = a0 (x - c0) s0 + a1 (y - c1) s1 + a2 (z - c2) s2 + a3
+    double out[4];
+    double off = a[3];
+    for (int k = 0; k < 3; ++k) {
+        out[k] = a[k] * nm.s[k];
+        off -= a[k] * nm.s[k] * nm.c[k];
+    }
+    out[3] = off;
+    for (int k = 0; k < 4; ++k) P[v * 8 + 4 * rhs + k] = out[k];
     if (params) {
-        params[v * 10 + 0] = cams ? cams[v].width : 0.0;
-        params[v * 10 + 1] = cams ? cams[v].height : 0.0;
-        for (int k = 0; k < 8; ++k) params[v * 10 + 2 + k] = out[k];
+        params[v * 10 + rhs] = cams ? (rhs ? cams[v].height : cams[v].width) : 0.0;
+        for (int k = 0; k < 4; ++k) params[v * 10 + 2 + 4 * rhs + k] = out[k];
     }
-    if (status) status[v] = ok ? VS_OK : VS_ERR_DEGENERATE;
+    if (status && rhs == 0) status[v] = ok ? VS_OK : VS_ERR_DEGENERATE;
 }
 
 struct AffWs {
@@ -239,17 +261,16 @@ int run_affine(const double *x, const double *y, const double *z, long long stri
     const long long step = std::max<long long>(1, n / kAffSamples);
     const long long samples = ceil_div(n, step);
     aff_box_kernel<<<dim3(static_cast<unsigned>(std::max<long long>(1, std::min<long long>(ceil_div(samples, 256), 64))),
-                          n_views),
+                          stride ? n_views : 1),
                      256, 0, st>>>(x, y, z, stride, n, step, w.box);
     VS_LAUNCH_CHECK("aff_box_kernel");
-    aff_norm_kernel<<<static_cast<unsigned>(ceil_div(n_views, 128)), 128, 0, st>>>(w.box, n_views, w.norm);
+    aff_norm_kernel<<<static_cast<unsigned>(ceil_div(n_views, 128)), 128, 0, st>>>(w.box, n_views, stride == 0, w.norm);
     VS_LAUNCH_CHECK("aff_norm_kernel");
     const int blocks = aff_blocks(n);
     aff_moments_kernel<<<dim3(blocks, n_views), kAffThreads, 0, st>>>(x, y, z, stride, col, row, keep, n, w.norm,
                                                                       w.partial);
     VS_LAUNCH_CHECK("aff_moments_kernel");
-    aff_solve_kernel<<<static_cast<unsigned>(ceil_div(n_views, 64)), 64, 0, st>>>(w.partial, blocks, n_views, w.norm,
-                                                                                  cams, P ? P : w.P, params, status);
+    aff_solve_kernel<<<n_views, kAffSolveThreads, 0, st>>>(w.partial, blocks, w.norm, cams, P ? P : w.P, params, status);
     VS_LAUNCH_CHECK("aff_solve_kernel");
     return VS_OK;
 }
