@@ -9,7 +9,7 @@
 //          (8 accumulators for 8 <= V <= 128, halving above), started from 0, then the
 //          float32 division by the kept count                     (:78)
 // then optionally the 3x3 median blur (:81), launched from raster.cu's blur kernel.
-// Views beyond 64 use a local-memory path with the same arithmetic.
+// Cells of more than 64 views are shared by 2, 4 or 8 lanes, with the same arithmetic.
 #include <algorithm>
 #include <math.h>
 #include <mutex>
@@ -21,92 +21,8 @@ int launch_blur_f32(const float *in, float *out, long long h, long long w, cudaS
 
 namespace {
 
-__device__ __forceinline__ float median_of_sorted(unsigned lo_key, unsigned hi_key) {
-    const float lo = float_from_key(lo_key), hi = float_from_key(hi_key);
-    return __fdiv_rn(__fadd_rn(__fadd_rn(0.0f, lo), hi), 2.0f);
-}
-
-// ---- V > 64: same arithmetic with local arrays -----------------------------------------
-// numpy's pairwise block of n <= 128 values: 8 accumulators, combined in a tree, then the
-// tail (n < 8: a plain sequential sum from 0).
-__device__ __forceinline__ float pairwise_block(const float *x, int n) {
-    float res;
-    if (n < 8) {
-        res = 0.0f;
-        for (int i = 0; i < n; ++i) res = __fadd_rn(res, x[i]);
-        return res;
-    }
-    float r[8];
-    for (int j = 0; j < 8; ++j) r[j] = x[j];
-    int i = 8;
-    for (; i < n - (n % 8); i += 8)
-        for (int j = 0; j < 8; ++j) r[j] = __fadd_rn(r[j], x[i + j]);
-    res = __fadd_rn(__fadd_rn(__fadd_rn(r[0], r[1]), __fadd_rn(r[2], r[3])),
-                    __fadd_rn(__fadd_rn(r[4], r[5]), __fadd_rn(r[6], r[7])));
-    for (; i < n; ++i) res = __fadd_rn(res, x[i]);
-    return res;
-}
-
-// numpy's halving recursion above 128 values, unrolled at compile time (no call stack):
-// D levels of halving cover n <= 128 * 2^D.
-template <int D>
-__device__ __forceinline__ float pairwise_any(const float *x, int n) {
-    if constexpr (D == 0) {
-        return pairwise_block(x, n);
-    } else {
-        if (n <= 128) return pairwise_block(x, n);
-        int n2 = n / 2;
-        n2 -= n2 % 8;
-        return __fadd_rn(pairwise_any<D - 1>(x, n2), pairwise_any<D - 1>(x + n2, n - n2));
-    }
-}
-
-constexpr int kMaxViewsLocal = 512;
-
-__device__ void insertion_sort(unsigned *a, int n) {
-    for (int i = 1; i < n; ++i) {
-        unsigned v = a[i];
-        int j = i - 1;
-        while (j >= 0 && a[j] > v) { a[j + 1] = a[j]; --j; }
-        a[j + 1] = v;
-    }
-}
-
-__global__ void fuse_kernel_large(const float *__restrict__ dsm, int layout, int V, long long cells,
-                                  float *__restrict__ out) {
-    float x[kMaxViewsLocal];
-    unsigned k[kMaxViewsLocal];
-    for (long long c = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; c < cells;
-         c += static_cast<long long>(gridDim.x) * blockDim.x) {
-        int n = 0;
-        for (int i = 0; i < V; ++i) {
-            x[i] = layout == VS_LAYOUT_VHW ? dsm[i * cells + c] : dsm[c * V + i];
-            if (!isnan(x[i])) k[n++] = key_from_float(x[i]);
-        }
-        if (n <= 2) { out[c] = __int_as_float(0x7fffffff); continue; }
-        insertion_sort(k, n);
-        const float med = median_of_sorted(k[(n - 1) >> 1], k[n >> 1]);
-        int nd = 0;
-        for (int i = 0; i < V; ++i)
-            if (!isnan(x[i])) {
-                float d = fabsf(__fsub_rn(x[i], med));
-                if (!isnan(d)) k[nd++] = key_from_float(d);
-            }
-        float mad = __int_as_float(0x7fffffff);
-        if (nd > 0) {
-            insertion_sort(k, nd);
-            mad = median_of_sorted(k[(nd - 1) >> 1], k[nd >> 1]);
-        }
-        int cnt = 0;
-        for (int i = 0; i < V; ++i) {
-            bool keep = !isnan(x[i]) && !(fabsf(__fsub_rn(x[i], med)) > mad);
-            cnt += keep;
-            x[i] = keep ? x[i] : 0.0f;
-        }
-        const float tot = __fadd_rn(0.0f, pairwise_any<4>(x, V));   // 4 levels: V <= 2048
-        out[c] = __fdiv_rn(tot, static_cast<float>(cnt));
-    }
-}
+constexpr int kMaxViews = 512;
+constexpr int kNaN = 0x7fffffff;
 
 // ---- fusion for V <= 64 -------------------------------------------------------------------
 // One thread fuses one cell:
@@ -186,6 +102,32 @@ __device__ __forceinline__ float median_pair(float lo, float hi) {
     return __fdiv_rn(__fadd_rn(__fadd_rn(0.0f, lo), hi), 2.0f);
 }
 
+// The median of the deviations |s(q) - med| of n sorted values with a finite median.
+template <class S>
+__device__ __forceinline__ float mad_of_sorted(const S &s, int n, float med) {
+    const float inf = __int_as_float(0x7f800000);
+    // left run A_j = med - s[m-1-j] (j < m), right run B_j = s[m+j] - med (j < n-m)
+    const int m = (n & 1) ? (n - 1) >> 1 : n >> 1, nb = n - m;
+    const int k = (n - 1) >> 1;
+    int lo = max(0, k + 1 - nb), hi = min(k + 1, m);
+    while (lo < hi) {
+        const int i = (lo + hi) >> 1, j = k + 1 - i;
+        if (__fsub_rn(med, s(m - 1 - i)) < __fsub_rn(s(m + j - 1), med)) lo = i + 1;
+        else hi = i;
+    }
+    const int i = lo, j = k + 1 - i;
+    const float a_last = i > 0 ? __fsub_rn(med, s(m - i)) : -inf;
+    const float b_last = j > 0 ? __fsub_rn(s(m + j - 1), med) : -inf;
+    const float kth = fmaxf(a_last, b_last);
+    float nxt = kth;
+    if (!(n & 1)) {
+        const float a_next = i < m ? __fsub_rn(med, s(m - 1 - i)) : inf;
+        const float b_next = j < nb ? __fsub_rn(s(m + j), med) : inf;
+        nxt = fminf(a_next, b_next);
+    }
+    return median_pair(kth, nxt);
+}
+
 // The cell's values: value i at xs[i * si] (shared memory or global); sorted values are
 // written to srt[i * ss] (shared memory); the values are read again, in view order, at
 // xg[i * sg].
@@ -214,27 +156,7 @@ __device__ __forceinline__ float fuse_cell_v64(const float *xs, long long si, in
     const float med = median_pair(srt[((n - 1) >> 1) * ss], srt[(n >> 1) * ss]);
     float mad = __int_as_float(0x7fffffff);
     if (isfinite(med)) {
-        // left run A_j = med - s[m-1-j] (j < m), right run B_j = s[m+j] - med (j < n-m)
-        const int m = (n & 1) ? (n - 1) >> 1 : n >> 1, nb = n - m;
-        const float *left = srt + (m - 1) * ss, *right = srt + m * ss;
-        const int k = (n - 1) >> 1;
-        int lo = max(0, k + 1 - nb), hi = min(k + 1, m);
-        while (lo < hi) {
-            const int i = (lo + hi) >> 1, j = k + 1 - i;
-            if (__fsub_rn(med, left[-i * ss]) < __fsub_rn(right[(j - 1) * ss], med)) lo = i + 1;
-            else hi = i;
-        }
-        const int i = lo, j = k + 1 - i;
-        const float a_last = i > 0 ? __fsub_rn(med, left[-(i - 1) * ss]) : -inf;
-        const float b_last = j > 0 ? __fsub_rn(right[(j - 1) * ss], med) : -inf;
-        const float kth = fmaxf(a_last, b_last);
-        float nxt = kth;
-        if (!(n & 1)) {
-            const float a_next = i < m ? __fsub_rn(med, left[-i * ss]) : inf;
-            const float b_next = j < nb ? __fsub_rn(right[j * ss], med) : inf;
-            nxt = fminf(a_next, b_next);
-        }
-        mad = median_pair(kth, nxt);
+        mad = mad_of_sorted([&](int q) -> const float & { return srt[q * ss]; }, n, med);
     } else {
         // deviations of the original values (inf - inf is NaN: missing)
         int nd = 0;
@@ -336,6 +258,218 @@ __global__ void __launch_bounds__(kTileCells) fuse_tile_kernel(const float *__re
     }
 }
 
+// ---- fusion for 64 < V <= 512 -----------------------------------------------------------------
+// L lanes of a warp fuse one cell: lane l holds values l, l + L, ... (at most 64, sorted by the
+// network above for N slots), the lanes' runs are merged by bitonic exchanges (shuffles
+// between lanes, registers within), and the sorted cell goes to shared memory, where the MAD
+// is searched as above.  The pairwise mean's 8 accumulators are shared out the same way
+// (accumulator j on lane j mod L), its sums formed as numpy forms them.
+//
+// Bound by the comparators (ALU pipe, two per clock and lane), like the kernel above.  One thread per
+// cell would need up to 512 values in registers or local memory: the local-memory
+// insertion sort this replaces took 1.98 ms for 97 views of 409 x 451 cells, this 0.108 ms.
+// The layouts keep both the staging copies and the lanes' reads free of bank conflicts.
+template <int L>
+struct WideTile {
+    static constexpr int CS = kTileCells / L;               // cells of a tile
+    static constexpr int TS = CS + 32 / L;                  // view stride of a staged [V][cells] tile
+    static constexpr int RS = 64 * CS + 32 / L;             // run stride of the sorted cells
+    static constexpr int kSorted = L * RS;
+    // cell pitch of a staged [cells][V] tile: congruent to L, so that 32 lanes meet 32 banks
+    static __host__ __device__ int pitch(int V) { return V + ((L - V % 32 + 32) % 32); }
+    static __host__ __device__ size_t floats(int layout, int V) {
+        return layout == VS_LAYOUT_VHW ? static_cast<size_t>(V) * TS : static_cast<size_t>(CS) * pitch(V);
+    }
+};
+
+// Sorts the cell's 64 L values (64 per lane, each lane's first N unsorted, the others +inf)
+// across its lanes: rank 64 l + i ends in a[i] of lane l.
+template <int N, int L>
+__device__ __forceinline__ void wide_sort(float (&v)[N], float (&a)[64], int l) {
+    oems_sort(v);
+#pragma unroll
+    for (int i = 0; i < 64; ++i) a[i] = i < N ? v[i < N ? i : 0] : __int_as_float(0x7f800000);
+#pragma unroll
+    for (int w = 1; w < L; w <<= 1) {
+        // the halves of a group of 2w lanes are sorted: first against the other's reverse
+        bool up = (l & w) != 0;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            const float t = __shfl_xor_sync(0xffffffffu, a[63 - i], 2 * w - 1);
+            const float u = __shfl_xor_sync(0xffffffffu, a[i], 2 * w - 1);
+            a[i] = up ? fmaxf(a[i], t) : fminf(a[i], t);
+            a[63 - i] = up ? fmaxf(a[63 - i], u) : fminf(a[63 - i], u);
+        }
+#pragma unroll
+        for (int d = w >> 1; d >= 1; d >>= 1) {
+            up = (l & d) != 0;
+#pragma unroll
+            for (int i = 0; i < 64; ++i) {
+                const float t = __shfl_xor_sync(0xffffffffu, a[i], d);
+                a[i] = up ? fmaxf(a[i], t) : fminf(a[i], t);
+            }
+        }
+#pragma unroll
+        for (int d = 32; d >= 1; d >>= 1)
+#pragma unroll
+            for (int i = 0; i < 64; ++i)
+                if (!(i & d)) cmpx(a, i, i + d);
+    }
+}
+
+// Sum over the lanes of a cell.
+template <int L>
+__device__ __forceinline__ int lane_sum(int n) {
+#pragma unroll
+    for (int d = 1; d < L; d <<= 1) n += __shfl_xor_sync(0xffffffffu, n, d);
+    return n;
+}
+
+// numpy's pairwise sum of x(0..n-1), n <= 128, on the cell's lanes (x(i) is asked of lane i mod
+// L, and of every lane in the tail).
+template <int L, class X>
+__device__ __forceinline__ float wide_pairwise_block(const X &x, int first, int n, int l) {
+    if (n < 8) {
+        float res = 0.0f;
+        for (int i = 0; i < n; ++i) res = __fadd_rn(res, x(first + i));
+        return res;
+    }
+    constexpr int K = 8 / L;
+    const int full = n - n % 8;
+    float r[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) r[k] = x(first + k * L + l);
+    for (int b = 8; b < full; b += 8)
+#pragma unroll
+        for (int k = 0; k < K; ++k) r[k] = __fadd_rn(r[k], x(first + b + k * L + l));
+    // ((r0 + r1) + (r2 + r3)) + ((r4 + r5) + (r6 + r7)): neighbours first between the lanes, then
+    // within one (a sum of two is the same on both)
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+        for (int d = 1; d < L; d <<= 1) r[k] = __fadd_rn(r[k], __shfl_xor_sync(0xffffffffu, r[k], d));
+#pragma unroll
+    for (int h = 1; h < K; h <<= 1)
+#pragma unroll
+        for (int k = 0; k + h < K; k += 2 * h) r[k] = __fadd_rn(r[k], r[k + h]);
+    float res = r[0];
+    for (int i = full; i < n; ++i) res = __fadd_rn(res, x(first + i));
+    return res;
+}
+
+// numpy's halving recursion above 128 values, unrolled at compile time (no call stack): D levels
+// cover n <= 512.
+template <int L, int D, class X>
+__device__ __forceinline__ float wide_pairwise(const X &x, int first, int n, int l) {
+    if constexpr (D == 0) {
+        return wide_pairwise_block<L>(x, first, n, l);
+    } else {
+        if (n <= 128) return wide_pairwise_block<L>(x, first, n, l);
+        int n2 = n / 2;
+        n2 -= n2 % 8;
+        const float lo = wide_pairwise<L, D - 1>(x, first, n2, l);
+        return __fadd_rn(lo, wide_pairwise<L, D - 1>(x, first + n2, n - n2, l));
+    }
+}
+
+template <int N, int L>
+__global__ void __launch_bounds__(kTileCells, 3) fuse_wide_kernel(const float *__restrict__ dsm, int layout, int V,
+                                                               long long cells, float *__restrict__ out,
+                                                               long long n_tiles, int aligned) {
+    using T = WideTile<L>;
+    extern __shared__ __align__(16) float fsm[];            // the sorted cells, then the tile
+    float *tile = fsm + ((T::kSorted + 3) & ~3);
+    const int tid = threadIdx.x, cell = tid / L, l = tid % L;
+    const bool vhw = layout == VS_LAYOUT_VHW;
+    const int pitch = T::pitch(V);
+    const int sc = vhw ? 1 : pitch, sv = vhw ? T::TS : 1;
+    const float inf = __int_as_float(0x7f800000);
+    const float *mine = tile + cell * sc;                   // value v of the cell at mine[v * sv]
+    auto sorted = [&](int q) -> float & { return fsm[(q & 63) * T::CS + (q >> 6) * T::RS + cell]; };
+    for (long long tl = blockIdx.x; tl < n_tiles; tl += gridDim.x) {
+        const long long c0 = tl * T::CS;
+        const int len = static_cast<int>(min(static_cast<long long>(T::CS), cells - c0));
+        if (vhw && aligned) {
+            for (int q = tid; q < V * (T::CS / 4); q += kTileCells) {
+                const int v = q / (T::CS / 4), ch = q - v * (T::CS / 4);
+                if (4 * ch < len) cp_async16(tile + v * T::TS + 4 * ch, dsm + v * cells + c0 + 4 * ch);
+            }
+        } else if (vhw) {
+            for (int q = tid; q < V * T::CS; q += kTileCells) {
+                const int v = q / T::CS, c = q - v * T::CS;
+                if (c < len) cp_async4(tile + v * T::TS + c, dsm + v * cells + c0 + c);
+            }
+        } else {                     // the tile is one run of len * V values
+            int c = tid / V, v = tid - c * V;
+            for (int q = tid; q < len * V; q += kTileCells) {
+                cp_async4(tile + c * pitch + v, dsm + c0 * V + q);
+                v += kTileCells;
+                while (v >= V) {
+                    v -= V;
+                    ++c;
+                }
+            }
+        }
+        cp_async_commit();
+        cp_async_wait_all();
+        __syncthreads();
+        const bool in = cell < len;
+        // pass 0 sorts the values; a second pass, over the deviations, is only taken for a median
+        // that is not finite
+        int n = 0;
+        float med = 0.0f, mad = __int_as_float(kNaN);
+        bool again = false;
+#pragma unroll 1
+        for (int pass = 0; pass < 2; ++pass) {
+            float v[N], a[64];
+            int valid = 0;
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                const int k = i * L + l;
+                float x = inf;
+                if (in && k < V) {
+                    x = mine[k * sv];
+                    if (pass) x = fabsf(__fsub_rn(x, med));
+                    const bool ok = !isnan(x);
+                    valid += ok;
+                    x = ok ? x : inf;
+                }
+                v[i] = x;
+            }
+            valid = lane_sum<L>(valid);
+            wide_sort<N, L>(v, a, l);
+#pragma unroll
+            for (int i = 0; i < 64; ++i) sorted(64 * l + i) = a[i];
+            __syncwarp();
+            if (pass == 0) {
+                n = valid;
+                if (n > 2) {
+                    med = median_pair(sorted((n - 1) >> 1), sorted(n >> 1));
+                    if (isfinite(med)) mad = mad_of_sorted(sorted, n, med);
+                    else again = true;
+                }
+                __syncwarp();
+                if (!__any_sync(0xffffffffu, again)) break;
+            } else if (again && valid > 0) {
+                mad = median_pair(sorted((valid - 1) >> 1), sorted(valid >> 1));
+            }
+        }
+        // keep |x - med| <= mad, numpy's float32 pairwise sum of the kept values (others 0)
+        int cnt = 0;
+        auto kept = [&](int i) {
+            const float x = in ? mine[i * sv] : 0.0f;
+            const bool keep = !isnan(x) && !(fabsf(__fsub_rn(x, med)) > mad);
+            cnt += keep && i % L == l;
+            return keep ? x : 0.0f;
+        };
+        const float res = wide_pairwise<L, 4>(kept, 0, V, l);
+        cnt = lane_sum<L>(cnt);
+        if (in && l == 0)
+            out[c0 + cell] = n <= 2 ? __int_as_float(kNaN) : __fdiv_rn(__fadd_rn(0.0f, res), static_cast<float>(cnt));
+        __syncthreads();                           // the tile is refilled next
+    }
+}
+
 size_t fuse_tile_smem(int V, int N) { return sizeof(float) * static_cast<size_t>(V + N) * kTileCells; }
 
 template <int N>
@@ -358,6 +492,39 @@ bool launch_fuse_v64(const float *dsm, int layout, int V, long long cells, float
     return true;
 }
 
+template <int N, int L>
+bool launch_fuse_wide_n(const float *dsm, int layout, int V, long long cells, float *out, bool aligned,
+                        cudaStream_t st) {
+    using T = WideTile<L>;
+    const size_t base = (static_cast<size_t>(T::kSorted) + 3) & ~size_t(3);
+    const size_t sh = sizeof(float) * (base + T::floats(layout, V));
+    static bool configured = false;     // per instantiation: room for the largest tile (V = 64 L)
+    if (!configured) {
+        const size_t most = sizeof(float) * (base + std::max<size_t>(64 * L * T::TS, T::CS * (64 * L + 32)));
+        if (cudaFuncSetAttribute(fuse_wide_kernel<N, L>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(most)) != cudaSuccess)
+            return false;
+        configured = true;
+    }
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fuse_wide_kernel<N, L>, kTileCells, sh) != cudaSuccess ||
+        per_sm <= 0)
+        return false;
+    const long long n_tiles = ceil_div(cells, static_cast<long long>(T::CS));
+    const unsigned g = static_cast<unsigned>(std::min<long long>(n_tiles, 1LL * sm_count() * per_sm));
+    fuse_wide_kernel<N, L><<<g, kTileCells, sh, st>>>(dsm, layout, V, cells, out, n_tiles, aligned ? 1 : 0);
+    return true;
+}
+
+// The fewest lanes that hold the views, each with the smaller of two networks that takes its share.
+template <int L>
+bool launch_fuse_wide_l(const float *dsm, int layout, int V, long long cells, float *out, bool aligned,
+                        cudaStream_t st) {
+    const int share = (V + L - 1) / L;
+    if (share <= 48) return launch_fuse_wide_n<48, L>(dsm, layout, V, cells, out, aligned, st);
+    return launch_fuse_wide_n<64, L>(dsm, layout, V, cells, out, aligned, st);
+}
+
 // 16-byte copies need 16-byte aligned view rows (VHW) or cell blocks (HWV).
 bool fuse_tile_aligned(const float *dsm, int layout, int V, long long cells) {
     (void)layout;
@@ -365,10 +532,14 @@ bool fuse_tile_aligned(const float *dsm, int layout, int V, long long cells) {
     return (reinterpret_cast<uintptr_t>(dsm) & 15) == 0 && cells % 4 == 0;
 }
 
-int launch_fuse_small(const float *dsm, int layout, int V, long long cells, float *out, cudaStream_t st) {
+int launch_fuse(const float *dsm, int layout, int V, long long cells, float *out, cudaStream_t st) {
     const bool aligned = fuse_tile_aligned(dsm, layout, V, cells);
     bool ok = false;
-    switch ((V + 3) / 4) {
+    if (V > 64) {
+        ok = V <= 128   ? launch_fuse_wide_l<2>(dsm, layout, V, cells, out, aligned, st)
+             : V <= 256 ? launch_fuse_wide_l<4>(dsm, layout, V, cells, out, aligned, st)
+                        : launch_fuse_wide_l<8>(dsm, layout, V, cells, out, aligned, st);
+    } else switch ((V + 3) / 4) {
         case 0: case 1: ok = launch_fuse_v64<4>(dsm, layout, V, cells, out, aligned, st); break;
         case 2: ok = launch_fuse_v64<8>(dsm, layout, V, cells, out, aligned, st); break;
         case 3: ok = launch_fuse_v64<12>(dsm, layout, V, cells, out, aligned, st); break;
@@ -417,7 +588,7 @@ extern "C" size_t vs_fuse_dsms_workspace_size(int64_t h, int64_t w) {
 
 extern "C" int vs_fuse_dsms(const float *dsm, int layout, int64_t n_views, int64_t h, int64_t w, float *out,
                             int median_blur, void *workspace, size_t workspace_bytes, void *stream) {
-    VS_REQUIRE(checked_cells(h, w, kMaxFuseCells) > 0 && n_views > 0 && n_views <= kMaxViewsLocal,
+    VS_REQUIRE(checked_cells(h, w, kMaxFuseCells) > 0 && n_views > 0 && n_views <= kMaxViews,
                "vs_fuse_dsms: bad sizes views=%lld grid=%lldx%lld", (long long)n_views, (long long)h,
                (long long)w);
     VS_REQUIRE(layout == VS_LAYOUT_HWV || layout == VS_LAYOUT_VHW, "vs_fuse_dsms: bad layout %d", layout);
@@ -435,14 +606,8 @@ extern "C" int vs_fuse_dsms(const float *dsm, int layout, int64_t n_views, int64
         dst = static_cast<float *>(workspace);
     }
     const int V = static_cast<int>(n_views);
-    if (V <= 64) {
-        const int s = launch_fuse_small(dsm, layout, V, cells, dst, st);
-        if (s != VS_OK) return s;
-    } else {
-        const int threads = 64;
-        unsigned g = static_cast<unsigned>(std::min<long long>(ceil_div(cells, threads), sm_count() * 8LL));
-        fuse_kernel_large<<<g, threads, 0, st>>>(dsm, layout, V, cells, dst);
-    }
+    const int s = launch_fuse(dsm, layout, V, cells, dst, st);
+    if (s != VS_OK) return s;
     VS_LAUNCH_CHECK("fuse_kernel");
     if (median_blur) return launch_blur_f32(dst, out, h, w, st);
     return VS_OK;
