@@ -110,20 +110,30 @@ __device__ __forceinline__ int axis_index(const Axis &ax, double v) {
 
 // T[r] = smallest d >= 0 with floor(fl(d*ulp / res)) >= r, for r = 0..n.  d*ulp is exact,
 // so this is the reference's expression evaluated at the representable differences.
-__global__ void axis_thresholds_kernel(long long *thr, long long n, double ulp, double res) {
-    long long r = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-    if (r > n) return;
-    if (r == 0) {
-        thr[0] = 0;
-        return;
-    }
+__device__ __forceinline__ long long axis_threshold(long long r, double ulp, double res) {
+    if (r == 0) return 0;
     const double rd = static_cast<double>(r);
     long long d = static_cast<long long>(ceil(rd * res / ulp));
     if (d < 0) d = 0;
     // walk to the exact boundary (a handful of steps; bounded)
     for (int it = 0; it < 64 && d > 0 && floor(__ddiv_rn(static_cast<double>(d - 1) * ulp, res)) >= rd; ++it) --d;
     for (int it = 0; it < 64 && floor(__ddiv_rn(static_cast<double>(d) * ulp, res)) < rd; ++it) ++d;
-    thr[r] = d;
+    return d;
+}
+
+// One axis's table; n < 0: none (the axis has no fast path).
+struct ThresholdJob {
+    long long *thr;
+    long long n;
+    double ulp, res;
+};
+
+// The tables of both axes in one launch: 5 us of launch and FP64 latency, not twice.
+__global__ void __launch_bounds__(64) axis_thresholds_kernel(ThresholdJob row, ThresholdJob col) {
+    const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    if (i <= row.n) row.thr[i] = axis_threshold(i, row.ulp, row.res);
+    const long long j = i - (row.n + 1);
+    if (j >= 0 && j <= col.n) col.thr[j] = axis_threshold(j, col.ulp, col.res);
 }
 
 __device__ __forceinline__ bool is_nan_bits(unsigned long long b) {
@@ -399,19 +409,6 @@ __device__ __forceinline__ unsigned long long cell_key(unsigned long long k, lon
     return k != kZeroKey ? k : zero_key(cell, first, pts);
 }
 
-__device__ __forceinline__ double key_value(unsigned long long k) {
-    return k == kEmptyKey ? __longlong_as_double(0x7ff8000000000000ll) : double_from_key(k);
-}
-
-// nanmax grid (FP64) from the keys.
-__global__ void decode_kernel(const unsigned long long *__restrict__ keys,
-                              const unsigned long long *__restrict__ first,
-                              const double *__restrict__ pts, double *__restrict__ out, long long total) {
-    for (long long c = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; c < total;
-         c += static_cast<long long>(gridDim.x) * blockDim.x)
-        out[c] = key_value(cell_key(keys[c], c, first, pts));
-}
-
 // numpy's median of the non-empty keys among 8 (empty = 0), without local memory: the
 // keys are sorted by an 8-input network with empty slots ordered last, and the middle
 // one(s) selected by the count.
@@ -456,42 +453,63 @@ __device__ __forceinline__ double median8_keys(unsigned long long (&s)[8]) {
     return median_from_middle(select8(s, (n - 1) >> 1), select8(s, n >> 1), n);
 }
 
-__device__ __forceinline__ bool nan_double(double v) {
-    return is_nan_bits(static_cast<unsigned long long>(__double_as_longlong(v)));
-}
+// The FP64 grid from the keys: nanmax values and the non-propagating hole fill
+// (lib/proj_to_grid.py:64-79) in one pass over 32 x 32 tiles.  The keys and a 1-cell halo are
+// loaded at once (six loads in flight per thread, one trip to L2) and staged; empty cells go
+// to a list that consecutive threads fill, so that a warp with one hole does not run the
+// median for 32 cells.  1025 x 1025 cells: 32 us as a decode and a per-cell fill, 11 us.
+constexpr int kGridTile = 32, kGridRaw = kGridTile + 2, kGridThreads = 256;
 
-// Non-propagating hole fill (lib/proj_to_grid.py:64-79) on an FP64 grid.
-__global__ void hole_fill_kernel(const double *__restrict__ in, double *__restrict__ out, long long H,
-                                 long long W, long long total) {
-    for (long long c = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; c < total;
-         c += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const long long plane = c / (H * W);
-        const long long rc = c - plane * H * W;
-        const long long r = rc / W, col = rc - r * W;
-        const double *img = in + plane * H * W;
-        double v = img[rc];
-        if (!nan_double(v)) {
-            out[c] = v;
-            continue;
+__global__ void __launch_bounds__(kGridThreads) grid_f64_kernel(const unsigned long long *__restrict__ keys,
+                                                                const unsigned long long *__restrict__ first,
+                                                                const double *__restrict__ pts,
+                                                                double *__restrict__ out, int H, int W) {
+    __shared__ unsigned long long raw[kGridRaw * kGridRaw];
+    __shared__ unsigned short holes[kGridTile * kGridTile];
+    __shared__ int n_holes;
+    constexpr int kLoads = (kGridRaw * kGridRaw + kGridThreads - 1) / kGridThreads;
+    const int tid = threadIdx.x, r0 = blockIdx.y * kGridTile, c0 = blockIdx.x * kGridTile;
+    if (tid == 0) n_holes = 0;
+    unsigned long long k[kLoads];
+#pragma unroll
+    for (int q = 0; q < kLoads; ++q) {
+        const int i = q * kGridThreads + tid, ly = i / kGridRaw, lx = i - ly * kGridRaw;
+        const int r = r0 + ly - 1, c = c0 + lx - 1;
+        k[q] = kEmptyKey;
+        if (i < kGridRaw * kGridRaw && static_cast<unsigned>(r) < static_cast<unsigned>(H) &&
+            static_cast<unsigned>(c) < static_cast<unsigned>(W))
+            k[q] = keys[static_cast<long long>(r) * W + c];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kLoads; ++q) {
+        const int i = q * kGridThreads + tid, ly = i / kGridRaw, lx = i - ly * kGridRaw;
+        if (i >= kGridRaw * kGridRaw) break;
+        const int r = r0 + ly - 1, c = c0 + lx - 1;
+        const long long cell = static_cast<long long>(r) * W + c;
+        k[q] = cell_key(k[q], cell, first, pts);
+        raw[i] = k[q];
+        if (ly >= 1 && ly <= kGridTile && lx >= 1 && lx <= kGridTile && r < H && c < W) {
+            if (k[q] != kEmptyKey) out[cell] = double_from_key(k[q]);
+            else holes[atomicAdd(&n_holes, 1)] = static_cast<unsigned short>(i);
         }
+    }
+    __syncthreads();
+    for (int h = tid; h < n_holes; h += kGridThreads) {
+        const int i = holes[h], ly = i / kGridRaw, lx = i - ly * kGridRaw;
         unsigned long long s[8];
         int m = 0;
         bool any = false;
 #pragma unroll
         for (int dj = -1; dj <= 1; ++dj)
 #pragma unroll
-            for (int dk = -1; dk <= 1; ++dk) {
-                if (dj == 0 && dk == 0) continue;
-                const long long j = r + dj, k = col + dk;
-                unsigned long long key = kEmptyKey;
-                if (j >= 0 && j < H && k >= 0 && k < W) {
-                    const double u = img[j * W + k];
-                    if (!nan_double(u)) key = key_from_double(u);
+            for (int dk = -1; dk <= 1; ++dk)
+                if (dj != 0 || dk != 0) {
+                    s[m] = raw[i + dj * kGridRaw + dk];
+                    any |= s[m++] != kEmptyKey;
                 }
-                any |= key != kEmptyKey;
-                s[m++] = key;
-            }
-        out[c] = any ? median8_keys(s) : v;
+        out[static_cast<long long>(r0 + ly - 1) * W + (c0 + lx - 1)] =
+            any ? median8_keys(s) : __longlong_as_double(0x7ff8000000000000ll);
     }
 }
 
@@ -561,31 +579,79 @@ __device__ __forceinline__ float as_f32(T v) { return static_cast<float>(v); }
 template <>
 __device__ __forceinline__ float as_f32<double>(double v) { return f64_to_f32(v); }
 
-template <typename T>
-__global__ void median_blur3x3_kernel(const T *__restrict__ in, float *__restrict__ out, long long H,
-                                      long long W, long long total) {
-    for (long long c = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; c < total;
-         c += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const long long plane = c / (H * W);
-        const long long rc = c - plane * H * W;
-        const long long r = rc / W, col = rc - r * W;
-        const T *img = in + plane * H * W;
-        const long long rm = r > 0 ? r - 1 : 0, rp = r + 1 < H ? r + 1 : H - 1;
-        const long long cm = col > 0 ? col - 1 : 0, cp = col + 1 < W ? col + 1 : W - 1;
-        if (H == 1 || W == 1) {
-            // the line runs along the dimension that is longer than 1 (both 1: the value)
-            const long long a = H == 1 ? cm : rm * W, b = H == 1 ? col : r * W, d = H == 1 ? cp : rp * W;
-            out[c] = cv_median3_line(as_f32(img[a]), as_f32(img[b]), as_f32(img[d]));
-            continue;
-        }
-        float p[9];
-        const long long rows[3] = {rm, r, rp}, cols[3] = {cm, col, cp};
+// One warp blurs kBlurRows rows of 30 columns: lane l holds column 30 g + l - 1 (clamped into the
+// image, which is the replicated border), all its rows loaded before any arithmetic, and the
+// neighbours' sorted columns come by shuffles -- each cell is read once per warp instead of
+// nine times and converted (FP64 input) once.  Rows whose 3-row window holds a NaN or a zero in the
+// warp take OpenCV's network per cell; for the others the sorted-column median (median of
+// the columns' largest low, middle mid, smallest high) is the same value bit for bit.
+// 2000 x 2000 float32: 35.5 us with nine loads and a 64-bit division per cell, 13 us;
+// 1025 x 1025 FP64: 20 us, 9 us.
+constexpr int kBlurRows = 8, kBlurCols = 30;
+
+// I: the index type, 32 bits unless a side or the number of warps needs more (a 64-bit division
+// costs as much as a row).
+template <typename T, typename I>
+__global__ void __launch_bounds__(256) median_blur3x3_kernel(const T *__restrict__ in, float *__restrict__ out, I H, I W,
+                                                             I strips, I groups, I warps) {
+    const int lane = threadIdx.x & 31;
+    const I wid = static_cast<I>(blockIdx.x) * 8 + static_cast<I>(threadIdx.x >> 5);
+    if (wid >= warps) return;
+    const I plane = wid / (strips * groups), rest = wid - plane * (strips * groups);
+    const I strip = rest / groups, c = (rest - strip * groups) * kBlurCols + lane - 1, r0 = strip * kBlurRows;
+    const long long offset = static_cast<long long>(plane) * H * W;
+    const T *img = in + offset + min(max(c, I(0)), W - 1);
+    float *dst = out + offset + c;
+    float v[kBlurRows + 2];
+    {
+        T x[kBlurRows + 2];
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
+        for (int k = 0; k < kBlurRows + 2; ++k)
+            x[k] = __ldg(img + static_cast<long long>(min(max(r0 + k - 1, I(0)), H - 1)) * W);
 #pragma unroll
-            for (int b = 0; b < 3; ++b) p[3 * a + b] = as_f32(img[rows[a] * W + cols[b]]);
-        out[c] = cv_median9(cv_vector_column(col, W), p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], p[8]);
+        for (int k = 0; k < kBlurRows + 2; ++k) v[k] = as_f32(x[k]);
     }
+    unsigned special = H == 1 || W == 1 ? ~0u : 0u;     // bit k: row k holds a NaN or a zero
+#pragma unroll
+    for (int k = 0; k < kBlurRows + 2; ++k)
+        special |= __any_sync(0xffffffffu, isnan(v[k]) || v[k] == 0.0f) ? 1u << k : 0u;
+    const bool store = lane >= 1 && lane <= kBlurCols && c < W;
+#pragma unroll
+    for (int k = 0; k < kBlurRows; ++k) {
+        const I r = r0 + k;
+        if (r >= H) break;
+        float m;
+        if (!(special & (7u << k))) {
+            float lo, mid, hi;
+            sort3f(v[k], v[k + 1], v[k + 2], lo, mid, hi);
+            const float llo = __shfl_up_sync(0xffffffffu, lo, 1), rlo = __shfl_down_sync(0xffffffffu, lo, 1);
+            const float lmid = __shfl_up_sync(0xffffffffu, mid, 1), rmid = __shfl_down_sync(0xffffffffu, mid, 1);
+            const float lhi = __shfl_up_sync(0xffffffffu, hi, 1), rhi = __shfl_down_sync(0xffffffffu, hi, 1);
+            m = med3f(fmaxf(fmaxf(llo, lo), rlo), med3f(lmid, mid, rmid), fminf(fminf(lhi, hi), rhi));
+        } else {
+            const float p0 = __shfl_up_sync(0xffffffffu, v[k], 1), p2 = __shfl_down_sync(0xffffffffu, v[k], 1);
+            const float p3 = __shfl_up_sync(0xffffffffu, v[k + 1], 1), p5 = __shfl_down_sync(0xffffffffu, v[k + 1], 1);
+            const float p6 = __shfl_up_sync(0xffffffffu, v[k + 2], 1), p8 = __shfl_down_sync(0xffffffffu, v[k + 2], 1);
+            if (H == 1) m = cv_median3_line(p3, v[k + 1], p5);
+            else if (W == 1) m = cv_median3_line(v[k], v[k + 1], v[k + 2]);
+            else m = cv_median9(cv_vector_column(c, W), p0, v[k], p2, p3, v[k + 1], p5, p6, v[k + 2], p8);
+        }
+        if (store) dst[static_cast<long long>(r) * W] = m;
+    }
+}
+
+template <typename T>
+int launch_blur(const T *in, float *out, long long h, long long w, long long n_img, cudaStream_t st) {
+    const long long strips = ceil_div(h, kBlurRows), groups = ceil_div(w, kBlurCols), warps = n_img * strips * groups;
+    const unsigned blocks = static_cast<unsigned>(ceil_div(warps, 8));
+    const long long small = (1LL << 31) - 64;
+    if (h < small && w < small && warps < small)
+        median_blur3x3_kernel<T, int><<<blocks, 256, 0, st>>>(in, out, static_cast<int>(h), static_cast<int>(w),
+                                                              static_cast<int>(strips), static_cast<int>(groups),
+                                                              static_cast<int>(warps));
+    else
+        median_blur3x3_kernel<T, long long><<<blocks, 256, 0, st>>>(in, out, h, w, strips, groups, warps);
+    return check_launch("median_blur3x3_kernel");
 }
 
 // ---- fused produce_dsm epilogue: keys -> nanmax -> hole fill -> float32 -> blur ---------
@@ -611,26 +677,39 @@ struct EpilogueSmem {
 // concurrently, so no per-view memset is needed.  Empty cells (a few percent) are
 // collected in a shared list and filled by consecutive threads, so the hole-fill work does
 // not diverge every warp that happens to hold one.
-template <class Dec>
+// AHEAD: all of a thread's keys are loaded before the first is used -- the ballots order the steps,
+// and one load per step makes a tile wait for L2 six times (1503 x 1409 cells: 21.5 us,
+// 19.5 us; needs 40 registers, which raster_pipe_kernel's tiles do not have).
+template <bool AHEAD, class Dec>
 __device__ __forceinline__ void epilogue_tile(const unsigned long long *__restrict__ vk, const Dec &dec,
                                               float *__restrict__ out, unsigned long long *__restrict__ next_keys,
                                               int H, int W, int r0, int c0, EpilogueSmem &sm) {
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx, lane = tid & 31;
     bool special = false;          // this thread staged a NaN or a zero
     if (tid == 0) sm.n_holes = 0;
-    __syncthreads();
     // one pass over the key block: stage the keys (the hole fill reads the neighbours) and,
     // for the blur input's cells, the float32 values and the list of empty cells
-    for (int base = 0; base < RAW_H * RAW_W; base += TX * TY) {
-        const int i = base + tid;
+    constexpr int kSteps = (RAW_H * RAW_W + TX * TY - 1) / (TX * TY), kGroup = AHEAD ? kSteps : 1;
+    unsigned long long key[kGroup];
+#pragma unroll(kGroup)
+    for (int q = 0; q < kSteps; ++q) {
+        const int i = q * (TX * TY) + tid;
         const bool in = i < RAW_H * RAW_W;
         const int ly = i / RAW_W, lx = i - ly * RAW_W;
-        const int r = r0 + ly - 2, c = c0 + lx - 2;
-        unsigned long long k = kEmptyKey;
-        if (in && static_cast<unsigned>(r) < static_cast<unsigned>(H) && static_cast<unsigned>(c) < static_cast<unsigned>(W)) {
-            const long long cell = static_cast<long long>(r) * W + c;
-            k = dec(vk[cell], cell);
+        if (q % kGroup == 0) {
+#pragma unroll
+            for (int g = 0; g < kGroup; ++g) {
+                const int j = (q + g) * (TX * TY) + tid, jy = j / RAW_W, jx = j - jy * RAW_W;
+                const int r = r0 + jy - 2, c = c0 + jx - 2;
+                key[g] = kEmptyKey;
+                if (j < RAW_H * RAW_W && static_cast<unsigned>(r) < static_cast<unsigned>(H) &&
+                    static_cast<unsigned>(c) < static_cast<unsigned>(W))
+                    key[g] = vk[static_cast<long long>(r) * W + c];
+            }
+            if (q == 0) __syncthreads();             // n_holes
         }
+        unsigned long long k = key[q % kGroup];
+        if (k == kZeroKey) k = dec(k, static_cast<long long>(r0 + ly - 2) * W + (c0 + lx - 2));
         if (in) sm.raw[i] = k;
         const bool inner = in && ly >= 1 && ly <= RAW_H - 2 && lx >= 1 && lx <= RAW_W - 2;
         if (inner && k != kEmptyKey) {
@@ -741,7 +820,7 @@ __global__ void __launch_bounds__(TX *TY) dsm_epilogue_kernel(
     const double *__restrict__ pts, float *__restrict__ out, unsigned long long *__restrict__ next_keys, int H,
     int W) {
     __shared__ EpilogueSmem sm;
-    epilogue_tile(vk, PointsZeroDecoder{first, pts}, out, next_keys, H, W, blockIdx.y * TILE_Y, blockIdx.x * TX, sm);
+    epilogue_tile<true>(vk, PointsZeroDecoder{first, pts}, out, next_keys, H, W, blockIdx.y * TILE_Y, blockIdx.x * TX, sm);
 }
 
 // ---- pipelined rasterisation: view v's binning and view v-1's epilogue in one launch -----
@@ -805,7 +884,7 @@ __global__ void __launch_bounds__(TX *TY, MINB) raster_pipe_kernel(const double 
         if (code >= total) break;
         if (code >= 0) {
             const int ty = static_cast<int>(code / epi.tiles_x), tx = static_cast<int>(code - static_cast<long long>(ty) * epi.tiles_x);
-            epilogue_tile(epi.keys, PointsZeroDecoder{epi.first, pts}, epi.out, epi.clear, epi.H, epi.W, ty * TILE_Y,
+            epilogue_tile<false>(epi.keys, PointsZeroDecoder{epi.first, pts}, epi.out, epi.clear, epi.H, epi.W, ty * TILE_Y,
                           tx * TX, sm);
         } else {
             const long long c0 = begin + (-1 - code) * kChunkPoints;
@@ -830,7 +909,9 @@ long long host_threshold(long long r, double ulp, double res) {
     return d;
 }
 
-int make_axis(Axis &ax, double off, double res, long long n, int dir, long long *thr, cudaStream_t st) {
+// The axis's constants; `job` receives its threshold table's (n < 0 when the fast path does not apply).
+void make_axis(Axis &ax, double off, double res, long long n, int dir, long long *thr, ThresholdJob &job) {
+    job = {thr, -1, 0.0, 0.0};
     ax.off = off;
     ax.res = res;
     ax.n = n;
@@ -850,10 +931,10 @@ int make_axis(Axis &ax, double off, double res, long long n, int dir, long long 
     ax.mul = ax.fmask = ax.fsure = 0;
     ax.fbits = 0;
     // the FP32 estimate needs cell indices below 2^22 and sane resolutions
-    if (!(e >= 1 && e <= 2046 && isfinite(res) && res >= 1e-9 && res <= 1e9 && n < (1LL << 22))) return VS_OK;
+    if (!(e >= 1 && e <= 2046 && isfinite(res) && res >= 1e-9 && res <= 1e9 && n < (1LL << 22))) return;
     const double ulp = ldexp(1.0, static_cast<int>(e) - 1075);
     const double dmax = static_cast<double>(n + 1) * res / ulp + 2.0;   // > thr[n]
-    if (dmax >= 4503599627370496.0) return VS_OK;                       // differences below 2^52 ulps
+    if (dmax >= 4503599627370496.0) return;                       // differences below 2^52 ulps
     int bits = 0;
     frexp(dmax, &bits);                              // dmax < 2^bits
     ax.shift = bits > 32 ? bits - 32 : 0;            // d >> shift < 2^32
@@ -873,7 +954,7 @@ int make_axis(Axis &ax, double off, double res, long long n, int dir, long long 
         --fb;
         m = nearbyint(ldexp(scale, 32 + fb));
     }
-    if (fb < 4 || fb > 31 || m < 2147483648.0 || m >= 4294967296.0) return VS_OK;   // (cannot happen for n < 2^22)
+    if (fb < 4 || fb > 31 || m < 2147483648.0 || m >= 4294967296.0) return;   // (cannot happen for n < 2^22)
     ax.mul = static_cast<unsigned>(m);
     ax.fbits = fb;
     ax.fmask = (1u << fb) - 1u;
@@ -887,8 +968,13 @@ int make_axis(Axis &ax, double off, double res, long long n, int dir, long long 
     memcpy(&bf, &far, sizeof bf);
     memcpy(&bn, &near, sizeof bn);
     ax.contained = (bf >> 52) == (b >> 52) && (bn >> 52) == (b >> 52);
-    const int threads = 256;
-    axis_thresholds_kernel<<<static_cast<unsigned>(ceil_div(n + 1, threads)), threads, 0, st>>>(thr, n, ulp, res);
+    job = {thr, n, ulp, res};
+}
+
+int launch_thresholds(const ThresholdJob &row, const ThresholdJob &col, cudaStream_t st) {
+    const long long total = (row.n + 1) + (col.n + 1);
+    if (total <= 0) return VS_OK;
+    axis_thresholds_kernel<<<static_cast<unsigned>(ceil_div(total, 64)), 64, 0, st>>>(row, col);
     return check_launch("axis_thresholds_kernel");
 }
 
@@ -896,16 +982,17 @@ struct RasterWs {
     unsigned long long *keys[2];   // key grids, alternating view by view
     unsigned long long *first;     // "first zero" words (epoch-tagged)
     long long *row_thr, *col_thr;
-    size_t bytes;
+    size_t bytes, cleared;         // of the whole, and of its start that a call clears
 };
 
 RasterWs carve_raster(void *ws, long long xsize, long long ysize, bool two_grids) {
     Carver cv(ws);
     RasterWs r;
     const size_t cells = static_cast<size_t>(xsize) * ysize;
-    r.keys[0] = cv.take<unsigned long long>(cells);
-    r.keys[1] = two_grids ? cv.take<unsigned long long>(cells) : r.keys[0];
+    r.keys[0] = cv.take<unsigned long long>(cells);      // keys[0] and first: cleared as one range
     r.first = cv.take<unsigned long long>(cells);
+    r.cleared = cv.used;
+    r.keys[1] = two_grids ? cv.take<unsigned long long>(cells) : r.keys[0];
     r.row_thr = cv.take<long long>(ysize + 1);
     r.col_thr = cv.take<long long>(xsize + 1);
     r.bytes = cv.used;
@@ -914,10 +1001,11 @@ RasterWs carve_raster(void *ws, long long xsize, long long ysize, bool two_grids
 
 int make_tables(double xoff, double yoff, double xres, double yres, long long xsize, long long ysize,
                 RasterWs &w, Tables &tb, cudaStream_t st) {
-    int s;
     // rows: a = yoff - y divided by xresolution; cols: a = x - xoff divided by yresolution
-    if ((s = make_axis(tb.row, yoff, xres, ysize, -1, w.row_thr, st)) != VS_OK) return s;
-    return make_axis(tb.col, xoff, yres, xsize, +1, w.col_thr, st);
+    ThresholdJob row, col;
+    make_axis(tb.row, yoff, xres, ysize, -1, w.row_thr, row);
+    make_axis(tb.col, xoff, yres, xsize, +1, w.col_thr, col);
+    return launch_thresholds(row, col, st);
 }
 
 // CTAs per SM of the point-binning launches (0: as many as fit); set through
@@ -1446,11 +1534,7 @@ int clear(void *p, size_t bytes, cudaStream_t st) {
 }  // namespace
 
 int launch_blur_f32(const float *in, float *out, long long h, long long w, cudaStream_t st) {
-    const long long total = h * w;
-    const int threads = 256;
-    unsigned g = static_cast<unsigned>(std::min<long long>(ceil_div(total, threads), sm_count() * 16LL));
-    median_blur3x3_kernel<float><<<g, threads, 0, st>>>(in, out, h, w, total);
-    return check_launch("median_blur3x3_kernel<float>");
+    return launch_blur(in, out, h, w, 1, st);
 }
 
 }  // namespace vs
@@ -1459,7 +1543,7 @@ using namespace vs;
 
 extern "C" size_t vs_proj_to_grid_workspace_size(int64_t xsize, int64_t ysize) {
     if (xsize <= 0 || ysize <= 0) return 0;
-    return carve_raster(nullptr, xsize, ysize, false).bytes + sizeof(double) * xsize * ysize + 512;
+    return carve_raster(nullptr, xsize, ysize, false).bytes + 256;
 }
 
 static bool grid_ok(int64_t xsize, int64_t ysize) {
@@ -1479,22 +1563,15 @@ extern "C" int vs_proj_to_grid(const double *points, int64_t n, double xoff, dou
     }
     cudaStream_t st = as_stream(stream);
     RasterWs w = carve_raster(workspace, xsize, ysize, false);
-    Carver cv(workspace);
-    cv.used = w.bytes;
-    double *nanmax = cv.take<double>(static_cast<size_t>(xsize) * ysize);
     Tables tb;
-    const long long cells = xsize * ysize;
     int s = make_tables(xoff, yoff, xresolution, yresolution, xsize, ysize, w, tb, st);
-    if (s == VS_OK) s = clear(w.keys[0], sizeof(unsigned long long) * cells, st);
-    if (s == VS_OK) s = clear(w.first, sizeof(unsigned long long) * cells, st);
+    if (s == VS_OK) s = clear(w.keys[0], w.cleared, st);
     if (s == VS_OK) s = bin_launch(points, nullptr, 0, n, n, tb, w.keys[0], w.first, st);
     if (s != VS_OK) return s;
-    const int threads = 256;
-    unsigned g = static_cast<unsigned>(std::min<long long>(ceil_div(cells, threads), sm_count() * 16LL));
-    decode_kernel<<<g, threads, 0, st>>>(w.keys[0], w.first, points, nanmax, cells);
-    VS_LAUNCH_CHECK("decode_kernel");
-    hole_fill_kernel<<<g, threads, 0, st>>>(nanmax, dsm, ysize, xsize, cells);
-    VS_LAUNCH_CHECK("hole_fill_kernel");
+    const dim3 grid(static_cast<unsigned>(ceil_div(xsize, kGridTile)), static_cast<unsigned>(ceil_div(ysize, kGridTile)));
+    grid_f64_kernel<<<grid, kGridThreads, 0, st>>>(w.keys[0], w.first, points, dsm, static_cast<int>(ysize),
+                                                   static_cast<int>(xsize));
+    VS_LAUNCH_CHECK("grid_f64_kernel");
     return VS_OK;
 }
 
@@ -1520,8 +1597,7 @@ extern "C" int vs_dsm_from_points(const double *points, const int64_t *offsets, 
     Tables tb;
     const long long cells = xsize * ysize;
     int s = make_tables(xoff, yoff, xresolution, yresolution, xsize, ysize, w, tb, st);
-    if (s == VS_OK) s = clear(w.keys[0], sizeof(unsigned long long) * cells, st);
-    if (s == VS_OK) s = clear(w.first, sizeof(unsigned long long) * cells, st);
+    if (s == VS_OK) s = clear(w.keys[0], w.cleared, st);
     if (s != VS_OK) return s;
     // per-view counts live on the device: launch for a full GPU and let the grid stride
     const long long launch_points = static_cast<long long>(sm_count()) * 8 * 256 * kPts;
@@ -1548,15 +1624,17 @@ struct OverlapWs {
     unsigned long long *keys[3];
     unsigned long long *first[2];
     long long *row_thr, *col_thr;
-    size_t bytes;
+    size_t bytes, cleared;
 };
 
 OverlapWs carve_overlap(void *ws, long long xsize, long long ysize) {
     Carver cv(ws);
     OverlapWs r;
     const size_t cells = static_cast<size_t>(xsize) * ysize;
-    for (auto &k : r.keys) k = cv.take<unsigned long long>(cells);
+    for (int i = 0; i < 2; ++i) r.keys[i] = cv.take<unsigned long long>(cells);
     for (auto &f : r.first) f = cv.take<unsigned long long>(cells);
+    r.cleared = cv.used;                                 // all but keys[2], which an epilogue clears
+    r.keys[2] = cv.take<unsigned long long>(cells);
     r.row_thr = cv.take<long long>(ysize + 1);
     r.col_thr = cv.take<long long>(xsize + 1);
     r.bytes = cv.used;
@@ -1635,8 +1713,7 @@ extern "C" int vs_dsm_from_points_host(const double *host_points, const int64_t 
     Tables tb;
     const long long cells = xsize * ysize;
     int s = make_tables(xoff, yoff, xresolution, yresolution, xsize, ysize, w, tb, st);
-    if (s == VS_OK) s = clear(w.keys[0], sizeof(unsigned long long) * cells, st);
-    if (s == VS_OK) s = clear(w.first, sizeof(unsigned long long) * cells, st);
+    if (s == VS_OK) s = clear(w.keys[0], w.cleared, st);
     if (s != VS_OK) return s;
     cudaEvent_t freed[8], landed[8];
     int made = 0;
@@ -1722,8 +1799,7 @@ extern "C" int vs_dsm_from_points_overlap(const double *points, const int64_t *o
     Tables tb;
     const long long cells = xsize * ysize;
     s = make_tables(xoff, yoff, xresolution, yresolution, xsize, ysize, tw, tb, st);
-    for (int i = 0; i < 2 && s == VS_OK; ++i) s = clear(w.keys[i], sizeof(unsigned long long) * cells, st);
-    for (int i = 0; i < 2 && s == VS_OK; ++i) s = clear(w.first[i], sizeof(unsigned long long) * cells, st);
+    if (s == VS_OK) s = clear(w.keys[0], w.cleared, st);
     if (s != VS_OK) return s;
     const long long launch_points = static_cast<long long>(sm_count()) * 8 * 256 * kPts;
     const dim3 egrid(static_cast<unsigned>(ceil_div(xsize, TX)), static_cast<unsigned>(ceil_div(ysize, TILE_Y)));
@@ -1806,8 +1882,7 @@ extern "C" int vs_dsm_from_points_pipelined(const double *points, const int64_t 
     Tables tb;
     const long long cells = xsize * ysize;
     int s = make_tables(xoff, yoff, xresolution, yresolution, xsize, ysize, tw, tb, st);
-    for (int i = 0; i < 2 && s == VS_OK; ++i) s = clear(w.keys[i], sizeof(unsigned long long) * cells, st);
-    for (int i = 0; i < 2 && s == VS_OK; ++i) s = clear(w.first[i], sizeof(unsigned long long) * cells, st);
+    if (s == VS_OK) s = clear(w.keys[0], w.cleared, st);
     if (s == VS_OK) s = clear(counters, sizeof(unsigned) * (static_cast<size_t>(n_views) + 1), st);
     if (s != VS_OK) return s;
     const int tiles_x = static_cast<int>(ceil_div(xsize, TX));
@@ -1890,23 +1965,13 @@ extern "C" int vs_dsm_from_points_pipelined(const double *points, const int64_t 
 extern "C" int vs_median_blur3x3_f32(const float *in, float *out, int64_t h, int64_t w, int64_t n_img,
                                      void *stream) {
     VS_REQUIRE(h > 0 && w > 0 && n_img > 0 && in && out && in != out, "vs_median_blur3x3_f32: bad arguments");
-    const long long total = h * w * n_img;
-    const int threads = 256;
-    unsigned g = static_cast<unsigned>(std::min<long long>(ceil_div(total, threads), sm_count() * 16LL));
-    median_blur3x3_kernel<float><<<g, threads, 0, as_stream(stream)>>>(in, out, h, w, total);
-    VS_LAUNCH_CHECK("median_blur3x3_kernel<float>");
-    return VS_OK;
+    return launch_blur(in, out, h, w, n_img, as_stream(stream));
 }
 
 extern "C" int vs_median_blur3x3_f64(const double *in, float *out, int64_t h, int64_t w, int64_t n_img,
                                      void *stream) {
     VS_REQUIRE(h > 0 && w > 0 && n_img > 0 && in && out, "vs_median_blur3x3_f64: bad arguments");
-    const long long total = h * w * n_img;
-    const int threads = 256;
-    unsigned g = static_cast<unsigned>(std::min<long long>(ceil_div(total, threads), sm_count() * 16LL));
-    median_blur3x3_kernel<double><<<g, threads, 0, as_stream(stream)>>>(in, out, h, w, total);
-    VS_LAUNCH_CHECK("median_blur3x3_kernel<double>");
-    return VS_OK;
+    return launch_blur(in, out, h, w, n_img, as_stream(stream));
 }
 
 // ---- batched form: plan and run ------------------------------------------------------------
@@ -2020,10 +2085,12 @@ extern "C" int vs_aoi_batch_plan(const VsAoi *aois, int n_aois, const VsMapView 
         }
         expect_view += A.n_views;
         Tables tb;
-        int s = make_axis(tb.row, A.yoff, A.xres, A.ysize, -1, thr, st);
+        ThresholdJob row, col;
+        make_axis(tb.row, A.yoff, A.xres, A.ysize, -1, thr, row);
         thr += A.ysize + 1;
-        if (s == VS_OK) s = make_axis(tb.col, A.xoff, A.yres, A.xsize, +1, thr, st);
+        make_axis(tb.col, A.xoff, A.yres, A.xsize, +1, thr, col);
         thr += A.xsize + 1;
+        const int s = launch_thresholds(row, col, st);
         if (s != VS_OK) return fail(s);
         if (!(tb.row.fast && tb.row.contained && tb.col.fast && tb.col.contained)) {
             set_error("vs_aoi_batch_plan: AOI %d: grid extent crosses a power of two of its origin", a);
@@ -2313,7 +2380,7 @@ __global__ void __launch_bounds__(TX *TY) depth_epilogue_kernel(const unsigned l
                                                                unsigned long long *__restrict__ next_keys, int H,
                                                                int W) {
     __shared__ EpilogueSmem sm;
-    epilogue_tile(vk, SignZeroDecoder{first}, out, next_keys, H, W, blockIdx.y * TILE_Y, blockIdx.x * TX, sm);
+    epilogue_tile<true>(vk, SignZeroDecoder{first}, out, next_keys, H, W, blockIdx.y * TILE_Y, blockIdx.x * TX, sm);
 }
 
 }  // namespace
@@ -2352,8 +2419,7 @@ extern "C" int vs_dsm_from_depth_maps(const float *const *depths, const int64_t 
     if (s != VS_OK) return s;
     VS_REQUIRE(tb.row.fast && tb.row.contained && tb.col.fast && tb.col.contained && xoff > 0 && yoff > 0,
                "vs_dsm_from_depth_maps: the grid must be positive and inside its origins' binades");
-    if ((s = clear(w.keys[0], sizeof(unsigned long long) * cells, st)) != VS_OK) return s;
-    if ((s = clear(w.first, sizeof(unsigned long long) * cells, st)) != VS_OK) return s;
+    if ((s = clear(w.keys[0], w.cleared, st)) != VS_OK) return s;
     const FastAxis fr = fast_axis_of(tb.row), fc = fast_axis_of(tb.col);
     const GeoFast &gf = geo_plan_fast(plan);
     const GeoFrame *gfr = geo_plan_frame(plan);
