@@ -132,10 +132,9 @@ PIPE_TRAFFIC = None
 
 def launches_per_step(views, piped=False):
     # kernels only (memsets are not kernels); checked against the ncu launch list
-    camera = 15        # bbox init, bbox, norm, prepare, project, moments, solve, error points, error count,
-    #                    select step x3, select histogram x2, error final
-    # thresholds x2; per view: bin, epilogue -- or, pipelined, views + 1 launches
-    raster = 2 + (views + 1 if piped else views * 2)
+    camera = 11        # bbox, prepare, project, moments, solve, error points, select step x3, histogram x2
+    # thresholds; per view: bin, epilogue -- or, pipelined, views + 1 launches
+    raster = 1 + (views + 1 if piped else views * 2)
     fusion = 2               # fuse + blur
     return camera + raster + fusion
 

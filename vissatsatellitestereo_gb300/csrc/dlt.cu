@@ -87,52 +87,6 @@ struct Norm {
 // coordinate array, and 8192 of them bound the data's extent well enough for scaling.
 constexpr int kBoxSamples = 8192;
 
-// Min/max of x, y, z (and col, row when given) over a strided sample of the kept points,
-// as order-preserving keys (the min through the complemented key).  Any centre and scale
-// serve the normalisation; it only has to keep the moments well scaled.
-__global__ void bbox_init_kernel(unsigned long long *bb, int n_views) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n_views * 10) bb[i] = 0ull;
-}
-
-__global__ void __launch_bounds__(256) bbox_kernel(const double *__restrict__ x, const double *__restrict__ y,
-                                                   const double *__restrict__ z, long long xyz_stride,
-                                                   const double *__restrict__ col, const double *__restrict__ row,
-                                                   const uint8_t *__restrict__ keep, long long n, long long step,
-                                                   unsigned long long *__restrict__ bb) {
-    const int v = blockIdx.y;
-    const double *src[5] = {x + v * xyz_stride, y + v * xyz_stride, z + v * xyz_stride, col ? col + v * n : nullptr,
-                            row ? row + v * n : nullptr};
-    unsigned long long hi[5], lo[5];
-#pragma unroll
-    for (int j = 0; j < 5; ++j) hi[j] = lo[j] = 0ull;
-    for (long long i = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) * step; i < n;
-         i += static_cast<long long>(gridDim.x) * blockDim.x * step) {
-        if (keep && !keep[v * n + i]) continue;
-#pragma unroll
-        for (int j = 0; j < 5; ++j) {
-            if (!src[j]) continue;
-            const unsigned long long k = key_from_double(src[j][i]);
-            hi[j] = max(hi[j], k);
-            lo[j] = max(lo[j], ~k);
-        }
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-        for (int j = 0; j < 5; ++j) {
-            hi[j] = max(hi[j], __shfl_xor_sync(0xffffffffu, hi[j], off));
-            lo[j] = max(lo[j], __shfl_xor_sync(0xffffffffu, lo[j], off));
-        }
-    if ((threadIdx.x & 31) == 0) {
-        unsigned long long *b = bb + v * 10;
-        for (int j = 0; j < 5; ++j) {
-            if (hi[j]) atomicMax(b + j, hi[j]);
-            if (lo[j]) atomicMax(b + 5 + j, lo[j]);
-        }
-    }
-}
-
 __device__ __forceinline__ double finite_or(double v, double fallback) {
     return (isfinite(v)) ? v : fallback;
 }
@@ -156,28 +110,23 @@ __device__ __forceinline__ NormF make_normf(const Norm &nm) {
     return f;
 }
 
-// Normalisation from the sampled boxes.  For the fused camera path the pixel frame is the
-// RPC's own (colOff/rowOff, larger scale).
-__global__ void norm_kernel(const unsigned long long *__restrict__ bb, const VsRpcCamera *__restrict__ cams,
-                            int n_views, Norm *__restrict__ norm, NormF *__restrict__ normf) {
-    int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= n_views) return;
-    const unsigned long long *b = bb + v * 10;
+// Normalisation of one view from its sampled box.  For the fused camera path the pixel frame
+// is the RPC's own (colOff/rowOff, larger scale).
+__device__ __forceinline__ void make_norm(const unsigned long long *b, const VsRpcCamera *cam, Norm &nm) {
     double mx[5], mn[5];
     for (int j = 0; j < 5; ++j) {
         mx[j] = b[j] ? double_from_key(b[j]) : 0.0;
         mn[j] = b[5 + j] ? double_from_key(~b[5 + j]) : 0.0;
     }
-    Norm nm;
     nm.cx = finite_or(0.5 * (mn[0] + mx[0]), 0.0);
     nm.cy = finite_or(0.5 * (mn[1] + mx[1]), 0.0);
     nm.cz = finite_or(0.5 * (mn[2] + mx[2]), 0.0);
     double s = fmax(fmax(mx[0] - mn[0], mx[1] - mn[1]), mx[2] - mn[2]) * 0.5;
     nm.s = (s > 0.0 && isfinite(s)) ? s : 1.0;
-    if (cams) {
-        nm.c0 = cams[v].col_off;
-        nm.r0 = cams[v].row_off;
-        nm.sp = fmax(fabs(cams[v].col_scale), fabs(cams[v].row_scale));
+    if (cam) {
+        nm.c0 = cam->col_off;
+        nm.r0 = cam->row_off;
+        nm.sp = fmax(fabs(cam->col_scale), fabs(cam->row_scale));
         if (!(nm.sp > 0.0) || !isfinite(nm.sp)) nm.sp = 1.0;
     } else {
         nm.c0 = finite_or(0.5 * (mn[3] + mx[3]), 0.0);
@@ -185,6 +134,75 @@ __global__ void norm_kernel(const unsigned long long *__restrict__ bb, const VsR
         double sp = fmax(mx[3] - mn[3], mx[4] - mn[4]) * 0.5;
         nm.sp = (sp > 0.0 && isfinite(sp)) ? sp : 1.0;
     }
+}
+
+// The box of one view: order-preserving keys of the largest values, then of the smallest (the
+// keys' complements), and the number of blocks that have added theirs.  All zero to begin with.
+struct Box {
+    unsigned long long key[10];
+    unsigned done, pad;
+};
+
+// Min/max of x, y, z (and col, row when given) over a strided sample of the kept points, and
+// from them the view's normalisation: any centre and scale serve, it only has to keep the
+// moments well scaled.  The last block of a view to add its box computes the normalisation, which was
+// a launch of its own.  (50 views: 35 us of strided sectors; neither fewer blocks, nor one atomic per
+// block, nor four samples in flight per thread changes that.)
+__global__ void __launch_bounds__(256) bbox_kernel(const double *__restrict__ x, const double *__restrict__ y,
+                                                   const double *__restrict__ z, long long xyz_stride,
+                                                   const double *__restrict__ col, const double *__restrict__ row,
+                                                   const uint8_t *__restrict__ keep, long long n, long long step,
+                                                   const VsRpcCamera *__restrict__ cams, Box *__restrict__ boxes,
+                                                   Norm *__restrict__ norm, NormF *__restrict__ normf) {
+    __shared__ unsigned long long best[10];
+    chain_wait();
+    const int v = blockIdx.y;
+    const double *src[5] = {x + v * xyz_stride, y + v * xyz_stride, z + v * xyz_stride, col ? col + v * n : nullptr,
+                            row ? row + v * n : nullptr};
+    if (threadIdx.x < 10) best[threadIdx.x] = 0ull;
+    __syncthreads();
+    unsigned long long hi[5], lo[5];
+#pragma unroll
+    for (int j = 0; j < 5; ++j) hi[j] = lo[j] = 0ull;
+    for (long long i = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) * step; i < n;
+         i += static_cast<long long>(gridDim.x) * blockDim.x * step) {
+        if (keep && !keep[v * n + i]) continue;
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+            if (!src[j]) continue;
+            const unsigned long long k = key_from_double(src[j][i]);
+            hi[j] = max(hi[j], k);
+            lo[j] = max(lo[j], ~k);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 5; ++j) {
+        if (!src[j]) continue;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            hi[j] = max(hi[j], __shfl_xor_sync(0xffffffffu, hi[j], off));
+            lo[j] = max(lo[j], __shfl_xor_sync(0xffffffffu, lo[j], off));
+        }
+        if ((threadIdx.x & 31) == 0) {
+            atomicMax(best + j, hi[j]);
+            atomicMax(best + 5 + j, lo[j]);
+        }
+    }
+    __syncthreads();
+    Box &box = boxes[v];
+    if (threadIdx.x < 10 && best[threadIdx.x]) {
+        atomicMax(box.key + threadIdx.x, best[threadIdx.x]);
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(&box.done, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    unsigned long long k[10];
+    for (int j = 0; j < 10; ++j) k[j] = atomicAdd(box.key + j, 0ull);
+    Norm nm;
+    make_norm(k, cams ? cams + v : nullptr, nm);
     norm[v] = nm;
     normf[v] = make_normf(nm);     // once per view: the per-point kernels read it (no FP64 there)
 }
@@ -273,6 +291,7 @@ __global__ void __launch_bounds__(kMomThreads, 6) moments_kernel(
     const uint8_t *__restrict__ keep, const float *__restrict__ wh, long long n, const NormF *__restrict__ normf,
     double *__restrict__ partial) {
     __shared__ double red[(kMomThreads / 32) * kSlots];
+    chain_wait();
     const int v = blockIdx.y;
     const NormF nf = normf[v];
     const double *xv = x + v * xyz_stride, *yv = y + v * xyz_stride, *zv = z + v * xyz_stride;
@@ -338,6 +357,7 @@ __global__ void __launch_bounds__(kMomThreads, 6) moments_kernel(
 __global__ void __launch_bounds__(64) prepare_views_kernel(const VsRpcCamera *__restrict__ cams,
                                                            RpcFast *__restrict__ fast, float *__restrict__ wh) {
     const int v = blockIdx.x;
+    chain_wait();
     prepare_fast(cams[v], fast[v]);
     if (threadIdx.x == 0) {
         wh[2 * v] = fast[v].width;
@@ -357,6 +377,7 @@ __global__ void __launch_bounds__(256) project_view_kernel(const VsRpcCamera *__
     constexpr bool kExact = MODE == VS_PROJ_EXACT;
     __shared__ typename CameraOf<MODE>::type cam;
     const int v = blockIdx.y;
+    chain_wait();
     if constexpr (kExact) {
         load_exact(cams + v, cam);
     } else {
@@ -403,42 +424,56 @@ __global__ void __launch_bounds__(256) project_view_kernel(const VsRpcCamera *__
     }
 }
 
-// ---- 12x12 solve (one thread per view; FP64) -------------------------------------------
-struct Mmap {     // the exact map between normalised (q) and original (p) camera vectors
-    double cx, cy, cz, s, c0, r0, sp;
-};
+// ---- 12x12 solve (one warp per view; FP64) ---------------------------------------------
+// The exact map M between normalised (q) and original (p) camera vectors: q1 = T^T(p1 - c0
+// p3)/sp, q2 = T^T(p2 - r0 p3)/sp, q3 = T^T p3, T = [[s,0,0,cx],[0,s,0,cy],[0,0,s,cz],[0,0,0,1]].
+//
+// One warp: FP64 latency and divisions are all of its time, so lane l < 12 holds component l of the
+// vectors (component i = l mod 4 of row b = l / 4) and row l of the factor, and the divisions,
+// which were one after the other in one lane, run side by side; those by a pivot or a scale, which
+// repeat each iteration, use its reciprocal (div_known: 4 operations, the same bits).  Every
+// element sees the operations of the serial form in its order.  One view: 175 us, 96 us, of which about
+// 50 us are FP64 latency (59 cycles an operation, 600 a division or square root).
 
-// u = T^-1 w, T = [[s,0,0,cx],[0,s,0,cy],[0,0,s,cz],[0,0,0,1]]
-__device__ __forceinline__ void t_inv(const Mmap &m, const double *w, double *u) {
-    u[0] = (w[0] - m.cx * w[3]) / m.s;
-    u[1] = (w[1] - m.cy * w[3]) / m.s;
-    u[2] = (w[2] - m.cz * w[3]) / m.s;
-    u[3] = w[3];
+// A divisor and whether its quotients may take the reciprocal form.
+struct LaneDivisor {
+    Divisor d;
+    bool known;
+};
+// Exponent within 2^+-160 (no zero): div_known has the bits of the division.
+__device__ __forceinline__ bool mid_range(double v) {
+    return ((static_cast<unsigned>(__double2hiint(v)) >> 20) & 0x7ffu) - (1023u - 160u) <= 320u;
 }
-// u = T^-T w
-__device__ __forceinline__ void tt_inv(const Mmap &m, const double *w, double *u) {
-    u[0] = w[0] / m.s;
-    u[1] = w[1] / m.s;
-    u[2] = w[2] / m.s;
-    u[3] = w[3] - m.cx * u[0] - m.cy * u[1] - m.cz * u[2];
+__device__ __forceinline__ LaneDivisor lane_divisor(double v) {
+    LaneDivisor r;
+    r.known = mid_range(v);
+    r.d = divisor_of(v);
+    return r;
 }
-// solve M^T u = v   (q = M p with q1 = T^T(p1 - c0 p3)/sp, q2 = T^T(p2 - r0 p3)/sp, q3 = T^T p3)
-__device__ void solve_mt(const Mmap &m, const double *v, double *u) {
-    double w[4];
-    t_inv(m, v, u);
-    t_inv(m, v + 4, u + 4);
-    for (int i = 0; i < 8; ++i) u[i] *= m.sp;
-    for (int i = 0; i < 4; ++i) w[i] = v[8 + i] + m.c0 * v[i] + m.r0 * v[4 + i];
-    t_inv(m, w, u + 8);
+__device__ __forceinline__ double lane_div(double v, const LaneDivisor &d) {
+    if (__all_sync(0xffffffffu, d.known && mid_range(v))) return div_known(v, d.d);
+    return __ddiv_rn(v, d.d.d);
 }
-// solve M u = v
-__device__ void solve_m(const Mmap &m, const double *v, double *u) {
-    double w[4];
-    tt_inv(m, v + 8, u + 8);
-    for (int i = 0; i < 4; ++i) w[i] = m.sp * v[i] + m.c0 * v[8 + i];
-    tt_inv(m, w, u);
-    for (int i = 0; i < 4; ++i) w[i] = m.sp * v[4 + i] + m.r0 * v[8 + i];
-    tt_inv(m, w, u + 4);
+__device__ __forceinline__ double lane_get(double v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+
+// u = M^-T v, component by component: rows 0 and 1 are sp T^-1 v_b, row 2 is T^-1 (v_2 + c0 v_0 + r0 v_1).
+__device__ __forceinline__ double solve_mt(const Norm &m, const LaneDivisor &ds, int b, int i, double v) {
+    const double v0 = lane_get(v, i), v1 = lane_get(v, 4 + i);
+    const double t0 = lane_get(v, 3), t1 = lane_get(v, 7), t2 = lane_get(v, 11);
+    const double wi = b < 2 ? v : __fma_rn(m.r0, v1, __fma_rn(m.c0, v0, v));
+    const double w3 = b == 0 ? t0 : (b == 1 ? t1 : __fma_rn(m.r0, t1, __fma_rn(m.c0, t0, t2)));
+    const double c = i == 0 ? m.cx : (i == 1 ? m.cy : m.cz);
+    const double q = lane_div(__fma_rn(-c, w3, wi), ds);
+    const double u = i < 3 ? q : wi;
+    return b < 2 ? __dmul_rn(u, m.sp) : u;
+}
+// u = M^-1 v: row 2 is T^-T v_2, rows 0 and 1 are T^-T (sp v_b + {c0, r0} v_2).
+__device__ __forceinline__ double solve_m(const Norm &m, const LaneDivisor &ds, int b, int i, double v) {
+    const double v2 = lane_get(v, 8 + i);
+    const double w = b == 2 ? v : __fma_rn(m.sp, v, __dmul_rn(b == 0 ? m.c0 : m.r0, v2));
+    const double q = lane_div(w, ds);
+    const double q0 = lane_get(q, 4 * b), q1 = lane_get(q, 4 * b + 1), q2 = lane_get(q, 4 * b + 2);
+    return i < 3 ? q : __fma_rn(-m.cz, q2, __fma_rn(-m.cy, q1, __fma_rn(-m.cx, q0, w)));
 }
 
 __device__ double det3(const double *a) {
@@ -478,15 +513,39 @@ __device__ void quaternion(const double *R, double *q) {
     for (int i = 0; i < 4; ++i) q[i] *= f;
 }
 
+// The camera of one view in shared memory.
+struct CameraSmem {
+    double P[12], K[9], R[9], t[3], u[12], q[12];
+};
+
 // Positive-diagonal RQ of the left 3x3 block of P by Gram-Schmidt from the last row (with
-// one re-orthogonalisation), then the reference's normalisations.  Returns a status.
-__device__ int factorize(double *P, double *K, double *R, double *t) {
+// one re-orthogonalisation), then the reference's normalisations.  The whole warp runs the scalar
+// parts; lanes share the divisions.  Returns a status; s.K, s.R, s.t are zero unless set.
+__device__ int factorize(CameraSmem &s, int lane) {
+    double P[12], K[9], R[9];
+    for (int i = 0; i < 12; ++i) P[i] = s.P[i];
     const double *a0 = P, *a1 = P + 4, *a2 = P + 8;
     double r0[3], r1[3], r2[3], u[3];
+    auto unit = [&](const double *a, double n, double *r) {        // r = a / n
+        const double q = (lane == 0 ? a[0] : (lane == 1 ? a[1] : a[2])) / n;
+        for (int i = 0; i < 3; ++i) r[i] = lane_get(q, i);
+    };
     for (int i = 0; i < 9; ++i) K[i] = 0.0;
+    auto store = [&](int st) {
+        __syncwarp();
+        if (lane < 9) {
+            double k = 0.0, r = 0.0;
+            for (int i = 0; i < 9; ++i) k = lane == i ? K[i] : k, r = lane == i ? R[i] : r;
+            s.K[lane] = k;
+            s.R[lane] = r;
+        }
+        __syncwarp();
+        return st;
+    };
+    for (int i = 0; i < 9; ++i) R[i] = 0.0;
     double n2 = sqrt(a2[0] * a2[0] + a2[1] * a2[1] + a2[2] * a2[2]);
-    if (!(n2 > 0.0) || !isfinite(n2)) return VS_ERR_DEGENERATE;
-    for (int i = 0; i < 3; ++i) r2[i] = a2[i] / n2;
+    if (!(n2 > 0.0) || !isfinite(n2)) return store(VS_ERR_DEGENERATE);
+    unit(a2, n2, r2);
     K[8] = n2;
     double k12 = a1[0] * r2[0] + a1[1] * r2[1] + a1[2] * r2[2];
     for (int i = 0; i < 3; ++i) u[i] = a1[i] - k12 * r2[i];
@@ -494,8 +553,8 @@ __device__ int factorize(double *P, double *K, double *R, double *t) {
     for (int i = 0; i < 3; ++i) u[i] -= d * r2[i];
     k12 += d;
     double n1 = sqrt(u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
-    if (!(n1 > 0.0)) return VS_ERR_DEGENERATE;
-    for (int i = 0; i < 3; ++i) r1[i] = u[i] / n1;
+    if (!(n1 > 0.0)) return store(VS_ERR_DEGENERATE);
+    unit(u, n1, r1);
     K[4] = n1;
     K[5] = k12;
     double k02 = a0[0] * r2[0] + a0[1] * r2[1] + a0[2] * r2[2];
@@ -507,33 +566,45 @@ __device__ int factorize(double *P, double *K, double *R, double *t) {
     k02 += d2;
     k01 += d1;
     double n0 = sqrt(u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
-    if (!(n0 > 0.0)) return VS_ERR_DEGENERATE;
-    for (int i = 0; i < 3; ++i) r0[i] = u[i] / n0;
+    if (!(n0 > 0.0)) return store(VS_ERR_DEGENERATE);
+    unit(u, n0, r0);
     K[0] = n0;
     K[1] = k01;
     K[2] = k02;
     for (int i = 0; i < 3; ++i) R[i] = r0[i], R[3 + i] = r1[i], R[6 + i] = r2[i];
-    // K /= K[2,2], P /= K[2,2]
-    const double sc = K[8];
-    for (int i = 0; i < 9; ++i) K[i] /= sc;
-    for (int i = 0; i < 12; ++i) P[i] /= sc;
+    // K /= K[2,2], P /= K[2,2]: lanes 0..11 P, 12..20 K
+    {
+        const double sc = K[8];
+        double x = sc;
+        for (int i = 0; i < 12; ++i) x = lane == i ? P[i] : x;
+        for (int i = 0; i < 9; ++i) x = lane == 12 + i ? K[i] : x;
+        x /= sc;
+        for (int i = 0; i < 12; ++i) P[i] = lane_get(x, i);
+        for (int i = 0; i < 9; ++i) K[i] = lane_get(x, 12 + i);
+    }
     if (det3(R) < 0.0) {
         for (int i = 0; i < 9; ++i) R[i] = -R[i];
         for (int i = 0; i < 12; ++i) P[i] = -P[i];
     }
     // t = K^-1 P[:, 3] (upper triangular)
+    double t[3];
     t[2] = P[11] / K[8];
-    t[1] = (P[7] - K[5] * t[2]) / K[4];
-    t[0] = (P[3] - K[1] * t[1] - K[2] * t[2]) / K[0];
+    t[1] = __dsub_rn(P[7], __dmul_rn(K[5], t[2])) / K[4];
+    t[0] = __dsub_rn(__dsub_rn(P[3], __dmul_rn(K[1], t[1])), __dmul_rn(K[2], t[2])) / K[0];
+    store(VS_OK);
+    if (lane < 3) s.t[lane] = lane == 0 ? t[0] : (lane == 1 ? t[1] : t[2]);
+    __syncwarp();
     // the reference's assertions: det R ~ 1 and K [R | t] ~ P
     if (!isclose(det3(R), 1.0)) return VS_ERR_FACTORIZE;
-    for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 4; ++j) {
-            double kr = 0.0;
-            for (int l = 0; l < 3; ++l) kr += K[3 * i + l] * (j < 3 ? R[3 * l + j] : t[l]);
-            if (!isclose(P[4 * i + j], kr)) return VS_ERR_FACTORIZE;
-        }
-    return VS_OK;
+    bool near = true;
+    if (lane < 12) {
+        const int i = lane / 4, j = lane - 4 * i;
+        double kr = 0.0, p = 0.0;
+        for (int l = 0; l < 3; ++l) kr += s.K[3 * i + l] * (j < 3 ? s.R[3 * l + j] : s.t[l]);
+        for (int k = 0; k < 12; ++k) p = lane == k ? P[k] : p;
+        near = isclose(p, kr);
+    }
+    return __all_sync(0xffffffffu, near) ? VS_OK : VS_ERR_FACTORIZE;
 }
 
 // What the error pass needs of one view's camera: the camera in the normalised frame
@@ -548,187 +619,197 @@ struct ErrCam {
     int ok;
 };
 
-__device__ void make_errcam(const double *K, const double *R, const double *t, const Norm &nm, float w, float h,
-                            int ok, ErrCam &ec) {
-    double P[12];
-    for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 4; ++j) {
-            double s = 0.0;
-            for (int l = 0; l < 3; ++l) s += K[3 * i + l] * (j < 3 ? R[3 * l + j] : t[l]);
-            P[4 * i + j] = s;
-        }
-    double u[3][4];
-    for (int i = 0; i < 3; ++i) {   // T^T p_i
-        const double *p = P + 4 * i;
-        u[i][0] = nm.s * p[0];
-        u[i][1] = nm.s * p[1];
-        u[i][2] = nm.s * p[2];
-        u[i][3] = nm.cx * p[0] + nm.cy * p[1] + nm.cz * p[2] + p[3];
+// One warp fills a view's ErrCam from the camera in s.K, s.R, s.t (lanes 0..11: element (i, j) of
+// the 3x4 matrices; the divisions side by side).
+__device__ void make_errcam(CameraSmem &s, const Norm &nm, const NormF &nf, float w, float h, int ok, ErrCam &ec,
+                            int lane) {
+    const int l = min(lane, 11), i = l / 4, j = l - 4 * i;
+    {
+        double p = 0.0;
+        for (int k = 0; k < 3; ++k) p += s.K[3 * i + k] * (j < 3 ? s.R[3 * k + j] : s.t[k]);
+        __syncwarp();
+        if (lane < 12) s.P[lane] = p;
+        __syncwarp();
     }
-    double q[12], mx = 0.0;
-    for (int j = 0; j < 4; ++j) {
-        q[j] = (u[0][j] - nm.c0 * u[2][j]) / nm.sp;
-        q[4 + j] = (u[1][j] - nm.r0 * u[2][j]) / nm.sp;
-        q[8 + j] = u[2][j];
+    {
+        const double *p = s.P + 4 * i;                 // T^T p_i
+        const double last = nm.cx * p[0] + nm.cy * p[1] + nm.cz * p[2] + p[3];
+        const double u = j < 3 ? nm.s * p[j] : last;
+        if (lane < 12) s.u[lane] = u;
+        __syncwarp();
     }
-    for (int i = 0; i < 12; ++i) mx = fmax(mx, fabs(q[i]));
+    const double uij = s.u[l], u2j = s.u[8 + j];
+    const double off = i == 0 ? nm.c0 : nm.r0;
+    const double quo = (uij - off * u2j) / nm.sp;
+    const double q = i < 2 ? quo : u2j;
+    double mx = fmax(0.0, fabs(q));
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, d));
     const double sc = (mx > 0.0 && isfinite(mx)) ? 1.0 / mx : 1.0;
-    for (int i = 0; i < 12; ++i) ec.q[i] = df_from_double(q[i] * sc);
-    for (int j = 0; j < 4; ++j) {
-        ec.q01_hi[j] = make_float2(ec.q[j].hi, ec.q[4 + j].hi);
-        ec.q01_lo[j] = make_float2(ec.q[j].lo, ec.q[4 + j].lo);
+    const df qd = df_from_double(q * sc);
+    const float hi1 = __shfl_sync(0xffffffffu, qd.hi, (l + 4) & 15), lo1 = __shfl_sync(0xffffffffu, qd.lo, (l + 4) & 15);
+    if (lane < 12) ec.q[lane] = qd;
+    if (lane < 4) {
+        ec.q01_hi[lane] = make_float2(qd.hi, hi1);
+        ec.q01_lo[lane] = make_float2(qd.lo, lo1);
     }
-    ec.qscale = static_cast<float>(sc);
-    ec.nf = make_normf(nm);
-    const double a = K[0], b = K[1], c = K[2], d = K[3], e = K[4], f = K[5], g = K[6], hh = K[7], i9 = K[8];
+    // K^-1 by cofactors: entry (r, c) = (K[a] K[b] - K[c] K[d]) / det
+    const double a = s.K[0], b = s.K[1], c = s.K[2], d = s.K[3], e = s.K[4], f = s.K[5], g = s.K[6], hh = s.K[7],
+                 i9 = s.K[8];
     const double det = a * (e * i9 - f * hh) - b * (d * i9 - f * g) + c * (d * hh - e * g);
-    const double ki[9] = {(e * i9 - f * hh) / det, (c * hh - b * i9) / det, (b * f - c * e) / det,
-                          (f * g - d * i9) / det,  (a * i9 - c * g) / det,  (c * d - a * f) / det,
-                          (d * hh - e * g) / det,  (b * g - a * hh) / det,  (a * e - b * d) / det};
-    for (int k = 0; k < 9; ++k) ec.kinv[k] = static_cast<float>(ki[k]);
-    ec.w = w;
-    ec.h = h;
-    ec.ok = ok;
+    const double ki[9] = {e * i9 - f * hh, c * hh - b * i9, b * f - c * e, f * g - d * i9, a * i9 - c * g,
+                          c * d - a * f,   d * hh - e * g,  b * g - a * hh, a * e - b * d};
+    double x = det;
+    for (int k = 0; k < 9; ++k) x = lane == k ? ki[k] : x;
+    x /= det;
+    if (lane < 9) ec.kinv[lane] = static_cast<float>(x);
+    if (lane == 0) {
+        ec.qscale = static_cast<float>(sc);
+        ec.nf = nf;
+        ec.w = w;
+        ec.h = h;
+        ec.ok = ok;
+    }
 }
 
 // One CTA per view: sum the block partials in a fixed order, solve, factorise.
 __global__ void __launch_bounds__(64) solve_kernel(const double *__restrict__ partial, int n_blocks,
-                                                   const Norm *__restrict__ norm,
+                                                   const Norm *__restrict__ norm, const NormF *__restrict__ normf,
                                                    const VsRpcCamera *__restrict__ cams, double *__restrict__ K_out,
                                                    double *__restrict__ R_out, double *__restrict__ t_out,
                                                    double *__restrict__ params, ErrCam *__restrict__ errcam,
                                                    int32_t *__restrict__ status) {
     __shared__ double mom[kSlots];
+    chain_wait();
     const int v = blockIdx.x;
     if (threadIdx.x < kSlots) {
         double s = 0.0;
         const double *p = partial + static_cast<long long>(v) * n_blocks * kSlots + threadIdx.x;
-        for (int b = 0; b < n_blocks; ++b) s += p[b * kSlots];
+        int b = 0;
+        for (; b + 16 <= n_blocks; b += 16) {           // one chain of sums; its loads 16 at a time
+            double x[16];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) x[k] = p[(b + k) * kSlots];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) s += x[k];
+        }
+        for (; b < n_blocks; ++b) s += p[b * kSlots];
         mom[threadIdx.x] = s;
     }
     __syncthreads();
-    // warp 0 solves; lane 0 keeps the serial parts (maps, factorisation, outputs), the
-    // Cholesky factor and the triangular solves run across lanes 0..11 (one row each)
     if (threadIdx.x >= 32) return;
-    const int lane = threadIdx.x;
-    __shared__ double G[12][12];
-    __shared__ double vec[3][12];          // p, u, w
-    __shared__ double s_floor;
+    const int lane = threadIdx.x, l = min(lane, 11), bl = l >> 2, il = l & 3;   // lanes 12.. repeat lane 11
+    __shared__ double L[12][13];
+    __shared__ CameraSmem cam;
     const Norm nm = norm[v];
-    const double count = mom[kMom];
-    double K[9], R[9], t[3];
-    for (int i = 0; i < 9; ++i) K[i] = R[i] = 0.0;
-    t[0] = t[1] = t[2] = 0.0;
-    int st = VS_OK;
-    if (count < 6.0) st = VS_ERR_DEGENERATE;
-    double P[12];
+    if (lane < 9) cam.K[lane] = cam.R[lane] = 0.0;
+    if (lane < 3) cam.t[lane] = 0.0;
+    int st = mom[kMom] < 6.0 ? VS_ERR_DEGENERATE : VS_OK;
     if (st == VS_OK) {
-        // normalised Gram matrix G = [[S0,0,-Sc],[0,S0,-Sr],[-Sc,-Sr,Sq]]
-        if (lane == 0) {
-            const int ent[10][2] = {{0, 0}, {0, 1}, {0, 2}, {0, 3}, {1, 1}, {1, 2}, {1, 3}, {2, 2}, {2, 3}, {3, 3}};
-            for (int i = 0; i < 12; ++i)
-                for (int j = 0; j < 12; ++j) G[i][j] = 0.0;
-            for (int e = 0; e < 10; ++e) {
-                const int a = ent[e][0], b = ent[e][1];
-                const double s0 = mom[e], sc = mom[10 + e], sr = mom[20 + e], sq = mom[30 + e];
-                G[a][b] = G[b][a] = s0;
-                G[4 + a][4 + b] = G[4 + b][4 + a] = s0;
-                G[a][8 + b] = G[b][8 + a] = G[8 + a][b] = G[8 + b][a] = -sc;
-                G[4 + a][8 + b] = G[4 + b][8 + a] = G[8 + a][4 + b] = G[8 + b][4 + a] = -sr;
-                G[8 + a][8 + b] = G[8 + b][8 + a] = sq;
-            }
-            double dmax = 0.0;
-            for (int i = 0; i < 12; ++i) dmax = fmax(dmax, G[i][i]);
-            s_floor = dmax * 1e-30 + 1e-300;
-        }
-        __syncwarp();
-        // Cholesky G = L L^T, column by column (a non-positive pivot -- an exactly
-        // consistent system -- is floored; the inverse iteration then lands on the null
-        // vector).  Every element keeps the serial operation order.
-        const double floor_piv = s_floor;
+        // row l of the normalised Gram matrix G = [[S0,0,-Sc],[0,S0,-Sr],[-Sc,-Sr,Sq]], S* symmetric
+        double g[12];
+        const int ent[4] = {0, 3, 5, 6};               // entry (a, b >= a) of a 10-vector: ent[a] + b
+        double dmax = 0.0;
+#pragma unroll
         for (int j = 0; j < 12; ++j) {
-            if (lane == j) {
-                double d = G[j][j];
-                for (int k = 0; k < j; ++k) d -= G[j][k] * G[j][k];
-                d = d > floor_piv ? d : floor_piv;
-                G[j][j] = sqrt(d);
-            }
-            __syncwarp();
-            if (lane > j && lane < 12) {
-                double sum = G[lane][j];
-                for (int k = 0; k < j; ++k) sum -= G[lane][k] * G[j][k];
-                G[lane][j] = sum / G[j][j];
-            }
-            __syncwarp();
+            const int bj = j >> 2, ij = j & 3, lo = min(il, ij), hi = max(il, ij);
+            const double *m = mom + ((lo == 0 ? ent[0] : (lo == 1 ? ent[1] : (lo == 2 ? ent[2] : ent[3]))) + hi);
+            const int other = min(bl, bj);             // 0: column block, 1: row block, when just one is block 2
+            g[j] = bl == bj ? (bl < 2 ? m[0] : m[30]) : (max(bl, bj) < 2 ? 0.0 : (other == 0 ? -m[10] : -m[20]));
+            dmax = fmax(dmax, l == j ? g[j] : 0.0);
         }
-        const Mmap mm{nm.cx, nm.cy, nm.cz, nm.s, nm.c0, nm.r0, nm.sp};
-        if (lane < 12) vec[0][lane] = 0.28867513459481287;   // 1/sqrt(12)
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, d));
+        // Cholesky G = L L^T, column by column (a non-positive pivot -- an exactly
+        // consistent system -- is floored; the inverse iteration then lands on the null vector).
+        // Every lane forms the pivot; each element loses its products in the order of the columns.
+        const double floor_piv = dmax * 1e-30 + 1e-300;
+        double diag = 1.0;
+#pragma unroll
+        for (int k = 0; k < 12; ++k) {
+            double d = lane_get(g[k], k);
+            d = d > floor_piv ? d : floor_piv;
+            d = sqrt(d);
+            g[k] = l == k ? d : g[k] / d;
+            diag = l == k ? d : diag;
+#pragma unroll
+            for (int j = k + 1; j < 12; ++j) g[j] = __fma_rn(-g[k], lane_get(g[k], j), g[j]);
+        }
+        if (lane < 12)
+#pragma unroll
+            for (int j = 0; j < 12; ++j) L[lane][j] = g[j];
         __syncwarp();
+        double col[12];
+#pragma unroll
+        for (int j = 0; j < 12; ++j) col[j] = L[j][l];
+        const LaneDivisor pivot = lane_divisor(diag), scale = lane_divisor(nm.s);
+        double p = 0.28867513459481287;                // 1/sqrt(12)
+#pragma unroll 1
         for (int it = 0; it < 6; ++it) {
-            if (lane == 0) solve_mt(mm, vec[0], vec[1]);
-            __syncwarp();
+            double sum = solve_mt(nm, scale, bl, il, p), x = 0.0;
             // L w = u: lane i subtracts w[j] L[i][j] as each w[j] is formed
-            double sum = lane < 12 ? vec[1][lane] : 0.0;
+#pragma unroll
             for (int j = 0; j < 12; ++j) {
-                if (lane == j) vec[2][j] = sum / G[j][j];
-                __syncwarp();
-                if (lane > j && lane < 12) sum -= G[lane][j] * vec[2][j];
+                const double t = lane_div(sum, pivot), wj = lane_get(t, j);
+                x = l == j ? t : x;
+                sum = l > j ? __fma_rn(-g[j], wj, sum) : sum;
             }
-            __syncwarp();
             // L^T u = w
-            sum = lane < 12 ? vec[2][lane] : 0.0;
+            sum = x;
+#pragma unroll
             for (int j = 11; j >= 0; --j) {
-                if (lane == j) vec[1][j] = sum / G[j][j];
-                __syncwarp();
-                if (lane < j) sum -= G[j][lane] * vec[1][j];
+                const double t = lane_div(sum, pivot), uj = lane_get(t, j);
+                x = l == j ? t : x;
+                sum = l < j ? __fma_rn(-col[j], uj, sum) : sum;
             }
-            __syncwarp();
-            if (lane == 0) {
-                double pp[12];
-                solve_m(mm, vec[1], pp);
-                double nrm = 0.0;
-                for (int i = 0; i < 12; ++i) nrm += pp[i] * pp[i];
-                nrm = 1.0 / sqrt(nrm);
-                for (int i = 0; i < 12; ++i) vec[0][i] = pp[i] * nrm;
+            const double pp = solve_m(nm, scale, bl, il, x);
+            double nrm = 0.0;
+#pragma unroll
+            for (int i = 0; i < 12; ++i) {
+                const double y = lane_get(pp, i);
+                nrm = __fma_rn(y, y, nrm);
             }
-            __syncwarp();
+            p = __dmul_rn(pp, 1.0 / sqrt(nrm));
         }
-        if (lane != 0) return;
-        double p[12];
-        for (int i = 0; i < 12; ++i) p[i] = vec[0][i];
-        for (int i = 0; i < 12; ++i) P[i] = p[i];
-        bool finite = true;
-        for (int i = 0; i < 12; ++i) finite &= isfinite(P[i]);
-        st = finite ? factorize(P, K, R, t) : VS_ERR_DEGENERATE;
+        if (lane < 12) cam.P[lane] = p;
+        __syncwarp();
+        st = __all_sync(0xffffffffu, isfinite(p)) ? factorize(cam, lane) : VS_ERR_DEGENERATE;
     }
-    if (lane != 0) return;
-    for (int i = 0; i < 9; ++i) K_out[v * 9 + i] = K[i], R_out[v * 9 + i] = R[i];
-    for (int i = 0; i < 3; ++i) t_out[v * 3 + i] = t[i];
-    status[v] = st;
-    if (errcam)
-        make_errcam(K, R, t, nm, cams ? static_cast<float>(cams[v].width) : 0.f,
-                    cams ? static_cast<float>(cams[v].height) : 0.f, st == VS_OK, errcam[v]);
+    __syncwarp();
+    const double *K = cam.K, *R = cam.R, *t = cam.t;
+    if (lane < 9) K_out[v * 9 + lane] = K[lane], R_out[v * 9 + lane] = R[lane];
+    if (lane < 3) t_out[v * 3 + lane] = t[lane];
+    if (lane == 0) status[v] = st;
     if (params) {
         double q[4] = {0, 0, 0, 0};
         if (st == VS_OK) quaternion(R, q);
         double *o = params + v * VS_CAMERA_PARAMS;
-        o[0] = cams ? cams[v].width : 0.0;
-        o[1] = cams ? cams[v].height : 0.0;
-        o[2] = K[0]; o[3] = K[4]; o[4] = K[2]; o[5] = K[5]; o[6] = K[1];
-        o[7] = q[0]; o[8] = q[1]; o[9] = q[2]; o[10] = q[3];
-        o[11] = t[0]; o[12] = t[1]; o[13] = t[2];
+        if (lane == 0) {
+            o[0] = cams ? cams[v].width : 0.0;
+            o[1] = cams ? cams[v].height : 0.0;
+            o[2] = K[0]; o[3] = K[4]; o[4] = K[2]; o[5] = K[5]; o[6] = K[1];
+            o[7] = q[0]; o[8] = q[1]; o[9] = q[2]; o[10] = q[3];
+            o[11] = t[0]; o[12] = t[1]; o[13] = t[2];
+        }
     }
+    if (errcam)
+        make_errcam(cam, nm, normf[v], cams ? static_cast<float>(cams[v].width) : 0.f,
+                    cams ? static_cast<float>(cams[v].height) : 0.f, st == VS_OK, errcam[v], lane);
 }
 
 // ---------------------------------------------------------------------------------------
 // error statistics (check_perspective_error)
 // ---------------------------------------------------------------------------------------
-// ErrCam for given K, R, t (the drop-in statistics entry)
-__global__ void errcam_kernel(const double *K, const double *R, const double *t, const Norm *norm, int n_views,
-                              ErrCam *ec) {
-    int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= n_views) return;
-    make_errcam(K + 9 * v, R + 9 * v, t + 3 * v, norm[v], 0.f, 0.f, 1, ec[v]);
+// ErrCam for given K, R, t (the drop-in statistics entry), a warp per view
+__global__ void __launch_bounds__(32) errcam_kernel(const double *K, const double *R, const double *t,
+                                                    const Norm *norm, const NormF *normf, ErrCam *ec) {
+    __shared__ CameraSmem s;
+    chain_wait();
+    const int v = blockIdx.x, lane = threadIdx.x;
+    if (lane < 9) s.K[lane] = K[9 * v + lane], s.R[lane] = R[9 * v + lane];
+    if (lane < 3) s.t[lane] = t[3 * v + lane];
+    __syncwarp();
+    make_errcam(s, norm[v], normf[v], 0.f, 0.f, 1, ec[v], lane);
 }
 
 // Radix selection over the float bits of the per-point errors (non-negative floats, so
@@ -741,13 +822,118 @@ constexpr int kBins = 2048;
 struct ErrWs {
     unsigned *keys;          // [2][V][n] float bits of the per-point errors (kept points only)
     double *sums;            // [V][blocks][3]: pixel sum, metric sum, count
-    unsigned *maxk;          // [V][2]
-    unsigned *hist;          // [V][2][kBins] histogram of the current digit (pixel, metric)
-    unsigned *sel;           // [V][4][3]: prefix, mask, rank
-    double *cnt;             // [V]
+    unsigned *maxk;          // [V][2]; maxk and hist are cleared as one range
+    unsigned *hist;          // [V][2][kBins] of the leading digit (pixel, metric), then for each
+                             // later digit [V][4][kBins] (one per target)
+    size_t cleared;          // bytes from maxk to the end of hist
+    unsigned *sel;           // [V][4][2]: prefix, rank
+    __device__ unsigned *digit_hist(int pass, int V, int v) const {
+        return pass == 0 ? hist + static_cast<long long>(v) * 2 * kBins
+                         : hist + (2ll * V + 4ll * (pass - 1) * V + 4ll * v) * kBins;
+    }
 };
 
 constexpr int kErrThreads = 256;
+
+// Inclusive sum over the lanes up to this one.
+__device__ __forceinline__ unsigned warp_scan(unsigned x, int lane) {
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const unsigned u = __shfl_up_sync(0xffffffffu, x, off);
+        if (lane >= off) x += u;
+    }
+    return x;
+}
+
+// Picks digit `pass` of the four targets of one view: one block per view, one warp per target.
+// Pass 0 reads the two histograms the error kernel built (pixel, metric) and starts from the
+// ranks; later passes read one histogram per target, except that the high target shares its
+// low partner's while their prefixes agree.  A warp takes its bins in two looks -- all bins, a run
+// per lane, then the run that holds the rank -- instead of 32 bins at a time, each a trip to L2 (12
+// to 43 us, 6 to 8 now).  The last pass also writes the view's statistics, which, like the
+// ranks, were launches that summed the blocks' partials one by one (17 + 29 us for 210 blocks).
+// (A step by the last block of the pass before it saves a launch and costs every block a fence
+// behind its histogram's atomics: 50 us more for 50 views.)
+constexpr int kStepThreads = 128;
+
+__global__ void __launch_bounds__(kStepThreads) select_step_kernel(ErrWs w, int n_blocks, int pass,
+                                                                   double *__restrict__ err) {
+    const int v = blockIdx.x, V = gridDim.x;
+    const int t = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ double part[3][kStepThreads / 32];
+    __shared__ unsigned pre[4];
+    chain_wait();
+    double total[3] = {0.0, 0.0, 0.0};       // pixel sum, metric sum, count
+    if (pass != 1) {
+        for (int b = threadIdx.x; b < n_blocks; b += kStepThreads)
+#pragma unroll
+            for (int q = 0; q < 3; ++q) total[q] += w.sums[(static_cast<long long>(v) * n_blocks + b) * 3 + q];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) total[q] += __shfl_xor_sync(0xffffffffu, total[q], off);
+            if (lane == 0) part[q][t] = total[q];
+        }
+    }
+    unsigned *sel = w.sel + 2 * (v * 4 + t);
+    if (lane == 0) pre[t] = pass == 0 ? 0u : sel[0];
+    __syncthreads();
+    if (pass != 1)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) total[q] = ((part[q][0] + part[q][1]) + part[q][2]) + part[q][3];
+    const unsigned long long n = static_cast<unsigned long long>(total[2]);
+    const unsigned k = pass == 0 ? (n ? static_cast<unsigned>((t & 1) ? n / 2 : (n - 1) / 2) : 0u) : sel[1];
+    const int which = pass == 0 ? t >> 1 : ((t & 1) && pre[t] == pre[t ^ 1] ? t ^ 1 : t);
+    const unsigned *hist = w.digit_hist(pass, V, v) + which * kBins;
+    const int bins = 1 << digit_bits(pass), run = bins / 32;
+    unsigned c = 0;
+    const uint4 *mine = reinterpret_cast<const uint4 *>(hist + lane * run);
+#pragma unroll 8
+    for (int i = 0; i < run / 4; ++i) {
+        const uint4 x = mine[i];
+        c += (x.x + x.y) + (x.z + x.w);
+    }
+    unsigned incl = warp_scan(c, lane);
+    const unsigned hit = __ballot_sync(0xffffffffu, incl > k);
+    int digit = bins - 1;
+    unsigned skip;
+    if (hit) {
+        const int seg = __ffs(hit) - 1;
+        unsigned below = __shfl_sync(0xffffffffu, incl - c, seg);
+        digit = seg * run;
+        for (int i = 0; i < run; i += 32) {          // one or two looks
+            const unsigned x = hist[seg * run + i + lane], in = warp_scan(x, lane);
+            const unsigned h2 = __ballot_sync(0xffffffffu, below + in > k);
+            if (h2) {
+                digit = seg * run + i + __ffs(h2) - 1;
+                below += __shfl_sync(0xffffffffu, in - x, __ffs(h2) - 1);
+                break;
+            }
+            below += __shfl_sync(0xffffffffu, in, 31);
+        }
+        skip = below;
+    } else {                     // rank beyond the counts (no kept points): the last bin
+        skip = __shfl_sync(0xffffffffu, incl, 31) - hist[bins - 1];
+    }
+    const unsigned chosen = pre[t] | (static_cast<unsigned>(digit) << digit_shift(pass));
+    __syncthreads();                                     // every pre[] has been read
+    if (lane == 0) {
+        sel[0] = chosen;
+        sel[1] = k - skip;
+        pre[t] = chosen;
+    }
+    if (pass < 2) return;
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        const int q = threadIdx.x;
+        const double cnt = total[2], lo = __uint_as_float(pre[2 * q]), hi = __uint_as_float(pre[2 * q + 1]);
+        const double nan = __longlong_as_double(0x7ff8000000000000ll);
+        double *o = err + v * VS_ERROR_STATS + 3 * q;
+        o[0] = cnt > 0 ? (q ? total[1] : total[0]) / cnt : nan;
+        o[1] = cnt > 0 ? ((0.0 + lo) + hi) / 2.0 : nan;
+        o[2] = cnt > 0 ? static_cast<double>(__uint_as_float(w.maxk[2 * v + q])) : nan;
+    }
+}
 
 // compensated dot product of a double-float 4-vector with (x, y, z, 1), FP32 exact inputs
 __device__ __forceinline__ df dot2(const df *q, float x, float y, float z) {
@@ -799,6 +985,7 @@ __global__ void __launch_bounds__(kErrThreads, 4) error_points_kernel(
     __shared__ ErrCam ec;
     __shared__ double red[3][kErrThreads / 32];
     __shared__ unsigned hist[2][kBins];
+    chain_wait();
     const int v = blockIdx.y;
     const int V = gridDim.y;
     if (threadIdx.x == 0) ec = cams[v];
@@ -892,125 +1079,57 @@ __global__ void __launch_bounds__(kErrThreads, 4) error_points_kernel(
     }
     for (int i = threadIdx.x; i < 2 * kBins; i += blockDim.x) {
         const unsigned c = (&hist[0][0])[i];
-        if (c) atomicAdd(w.hist + static_cast<long long>(v) * 2 * kBins + i, c);
+        if (c) atomicAdd(w.digit_hist(0, V, v) + i, c);
     }
 }
 
-// per-view totals of the block sums (fixed order) and the selection ranks
-__global__ void error_count_kernel(ErrWs w, int n_views, int n_blocks) {
-    int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= n_views) return;
-    double c = 0.0;
-    for (int b = 0; b < n_blocks; ++b) c += w.sums[(static_cast<long long>(v) * n_blocks + b) * 3 + 2];
-    w.cnt[v] = c;
-    const unsigned long long n = static_cast<unsigned long long>(c);
-    for (int t = 0; t < 4; ++t) {
-        const int i = v * 4 + t;
-        w.sel[3 * i] = 0;       // prefix
-        w.sel[3 * i + 1] = 0;   // mask
-        w.sel[3 * i + 2] = n ? static_cast<unsigned>((t & 1) ? n / 2 : (n - 1) / 2) : 0u;
-    }
-}
+// Histograms of digit `pass` (1, 2) of the keys matching each target's prefix.  Issue-bound at 94
+// instructions per point with four masked compares and as many histograms whether the targets of a
+// pair differ or not: now each thread has 4 points' keys in flight and compares them with
+// its pair's one prefix unless the pair has split, in as many blocks as the SMs hold (a block
+// clears and adds 8192 bins).  50 x 800,000 points: 125 us a pass, 77 us.
+constexpr int kHistThreads = 256, kHistAhead = 4;
 
-// Histograms of digit `pass` (1, 2) of the keys matching each target's prefix.
-__global__ void __launch_bounds__(256) select_hist_kernel(ErrWs w, long long n, int pass) {
+__global__ void __launch_bounds__(kHistThreads) select_hist_kernel(ErrWs w, long long n, int pass) {
     __shared__ unsigned h[4][kBins];
+    chain_wait();
     const int v = blockIdx.y, V = gridDim.y;
-    const int shift = digit_shift(pass);
+    const int shift = digit_shift(pass), top = shift + digit_bits(pass);
     const unsigned dmask = (1u << digit_bits(pass)) - 1u;
-    for (int i = threadIdx.x; i < 4 * kBins; i += blockDim.x) (&h[0][0])[i] = 0;
+    unsigned pre[4];
+    for (int t = 0; t < 4; ++t) pre[t] = w.sel[2 * (v * 4 + t)] >> top;
+    const bool split[2] = {pre[0] != pre[1], pre[2] != pre[3]};
+    for (int t = 0; t < 4; ++t)
+        if (!(t & 1) || split[t >> 1])
+            for (int i = threadIdx.x; i < kBins; i += kHistThreads) h[t][i] = 0;
     __syncthreads();
-    unsigned pre[4], msk[4];
-    for (int t = 0; t < 4; ++t) pre[t] = w.sel[3 * (v * 4 + t)], msk[t] = w.sel[3 * (v * 4 + t) + 1];
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
-         i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const unsigned kp = w.keys[static_cast<long long>(v) * n + i];
-        const unsigned kq = w.keys[(static_cast<long long>(V) + v) * n + i];
-        const unsigned dp = (kp >> shift) & dmask, dq = (kq >> shift) & dmask;
-        if ((kp & msk[0]) == pre[0]) atomicAdd(&h[0][dp], 1u);
-        if ((kp & msk[1]) == pre[1] && pre[1] != pre[0]) atomicAdd(&h[1][dp], 1u);
-        if ((kq & msk[2]) == pre[2]) atomicAdd(&h[2][dq], 1u);
-        if ((kq & msk[3]) == pre[3] && pre[3] != pre[2]) atomicAdd(&h[3][dq], 1u);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < 4 * kBins; i += blockDim.x) {
-        const unsigned c = (&h[0][0])[i];
-        if (c) atomicAdd(w.hist + static_cast<long long>(v) * 4 * kBins + i, c);
-    }
-}
-
-// Picks the digit of the four targets of one view: one block per view, one warp per
-// target, the bins scanned 32 at a time with warp prefix sums.  Every prefix is read
-// before the barrier and written after it.  Pass 0 reads the two histograms the error
-// kernel built (pixel, metric); later passes read one histogram per target, except that
-// the high target shares its low partner's histogram while their prefixes agree.
-__global__ void __launch_bounds__(128) select_step_kernel(ErrWs w, int pass) {
-    const int v = blockIdx.x;
-    const int t = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int i = v * 4 + t;
-    __shared__ unsigned pre[4];
-    if (lane == 0) pre[t] = w.sel[3 * i];
-    __syncthreads();
-    const unsigned *hist;
-    if (pass == 0) {
-        hist = w.hist + static_cast<long long>(v) * 2 * kBins + (t >> 1) * kBins;
-    } else {
-        const bool shared_h = (t & 1) && pre[t] == pre[t ^ 1];
-        hist = w.hist + static_cast<long long>(v) * 4 * kBins + (shared_h ? (t ^ 1) : t) * kBins;
-    }
-    const int bins = 1 << digit_bits(pass);
-    const unsigned k = w.sel[3 * i + 2];
-    unsigned below = 0;          // count of keys in earlier chunks
-    int digit = -1;
-    unsigned skip = 0;
-    for (int base = 0; base < bins; base += 32) {
-        const unsigned c = hist[base + lane];
-        unsigned incl = c;       // inclusive warp scan
+    const unsigned *kp = w.keys + static_cast<long long>(v) * n, *kq = w.keys + (static_cast<long long>(V) + v) * n;
+    const long long step = static_cast<long long>(gridDim.x) * kHistThreads * kHistAhead;
+    for (long long i = static_cast<long long>(blockIdx.x) * kHistThreads * kHistAhead + threadIdx.x; i < n; i += step) {
+        unsigned k[2][kHistAhead];
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const unsigned u = __shfl_up_sync(0xffffffffu, incl, off);
-            if (lane >= off) incl += u;
+        for (int u = 0; u < kHistAhead; ++u) {
+            const long long j = i + u * kHistThreads;
+            k[0][u] = j < n ? __ldcs(kp + j) : 0xffffffffu;      // as a point that is not kept
+            k[1][u] = j < n ? __ldcs(kq + j) : 0xffffffffu;
         }
-        const unsigned excl = incl - c;
-        const unsigned hit = __ballot_sync(0xffffffffu, below + incl > k);
-        if (hit) {
-            const int l = __ffs(hit) - 1;
-            digit = base + l;
-            skip = below + __shfl_sync(0xffffffffu, excl, l);
-            break;
-        }
-        below += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (digit < 0) {             // rank beyond the counts (no kept points): the last bin
-        digit = bins - 1;
-        skip = below - hist[bins - 1];
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+#pragma unroll
+            for (int u = 0; u < kHistAhead; ++u) {
+                const unsigned head = k[q][u] >> top, digit = (k[q][u] >> shift) & dmask;
+                if (head == pre[2 * q]) atomicAdd(&h[2 * q][digit], 1u);
+                if (split[q] && head == pre[2 * q + 1]) atomicAdd(&h[2 * q + 1][digit], 1u);
+            }
     }
     __syncthreads();
-    if (lane == 0) {
-        w.sel[3 * i] = pre[t] | (static_cast<unsigned>(digit) << digit_shift(pass));
-        w.sel[3 * i + 1] |= static_cast<unsigned>(bins - 1) << digit_shift(pass);
-        w.sel[3 * i + 2] = k - skip;
-    }
-}
-
-__global__ void error_final_kernel(ErrWs w, int n_views, int n_blocks, double *err) {
-    int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= n_views) return;
-    const double cnt = w.cnt[v];
-    double s[2] = {0.0, 0.0};
-    for (int b = 0; b < n_blocks; ++b) {
-        s[0] += w.sums[(static_cast<long long>(v) * n_blocks + b) * 3];
-        s[1] += w.sums[(static_cast<long long>(v) * n_blocks + b) * 3 + 1];
-    }
-    double *o = err + v * VS_ERROR_STATS;
-    const double nan = __longlong_as_double(0x7ff8000000000000ll);
-    for (int q = 0; q < 2; ++q) {
-        const double lo = __uint_as_float(w.sel[3 * (v * 4 + 2 * q)]);
-        const double hi = __uint_as_float(w.sel[3 * (v * 4 + 2 * q + 1)]);
-        o[3 * q] = cnt > 0 ? s[q] / cnt : nan;
-        o[3 * q + 1] = cnt > 0 ? ((0.0 + lo) + hi) / 2.0 : nan;
-        o[3 * q + 2] = cnt > 0 ? static_cast<double>(__uint_as_float(w.maxk[2 * v + q])) : nan;
-    }
+    unsigned *out = w.digit_hist(pass, V, v);
+    for (int t = 0; t < 4; ++t)
+        if (!(t & 1) || split[t >> 1])
+            for (int i = threadIdx.x; i < kBins; i += kHistThreads) {
+                const unsigned c = h[t][i];
+                if (c) atomicAdd(out + t * kBins + i, c);
+            }
 }
 
 int err_blocks(long long n) {
@@ -1018,52 +1137,51 @@ int err_blocks(long long n) {
     return static_cast<int>(std::max<long long>(1, std::min<long long>(want, sm_count() * 2LL)));
 }
 
+// Blocks per view of a histogram pass: at least 16 points per thread, at most two rounds of
+// what the SMs hold over all views.
+int hist_blocks(long long n, int V) {
+    const long long most = std::max<long long>(1, ceil_div(sm_count() * 12LL, V));
+    return static_cast<int>(std::max<long long>(1, std::min<long long>(ceil_div(n, kHistThreads * 16), most)));
+}
+
 ErrWs carve_err(Carver &cv, int V, long long n, int blocks) {
     ErrWs w;
     w.keys = cv.take<unsigned>(2 * static_cast<size_t>(V) * n);
     w.sums = cv.take<double>(static_cast<size_t>(V) * blocks * 3);
-    w.maxk = cv.take<unsigned>(2 * V);
-    w.hist = cv.take<unsigned>(static_cast<size_t>(V) * 4 * kBins);
-    w.sel = cv.take<unsigned>(static_cast<size_t>(V) * 12);
-    w.cnt = cv.take<double>(V);
+    w.maxk = cv.take<unsigned>(2 * static_cast<size_t>(V));
+    w.hist = cv.take<unsigned>(static_cast<size_t>(V) * 10 * kBins);
+    w.cleared = reinterpret_cast<char *>(w.hist + static_cast<size_t>(V) * 10 * kBins) - reinterpret_cast<char *>(w.maxk);
+    w.sel = cv.take<unsigned>(static_cast<size_t>(V) * 8);
     return w;
 }
 
+int clear_async(void *p, size_t bytes, cudaStream_t st) {
+    if (cudaMemsetAsync(p, 0, bytes, st) == cudaSuccess) return VS_OK;
+    set_error("cudaMemsetAsync failed");
+    return VS_ERR_CUDA;
+}
+
+// w.maxk .. w.hist have been cleared.
 int run_error_stats(const double *x, const double *y, const double *z, long long xyz_stride, const double *col,
                     const double *row, const float4 *colrow, const uint8_t *keep, int V, long long n,
                     const ErrCam *cams, double *err, ErrWs &w, cudaStream_t st) {
     const int blocks = err_blocks(n);
-    const size_t hist_bytes = sizeof(unsigned) * 4 * kBins * V;
-    if (cudaMemsetAsync(w.maxk, 0, sizeof(unsigned) * 2 * V, st) != cudaSuccess ||
-        cudaMemsetAsync(w.hist, 0, hist_bytes, st) != cudaSuccess) {
-        set_error("cudaMemsetAsync failed");
-        return VS_ERR_CUDA;
-    }
+    int s;
     if (n > 0) {
-        error_points_kernel<<<dim3(blocks, V), kErrThreads, 0, st>>>(x, y, z, xyz_stride, col, row, colrow, keep, n,
+        launch_chained(error_points_kernel, dim3(blocks, V), kErrThreads, 0, st, x, y, z, xyz_stride, col, row, colrow, keep, n,
                                                                       cams, w);
         VS_LAUNCH_CHECK("error_points_kernel");
-    } else if (cudaMemsetAsync(w.sums, 0, sizeof(double) * V * blocks * 3, st) != cudaSuccess) {
-        set_error("cudaMemsetAsync failed");
-        return VS_ERR_CUDA;
+    } else if ((s = clear_async(w.sums, sizeof(double) * V * blocks * 3, st)) != VS_OK) {
+        return s;
     }
-    const unsigned vg = static_cast<unsigned>(ceil_div(V, 128));
-    error_count_kernel<<<vg, 128, 0, st>>>(w, V, blocks);
-    VS_LAUNCH_CHECK("error_count_kernel");
-    for (int pass = 0; pass < 3 && n > 0; ++pass) {
-        if (pass > 0) {
-            if (cudaMemsetAsync(w.hist, 0, hist_bytes, st) != cudaSuccess) {
-                set_error("cudaMemsetAsync failed");
-                return VS_ERR_CUDA;
-            }
-            select_hist_kernel<<<dim3(blocks, V), 256, 0, st>>>(w, n, pass);
+    for (int pass = n > 0 ? 0 : 2; pass < 3; ++pass) {
+        if (pass > 0 && n > 0) {
+            launch_chained(select_hist_kernel, dim3(hist_blocks(n, V), V), kHistThreads, 0, st, w, n, pass);
             VS_LAUNCH_CHECK("select_hist_kernel");
         }
-        select_step_kernel<<<V, 128, 0, st>>>(w, pass);
+        launch_chained(select_step_kernel, V, kStepThreads, 0, st, w, blocks, pass, err);
         VS_LAUNCH_CHECK("select_step_kernel");
     }
-    error_final_kernel<<<vg, 128, 0, st>>>(w, V, blocks, err);
-    VS_LAUNCH_CHECK("error_final_kernel");
     return VS_OK;
 }
 
@@ -1079,7 +1197,7 @@ int box_blocks(long long n) {
 }
 
 struct FitWs {
-    unsigned long long *bb;
+    Box *box;
     Norm *norm;
     NormF *normf;
     double *partial;
@@ -1091,7 +1209,7 @@ struct FitWs {
 
 FitWs carve_fit(Carver &cv, int V, long long n, bool fused) {
     FitWs f;
-    f.bb = cv.take<unsigned long long>(static_cast<size_t>(V) * 10);
+    f.box = cv.take<Box>(V);
     f.norm = cv.take<Norm>(V);
     f.normf = cv.take<NormF>(V);
     f.partial = cv.take<double>(static_cast<size_t>(V) * mom_blocks(n) * kSlots);
@@ -1102,18 +1220,22 @@ FitWs carve_fit(Carver &cv, int V, long long n, bool fused) {
     return f;
 }
 
+// f.box has been cleared.
 int launch_norm(const double *x, const double *y, const double *z, long long xyz_stride, const double *col,
                 const double *row, const uint8_t *keep, const VsRpcCamera *cams, int V, long long n, FitWs &f,
                 cudaStream_t st) {
-    bbox_init_kernel<<<static_cast<unsigned>(ceil_div(V * 10, 128)), 128, 0, st>>>(f.bb, V);
-    VS_LAUNCH_CHECK("bbox_init_kernel");
-    if (n > 0) {
-        bbox_kernel<<<dim3(box_blocks(n), V), 256, 0, st>>>(x, y, z, xyz_stride, col, row, keep, n, box_step(n), f.bb);
-        VS_LAUNCH_CHECK("bbox_kernel");
-    }
-    norm_kernel<<<static_cast<unsigned>(ceil_div(V, 64)), 64, 0, st>>>(f.bb, cams, V, f.norm, f.normf);
-    VS_LAUNCH_CHECK("norm_kernel");
+    launch_chained(bbox_kernel, dim3(box_blocks(n), V), 256, 0, st, x, y, z, xyz_stride, col, row, keep, n, box_step(n), cams,
+                                                          f.box, f.norm, f.normf);
+    VS_LAUNCH_CHECK("bbox_kernel");
     return VS_OK;
+}
+
+int launch_moments(const double *x, const double *y, const double *z, long long xyz_stride, const double *col,
+                   const double *row, const float4 *colrow, const uint8_t *keep, int V, long long n, FitWs &f,
+                   cudaStream_t st) {
+    launch_chained(moments_kernel, dim3(mom_blocks(n), V), kMomThreads, 0, st, x, y, z, xyz_stride, col, row, colrow, keep,
+                   colrow ? f.wh : nullptr, n, f.normf, f.partial);
+    return check_launch("moments_kernel");
 }
 
 }  // namespace
@@ -1167,13 +1289,14 @@ extern "C" int vs_dlt_fit(const double *x, const double *y, const double *z, int
     cudaStream_t st = as_stream(stream);
     Carver cv(workspace);
     FitWs f = carve_fit(cv, n_views, n, false);
-    int s = launch_norm(x, y, z, xyz_stride, col, row, keep, nullptr, n_views, n, f, st);
+    int s = clear_async(f.box, sizeof(Box) * n_views, st);
+    if (s != VS_OK) return s;
+    s = launch_norm(x, y, z, xyz_stride, col, row, keep, nullptr, n_views, n, f, st);
     if (s != VS_OK) return s;
     const int blocks = mom_blocks(n);
-    moments_kernel<<<dim3(blocks, n_views), kMomThreads, 0, st>>>(x, y, z, xyz_stride, col, row, nullptr, keep,
-                                                                   nullptr, n, f.normf, f.partial);
-    VS_LAUNCH_CHECK("moments_kernel");
-    solve_kernel<<<n_views, 64, 0, st>>>(f.partial, blocks, f.norm, nullptr, K, R, t, nullptr, nullptr, status);
+    if ((s = launch_moments(x, y, z, xyz_stride, col, row, nullptr, keep, n_views, n, f, st)) != VS_OK) return s;
+    launch_chained(solve_kernel, n_views, 64, 0, st, f.partial, blocks, f.norm, f.normf, nullptr, K, R, t, nullptr,
+                   nullptr, status);
     VS_LAUNCH_CHECK("solve_kernel");
     return VS_OK;
 }
@@ -1201,9 +1324,12 @@ extern "C" int vs_perspective_error(const double *x, const double *y, const doub
     Carver cv(workspace);
     FitWs f = carve_fit(cv, n_views, 0, false);
     ErrWs w = carve_err(cv, n_views, n, err_blocks(n));
-    int s = launch_norm(x, y, z, xyz_stride, col, row, keep, nullptr, n_views, n, f, st);
+    int s = clear_async(f.box, sizeof(Box) * n_views, st);
+    if (s == VS_OK) s = clear_async(w.maxk, w.cleared, st);
     if (s != VS_OK) return s;
-    errcam_kernel<<<static_cast<unsigned>(ceil_div(n_views, 64)), 64, 0, st>>>(K, R, t, f.norm, n_views, f.errcam);
+    s = launch_norm(x, y, z, xyz_stride, col, row, keep, nullptr, n_views, n, f, st);
+    if (s != VS_OK) return s;
+    launch_chained(errcam_kernel, n_views, 32, 0, st, K, R, t, f.norm, f.normf, f.errcam);
     VS_LAUNCH_CHECK("errcam_kernel");
     return run_error_stats(x, y, z, xyz_stride, col, row, nullptr, keep, n_views, n, f.errcam, err, w, st);
 }
@@ -1241,26 +1367,30 @@ extern "C" int vs_camera_approx_perspective(const VsRpcCamera *cams, int n_views
     double *R = cv.take<double>(static_cast<size_t>(n_views) * 9);
     double *t = cv.take<double>(static_cast<size_t>(n_views) * 3);
     ErrWs ew = carve_err(cv, n_views, n, err_blocks(n));
+    // the clears first, so that nothing comes between the kernels of the chain
+    int s = clear_async(f.box, sizeof(Box) * n_views, st);
+    if (s == VS_OK && err) s = clear_async(ew.maxk, ew.cleared, st);
+    if (s != VS_OK) return s;
     // ENU box (sampled) -> normalisation; pixel frame from each RPC
-    int s = launch_norm(x, y, z, point_stride, nullptr, nullptr, nullptr, cams, n_views, n, f, st);
+    s = launch_norm(x, y, z, point_stride, nullptr, nullptr, nullptr, cams, n_views, n, f, st);
     if (s != VS_OK) return s;
     const int blocks = mom_blocks(n);
-    prepare_views_kernel<<<n_views, 64, 0, st>>>(cams, f.fast, f.wh);
+    launch_chained(prepare_views_kernel, n_views, 64, 0, st, cams, f.fast, f.wh);
     VS_LAUNCH_CHECK("prepare_views_kernel");
     if (n > 0) {
         const unsigned pg = static_cast<unsigned>(std::min<long long>(ceil_div(n, 256), sm_count() * 8LL / n_views + 8));
         if (proj_mode == VS_PROJ_EXACT)
-            project_view_kernel<VS_PROJ_EXACT><<<dim3(pg, n_views), 256, 0, st>>>(cams, f.fast, lat, lon, alt, n,
+            launch_chained(project_view_kernel<VS_PROJ_EXACT>, dim3(pg, n_views), 256, 0, st, cams, f.fast, lat, lon, alt, n,
                                                                                   point_stride, f.colrow);
         else
-            project_view_kernel<VS_PROJ_FAST><<<dim3(pg, n_views), 256, 0, st>>>(cams, f.fast, lat, lon, alt, n,
+            launch_chained(project_view_kernel<VS_PROJ_FAST>, dim3(pg, n_views), 256, 0, st, cams, f.fast, lat, lon, alt, n,
                                                                                  point_stride, f.colrow);
         VS_LAUNCH_CHECK("project_view_kernel");
     }
-    moments_kernel<<<dim3(blocks, n_views), kMomThreads, 0, st>>>(x, y, z, point_stride, nullptr, nullptr, f.colrow,
-                                                                   nullptr, f.wh, n, f.normf, f.partial);
-    VS_LAUNCH_CHECK("moments_kernel");
-    solve_kernel<<<n_views, 64, 0, st>>>(f.partial, blocks, f.norm, cams, K, R, t, params, f.errcam, status);
+    if ((s = launch_moments(x, y, z, point_stride, nullptr, nullptr, f.colrow, nullptr, n_views, n, f, st)) != VS_OK)
+        return s;
+    launch_chained(solve_kernel, n_views, 64, 0, st, f.partial, blocks, f.norm, f.normf, cams, K, R, t, params, f.errcam,
+                   status);
     VS_LAUNCH_CHECK("solve_kernel");
     if (!err) return VS_OK;
     return run_error_stats(x, y, z, point_stride, nullptr, nullptr, f.colrow, nullptr, n_views, n, f.errcam, err, ew,
