@@ -149,17 +149,25 @@ static __device__ __noinline__ void geo_exact(const GeoFrame *__restrict__ gp, d
 }
 
 // ---- fast path --------------------------------------------------------------------------
-// round(x * 2^30) of a float with integer operations (|x| < 2^32).
-__device__ __forceinline__ long long fx30(float x) {
+// round(x * 2^30) of a double-float's words with integer operations, halves away from zero.
+// The high word |x| < 2^32: x = m * 2^(sh - 30), an exact shift for |x| >= 2^-7.  The low word |x| < 1, and
+// a high word below 2^-7, need 32 bits only (a shift by 31 stands for all that round to 0).
+__device__ __forceinline__ int fx30_round(unsigned m, int sh) {      // m < 2^24, sh < 0
+    const int s = min(-sh, 31);
+    return static_cast<int>((m + (1u << (s - 1))) >> s);
+}
+__device__ __forceinline__ long long fx30_hi(float x) {
     const unsigned u = __float_as_uint(x);
-    const int e = static_cast<int>((u >> 23) & 0xffu);
-    const long long m = static_cast<long long>((u & 0x7fffffu) | 0x800000u);
-    const int sh = e - 120;                   // x = m * 2^(e - 150) = m * 2^(sh - 30)
-    long long v;
-    if (e == 0) v = 0;                        // zero (and subnormals, < 2^-126 m)
-    else if (sh >= 0) v = m << sh;
-    else if (sh > -25) v = (m + (1ll << (-sh - 1))) >> (-sh);
-    else v = 0;
+    const unsigned m = (u & 0x7fffffu) | 0x800000u;
+    const int sh = static_cast<int>((u >> 23) & 0xffu) - 120;
+    const long long v = sh >= 0 ? static_cast<long long>(m) << sh : static_cast<long long>(fx30_round(m, sh));
+    return (u >> 31) ? -v : v;
+}
+__device__ __forceinline__ int fx30_lo(float x) {
+    const unsigned u = __float_as_uint(x);
+    const unsigned m = (u & 0x7fffffu) | 0x800000u;
+    const int sh = static_cast<int>((u >> 23) & 0xffu) - 120;
+    const int v = sh >= 0 ? static_cast<int>(m << sh) : fx30_round(m, sh);
     return (u >> 31) ? -v : v;
 }
 
@@ -187,9 +195,9 @@ __device__ __forceinline__ df df_dot3(const df (&c)[3], const df (&s)[3]) {
     return df_add_ops(acc, df_mul(c[2], s[2]));
 }
 
-// (easting, northing, altitude) FP64 bits of an ENU point given in double-float.  Returns
+// (easting, northing, altitude) of an ENU point given in double-float, in units of 2^-30 m.  Returns
 // false (nothing written) when the point lies outside the plan's box.
-__device__ __forceinline__ bool geo_fast(const GeoFast &f, const df (&enu)[3], unsigned long long (&bits)[3]) {
+__device__ __forceinline__ bool geo_fast_fixed(const GeoFast &f, const df (&enu)[3], long long (&S)[3]) {
     df s[3];
     bool inside = true;
 #pragma unroll
@@ -223,8 +231,16 @@ __device__ __forceinline__ bool geo_fast(const GeoFast &f, const df (&enu)[3], u
 #pragma unroll
         for (int j = kGeoNl - 1; j >= 0; --j) nl = __fmaf_rn(f.nl[o][j], m[j], nl);   // small terms first
         const df v = df_add_f(df_dot3(f.lin[o], s), nl);
-        bits[o] = fx30_to_bits(f.c0[o] + fx30(v.hi) + fx30(v.lo));
+        S[o] = f.c0[o] + fx30_hi(v.hi) + fx30_lo(v.lo);   // in the box |v| < 2^18 m, so |v.lo| < 1
     }
+    return true;
+}
+// The same as FP64 bits.
+__device__ __forceinline__ bool geo_fast(const GeoFast &f, const df (&enu)[3], unsigned long long (&bits)[3]) {
+    long long S[3];
+    if (!geo_fast_fixed(f, enu, S)) return false;
+#pragma unroll
+    for (int o = 0; o < 3; ++o) bits[o] = fx30_to_bits(S[o]);
     return true;
 }
 
