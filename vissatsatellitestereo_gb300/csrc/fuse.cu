@@ -221,6 +221,7 @@ template <int N>
 __global__ void __launch_bounds__(kTileCells) fuse_tile_kernel(const float *__restrict__ dsm, int layout, int V,
                                                                long long cells, float *__restrict__ out,
                                                                long long n_tiles, int aligned) {
+    chain_wait();
     extern __shared__ __align__(16) float fsm[];           // the tile: V x 128 (VHW) or 128 x V (HWV)
     float *scratch = fsm + V * kTileCells;                 // sorted columns: N x 128
     const int t = threadIdx.x;
@@ -376,6 +377,7 @@ template <int N, int L>
 __global__ void __launch_bounds__(kTileCells, 3) fuse_wide_kernel(const float *__restrict__ dsm, int layout, int V,
                                                                long long cells, float *__restrict__ out,
                                                                long long n_tiles, int aligned) {
+    chain_wait();
     using T = WideTile<L>;
     extern __shared__ __align__(16) float fsm[];            // the sorted cells, then the tile
     float *tile = fsm + ((T::kSorted + 3) & ~3);
@@ -488,7 +490,7 @@ bool launch_fuse_v64(const float *dsm, int layout, int V, long long cells, float
         return false;
     const long long n_tiles = ceil_div(cells, static_cast<long long>(kTileCells));
     const unsigned g = static_cast<unsigned>(std::min<long long>(n_tiles, 1LL * sm_count() * per_sm));
-    fuse_tile_kernel<N><<<g, kTileCells, sh, st>>>(dsm, layout, V, cells, out, n_tiles, aligned ? 1 : 0);
+    launch_chained(fuse_tile_kernel<N>, g, kTileCells, sh, st, dsm, layout, V, cells, out, n_tiles, aligned ? 1 : 0);
     return true;
 }
 
@@ -512,16 +514,17 @@ bool launch_fuse_wide_n(const float *dsm, int layout, int V, long long cells, fl
         return false;
     const long long n_tiles = ceil_div(cells, static_cast<long long>(T::CS));
     const unsigned g = static_cast<unsigned>(std::min<long long>(n_tiles, 1LL * sm_count() * per_sm));
-    fuse_wide_kernel<N, L><<<g, kTileCells, sh, st>>>(dsm, layout, V, cells, out, n_tiles, aligned ? 1 : 0);
+    launch_chained(fuse_wide_kernel<N, L>, g, kTileCells, sh, st, dsm, layout, V, cells, out, n_tiles, aligned ? 1 : 0);
     return true;
 }
 
-// The fewest lanes that hold the views, each with the smaller of two networks that takes its share.
+// The fewest lanes that hold the views, each with the smallest of three networks that takes its share.
 template <int L>
 bool launch_fuse_wide_l(const float *dsm, int layout, int V, long long cells, float *out, bool aligned,
                         cudaStream_t st) {
     const int share = (V + L - 1) / L;
-    if (share <= 48) return launch_fuse_wide_n<48, L>(dsm, layout, V, cells, out, aligned, st);
+    if (share <= 44) return launch_fuse_wide_n<44, L>(dsm, layout, V, cells, out, aligned, st);
+    if (share <= 52) return launch_fuse_wide_n<52, L>(dsm, layout, V, cells, out, aligned, st);
     return launch_fuse_wide_n<64, L>(dsm, layout, V, cells, out, aligned, st);
 }
 

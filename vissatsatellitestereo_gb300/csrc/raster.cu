@@ -130,6 +130,7 @@ struct ThresholdJob {
 
 // The tables of both axes in one launch: 5 us of launch and FP64 latency, not twice.
 __global__ void __launch_bounds__(64) axis_thresholds_kernel(ThresholdJob row, ThresholdJob col) {
+    chain_wait();
     const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
     if (i <= row.n) row.thr[i] = axis_threshold(i, row.ulp, row.res);
     const long long j = i - (row.n + 1);
@@ -185,6 +186,7 @@ __global__ void __launch_bounds__(256) bin_max_kernel(const double *__restrict__
                                                       long long single_n, Tables tb,
                                                       unsigned long long *__restrict__ vk,
                                                       unsigned long long *__restrict__ first) {
+    chain_wait();
     const long long begin = offsets ? offsets[v] : 0;
     const long long end = offsets ? offsets[v + 1] : single_n;
     const long long stride = static_cast<long long>(gridDim.x) * blockDim.x * kPts;
@@ -385,6 +387,7 @@ __global__ void __launch_bounds__(256) bin_fast_kernel(const double *__restrict_
                                                        long long single_n, FastAxis ra, FastAxis ca,
                                                        unsigned long long *__restrict__ vk,
                                                        unsigned long long *__restrict__ first) {
+    chain_wait();
     const long long begin = offsets ? offsets[v] : 0;
     const long long end = offsets ? offsets[v + 1] : single_n;
     const long long stride = static_cast<long long>(gridDim.x) * blockDim.x * kFastPts;
@@ -467,6 +470,7 @@ __global__ void __launch_bounds__(kGridThreads) grid_f64_kernel(const unsigned l
     __shared__ unsigned long long raw[kGridRaw * kGridRaw];
     __shared__ unsigned short holes[kGridTile * kGridTile];
     __shared__ int n_holes;
+    chain_wait();
     constexpr int kLoads = (kGridRaw * kGridRaw + kGridThreads - 1) / kGridThreads;
     const int tid = threadIdx.x, r0 = blockIdx.y * kGridTile, c0 = blockIdx.x * kGridTile;
     if (tid == 0) n_holes = 0;
@@ -594,6 +598,7 @@ constexpr int kBlurRows = 8, kBlurCols = 30;
 template <typename T, typename I>
 __global__ void __launch_bounds__(256) median_blur3x3_kernel(const T *__restrict__ in, float *__restrict__ out, I H, I W,
                                                              I strips, I groups, I warps) {
+    chain_wait();
     const int lane = threadIdx.x & 31;
     const I wid = static_cast<I>(blockIdx.x) * 8 + static_cast<I>(threadIdx.x >> 5);
     if (wid >= warps) return;
@@ -646,11 +651,10 @@ int launch_blur(const T *in, float *out, long long h, long long w, long long n_i
     const unsigned blocks = static_cast<unsigned>(ceil_div(warps, 8));
     const long long small = (1LL << 31) - 64;
     if (h < small && w < small && warps < small)
-        median_blur3x3_kernel<T, int><<<blocks, 256, 0, st>>>(in, out, static_cast<int>(h), static_cast<int>(w),
-                                                              static_cast<int>(strips), static_cast<int>(groups),
-                                                              static_cast<int>(warps));
+        launch_chained(median_blur3x3_kernel<T, int>, blocks, 256, 0, st, in, out, static_cast<int>(h),
+                       static_cast<int>(w), static_cast<int>(strips), static_cast<int>(groups), static_cast<int>(warps));
     else
-        median_blur3x3_kernel<T, long long><<<blocks, 256, 0, st>>>(in, out, h, w, strips, groups, warps);
+        launch_chained(median_blur3x3_kernel<T, long long>, blocks, 256, 0, st, in, out, h, w, strips, groups, warps);
     return check_launch("median_blur3x3_kernel");
 }
 
@@ -819,6 +823,7 @@ __global__ void __launch_bounds__(TX *TY) dsm_epilogue_kernel(
     const unsigned long long *__restrict__ vk, const unsigned long long *__restrict__ first,
     const double *__restrict__ pts, float *__restrict__ out, unsigned long long *__restrict__ next_keys, int H,
     int W) {
+    chain_wait();
     __shared__ EpilogueSmem sm;
     epilogue_tile<true>(vk, PointsZeroDecoder{first, pts}, out, next_keys, H, W, blockIdx.y * TILE_Y, blockIdx.x * TX, sm);
 }
@@ -854,6 +859,7 @@ struct PipeEpi {          // view v-1's epilogue (n_tiles = 0: none)
 template <bool FLIP_ROW, bool FLIP_COL, int MINB>
 __global__ void __launch_bounds__(TX *TY, MINB) raster_pipe_kernel(const double *__restrict__ pts, PipeBin bin,
                                                                     PipeEpi epi, unsigned *__restrict__ counter) {
+    chain_wait();
     __shared__ EpilogueSmem sm;
     __shared__ long long item_sh[2];
     const int tid = threadIdx.y * TX + threadIdx.x;
@@ -974,7 +980,7 @@ void make_axis(Axis &ax, double off, double res, long long n, int dir, long long
 int launch_thresholds(const ThresholdJob &row, const ThresholdJob &col, cudaStream_t st) {
     const long long total = (row.n + 1) + (col.n + 1);
     if (total <= 0) return VS_OK;
-    axis_thresholds_kernel<<<static_cast<unsigned>(ceil_div(total, 64)), 64, 0, st>>>(row, col);
+    launch_chained(axis_thresholds_kernel, static_cast<unsigned>(ceil_div(total, 64)), 64, 0, st, row, col);
     return check_launch("axis_thresholds_kernel");
 }
 
@@ -1019,8 +1025,7 @@ size_t g_l2_persist = 0, g_l2_window_max = 0;
 
 // Launches `kernel` with an access-policy window that marks the key grid [base, base + bytes)
 // persisting in L2 -- the streamed points (evict-first loads) then cannot push the grid the
-// binning's atomics land in out of L2 -- when a set-aside is configured; otherwise a plain
-// launch.  The window is a per-launch attribute: the caller's stream keeps its own.
+// binning's atomics land in out of L2 -- when a set-aside is configured.  The window is a per-launch attribute: the caller's stream keeps its own.
 template <typename... KArgs, typename... Args>
 cudaError_t launch_with_key_window(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t st,
                                    const void *base, size_t bytes, Args... args) {
@@ -1029,18 +1034,21 @@ cudaError_t launch_with_key_window(void (*kernel)(KArgs...), dim3 grid, dim3 blo
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = 0;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;       // as launch_chained
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
     if (g_l2_persist > 0 && base && bytes > 0) {
         const size_t nb = std::min(bytes, g_l2_window_max);
-        attr[0].id = cudaLaunchAttributeAccessPolicyWindow;
-        attr[0].val.accessPolicyWindow.base_ptr = const_cast<void *>(base);
-        attr[0].val.accessPolicyWindow.num_bytes = nb;
-        attr[0].val.accessPolicyWindow.hitRatio =
+        attr[1].id = cudaLaunchAttributeAccessPolicyWindow;
+        attr[1].val.accessPolicyWindow.base_ptr = const_cast<void *>(base);
+        attr[1].val.accessPolicyWindow.num_bytes = nb;
+        attr[1].val.accessPolicyWindow.hitRatio =
             nb <= g_l2_persist ? 1.0f : static_cast<float>(g_l2_persist) / static_cast<float>(nb);
-        attr[0].val.accessPolicyWindow.hitProp = cudaAccessPropertyPersisting;
-        attr[0].val.accessPolicyWindow.missProp = cudaAccessPropertyStreaming;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        attr[1].val.accessPolicyWindow.hitProp = cudaAccessPropertyPersisting;
+        attr[1].val.accessPolicyWindow.missProp = cudaAccessPropertyStreaming;
+        cfg.numAttrs = 2;
     }
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
@@ -1087,7 +1095,7 @@ int bin_launch(const double *points, const long long *offsets, int v, long long 
                                    fa[0], fa[1], keys, first) != cudaSuccess)
             return check_launch("bin_fast_kernel");
     } else {
-        bin_max_kernel<true><<<gx, threads, 0, st>>>(points, offsets, v, single_n, tb, keys, first);
+        launch_chained(bin_max_kernel<true>, gx, threads, 0, st, points, offsets, v, single_n, tb, keys, first);
     }
     return check_launch("bin_max_kernel");
 }
@@ -1564,12 +1572,12 @@ extern "C" int vs_proj_to_grid(const double *points, int64_t n, double xoff, dou
     cudaStream_t st = as_stream(stream);
     RasterWs w = carve_raster(workspace, xsize, ysize, false);
     Tables tb;
-    int s = make_tables(xoff, yoff, xresolution, yresolution, xsize, ysize, w, tb, st);
-    if (s == VS_OK) s = clear(w.keys[0], w.cleared, st);
+    int s = clear(w.keys[0], w.cleared, st);         // first, so that only kernels follow one another
+    if (s == VS_OK) s = make_tables(xoff, yoff, xresolution, yresolution, xsize, ysize, w, tb, st);
     if (s == VS_OK) s = bin_launch(points, nullptr, 0, n, n, tb, w.keys[0], w.first, st);
     if (s != VS_OK) return s;
     const dim3 grid(static_cast<unsigned>(ceil_div(xsize, kGridTile)), static_cast<unsigned>(ceil_div(ysize, kGridTile)));
-    grid_f64_kernel<<<grid, kGridThreads, 0, st>>>(w.keys[0], w.first, points, dsm, static_cast<int>(ysize),
+    launch_chained(grid_f64_kernel, grid, kGridThreads, 0, st, w.keys[0], w.first, points, dsm, static_cast<int>(ysize),
                                                    static_cast<int>(xsize));
     VS_LAUNCH_CHECK("grid_f64_kernel");
     return VS_OK;
@@ -1596,8 +1604,8 @@ extern "C" int vs_dsm_from_points(const double *points, const int64_t *offsets, 
     RasterWs w = carve_raster(workspace, xsize, ysize, true);
     Tables tb;
     const long long cells = xsize * ysize;
-    int s = make_tables(xoff, yoff, xresolution, yresolution, xsize, ysize, w, tb, st);
-    if (s == VS_OK) s = clear(w.keys[0], w.cleared, st);
+    int s = clear(w.keys[0], w.cleared, st);         // first, so that only kernels follow one another
+    if (s == VS_OK) s = make_tables(xoff, yoff, xresolution, yresolution, xsize, ysize, w, tb, st);
     if (s != VS_OK) return s;
     // per-view counts live on the device: launch for a full GPU and let the grid stride
     const long long launch_points = static_cast<long long>(sm_count()) * 8 * 256 * kPts;
@@ -1606,7 +1614,7 @@ extern "C" int vs_dsm_from_points(const double *points, const int64_t *offsets, 
         unsigned long long *cur = w.keys[v & 1], *nxt = (v + 1 < n_views) ? w.keys[(v + 1) & 1] : nullptr;
         s = bin_launch(points, reinterpret_cast<const long long *>(offsets), v, 0, launch_points, tb, cur, w.first, st);
         if (s != VS_OK) return s;
-        dsm_epilogue_kernel<<<egrid, dim3(TX, TY), 0, st>>>(cur, w.first, points, dsm + v * cells, nxt,
+        launch_chained(dsm_epilogue_kernel, egrid, dim3(TX, TY), 0, st, cur, w.first, points, dsm + v * cells, nxt,
                                                             static_cast<int>(ysize), static_cast<int>(xsize));
         VS_LAUNCH_CHECK("dsm_epilogue_kernel");
     }
@@ -1712,8 +1720,8 @@ extern "C" int vs_dsm_from_points_host(const double *host_points, const int64_t 
     char *ring_base = static_cast<char *>(workspace) + ((w.bytes + 255) & ~size_t(255));
     Tables tb;
     const long long cells = xsize * ysize;
-    int s = make_tables(xoff, yoff, xresolution, yresolution, xsize, ysize, w, tb, st);
-    if (s == VS_OK) s = clear(w.keys[0], w.cleared, st);
+    int s = clear(w.keys[0], w.cleared, st);         // first, so that only kernels follow one another
+    if (s == VS_OK) s = make_tables(xoff, yoff, xresolution, yresolution, xsize, ysize, w, tb, st);
     if (s != VS_OK) return s;
     cudaEvent_t freed[8], landed[8];
     int made = 0;
@@ -1754,7 +1762,7 @@ extern "C" int vs_dsm_from_points_host(const double *host_points, const int64_t 
         }
         unsigned long long *cur = w.keys[v & 1], *nxt = (v + 1 < n_views) ? w.keys[(v + 1) & 1] : nullptr;
         if ((s = bin_launch(buf, nullptr, v, cnt, cnt, tb, cur, w.first, st)) != VS_OK) break;
-        dsm_epilogue_kernel<<<egrid, dim3(TX, TY), 0, st>>>(cur, w.first, buf, dsm + v * cells, nxt,
+        launch_chained(dsm_epilogue_kernel, egrid, dim3(TX, TY), 0, st, cur, w.first, buf, dsm + v * cells, nxt,
                                                             static_cast<int>(ysize), static_cast<int>(xsize));
         if ((s = check_launch("dsm_epilogue_kernel")) != VS_OK) break;
         if (cudaEventRecord(freed[b], st) != cudaSuccess) {
@@ -1897,7 +1905,7 @@ extern "C" int vs_dsm_from_points_pipelined(const double *points, const int64_t 
                            w.first[v & 1], st);
             if (s != VS_OK) return s;
             unsigned long long *nxt = (v + 2 < n_views) ? w.keys[(v + 2) % 3] : nullptr;
-            dsm_epilogue_kernel<<<egrid, dim3(TX, TY), 0, st>>>(w.keys[v % 3], w.first[v & 1], points,
+            launch_chained(dsm_epilogue_kernel, egrid, dim3(TX, TY), 0, st, w.keys[v % 3], w.first[v & 1], points,
                                                                 dsm + v * cells, nxt, static_cast<int>(ysize),
                                                                 static_cast<int>(xsize));
             VS_LAUNCH_CHECK("dsm_epilogue_kernel");
@@ -2342,6 +2350,7 @@ __global__ void __launch_bounds__(256, 3) depth_bin_kernel(const float *__restri
                                                         DirectAxis cd, int view,
                                                         unsigned long long *__restrict__ vk,
                                                         unsigned long long *__restrict__ first, int *flags) {
+    chain_wait();
     __shared__ double smd[16];
     stage_matrix(v, smd);
     const long long total = H * W;
@@ -2438,6 +2447,7 @@ __global__ void __launch_bounds__(TX *TY) depth_epilogue_kernel(const unsigned l
                                                                float *__restrict__ out,
                                                                unsigned long long *__restrict__ next_keys, int H,
                                                                int W) {
+    chain_wait();
     __shared__ EpilogueSmem sm;
     epilogue_tile<true>(vk, SignZeroDecoder{first}, out, next_keys, H, W, blockIdx.y * TILE_Y, blockIdx.x * TX, sm);
 }
@@ -2494,10 +2504,10 @@ extern "C" int vs_dsm_from_depth_maps(const float *const *depths, const int64_t 
         const unsigned gx = static_cast<unsigned>(
             std::max<long long>(1, std::min<long long>(ceil_div(ceil_div(total, kDepthPix), 256), sm_count() * 8LL)));
         // rows: a = off - v for the positive origin; columns: a = v - off
-        depth_bin_kernel<true, false><<<gx, 256, 0, st>>>(depths[v], heights[v], widths[v], dv, gf, gfr, mode, south,
+        launch_chained(depth_bin_kernel<true, false>, gx, 256, 0, st, depths[v], heights[v], widths[v], dv, gf, gfr, mode, south,
                                                           fr, fc, rd, cd, v, cur, w.first, fl);
         VS_LAUNCH_CHECK("depth_bin_kernel");
-        depth_epilogue_kernel<<<egrid, dim3(TX, TY), 0, st>>>(cur, w.first, dsm + v * cells, nxt,
+        launch_chained(depth_epilogue_kernel, egrid, dim3(TX, TY), 0, st, cur, w.first, dsm + v * cells, nxt,
                                                               static_cast<int>(ysize), static_cast<int>(xsize));
         VS_LAUNCH_CHECK("depth_epilogue_kernel");
     }
