@@ -19,6 +19,14 @@ from ._dev import as_device, is_cuda_tensor, ptr, require_cuda, stream_handle, w
 MODES = {'exact': _lib.VS_PROJ_EXACT, 'fast': _lib.VS_PROJ_FAST}
 
 
+def _same_layout(*ts):
+    """Contiguous float64 tensors of one shape on the current device: nothing to broadcast,
+    convert or copy (working that out costs a small call more than its kernel)."""
+    dev = torch.cuda.current_device()
+    return all(isinstance(t, torch.Tensor) and t.is_cuda and t.device.index == dev and t.dtype == torch.float64
+               and t.shape == ts[0].shape and t.is_contiguous() for t in ts)
+
+
 class RPCModel(object):
     def __init__(self, meta_dict, mode='exact'):
         rpc = meta_dict['rpc']
@@ -46,7 +54,10 @@ class RPCModel(object):
     def projection(self, lat, lon, alt):
         require_cuda()
         on_device = any(is_cuda_tensor(a) for a in (lat, lon, alt))
-        if on_device:
+        if on_device and _same_layout(lat, lon, alt):
+            shape = lat.shape
+            la, lo, al = lat, lon, alt
+        elif on_device:
             shape = torch.broadcast_shapes(*(torch.as_tensor(a).shape if not isinstance(a, torch.Tensor) else a.shape
                                              for a in (lat, lon, alt)))
             la, lo, al = (torch.as_tensor(a, dtype=torch.float64, device='cuda').expand(shape).contiguous()
