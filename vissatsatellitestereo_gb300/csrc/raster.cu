@@ -1175,16 +1175,17 @@ constexpr int kMapUnitPx = 8;                   // consecutive pixels of a row p
 // carries a 2-cell halo (the hole fill of the blur's 1-cell halo needs its neighbours);
 // its keys are 32-bit order keys of the float32 heights (0: no point), enough for the
 // nanmax because the heights are float32.  The "first zero" words, needed only when a
-// cell's maximum is a zero, share storage with the epilogue's arrays.
+// cell's maximum is a zero, share storage with the epilogue's arrays.  Column f of the blur input
+// (0: the halo) is kept at fk[][f + 1], so that a lane's columns 2l + 1 and 2l + 2 are one access.
 template <int OW, int OH>
-struct MapTileSmem {
+struct __align__(16) MapTileSmem {
     static constexpr int KW = OW + 4, KH = OH + 4, FW = OW + 2, FH = OH + 2;
     static constexpr int NK = KW * KH, NF = FW * FH;
     unsigned keys[NK];
     union {
         unsigned zw[NK];                    // (2^28 - 1 - first zero's pixel) << 1 | its sign
         struct {
-            float fk[FH][FW];               // hole-filled values: the blur's input
+            float fk[FH][OW + 4];           // hole-filled values: the blur's input
             unsigned short holes[NF];       // empty in-grid cells of the blur input
         } e;
     } u;
@@ -1346,30 +1347,65 @@ __device__ __forceinline__ float median8_keys32(unsigned (&s)[8]) {
 // view's DSM; the same arithmetic as epilogue_tile.  Output rows whose 3x3 windows hold
 // no NaN and no zero take the sorted-column median (bit-identical there); the others run
 // OpenCV's network per cell.  Clears the key tile for the next item.
+//
+// The kernel is issue-bound, and at two pixels per cell most of its slots were spent here, on
+// two-dimensional indexing of single cells, border tests per cell and three loads per column and
+// output.  A warp now walks rows with OW / 32 columns per lane -- staging them with the indices of a
+// row, blurring eight consecutive rows that each load one new row -- and the image's border is
+// copied around the tile once, in the tiles that have one: 416 -> 305 instructions per cell, 107 M cells and
+// 226 M pixels 1.53 -> 1.19 ms.
 template <int OW, int OH>
 __device__ __forceinline__ void map_tile_finish(MapTileSmem<OW, OH> &sm, float *__restrict__ out, int H, int W,
                                                 int r0, int c0) {
     using S = MapTileSmem<OW, OH>;
-    const int tid = threadIdx.x, lane = tid & 31;
+    constexpr int C = OW / 32, kWarps = kMapThreads / 32, kRows = OH / kWarps;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float qnan = __uint_as_float(0x7fffffffu);
-    for (int base = 0; base < S::NF; base += kMapThreads) {
-        const int idx = base + tid;
-        const bool in = idx < S::NF;
-        const int ly = idx / S::FW, lx = idx - ly * S::FW;
-        const bool grid = in && static_cast<unsigned>(r0 - 1 + ly) < static_cast<unsigned>(H) &&
-                          static_cast<unsigned>(c0 - 1 + lx) < static_cast<unsigned>(W);
-        const unsigned k = in ? sm.keys[(ly + 1) * S::KW + lx + 1] : 1u;
-        if (in) {
-            const float f = k ? float_from_key(k) : qnan;
-            sm.u.e.fk[ly][lx] = f;
-            if (grid && k && f == 0.0f) sm.specrow[ly] = 1;
+    float(&fk)[S::FH][OW + 4] = sm.u.e.fk;
+    for (int ly = warp; ly < S::FH; ly += kWarps) {
+        const bool row = static_cast<unsigned>(r0 - 1 + ly) < static_cast<unsigned>(H);
+        const unsigned *src = &sm.keys[(ly + 1) * S::KW + C * lane + 2];
+        unsigned k[C];
+        if constexpr (C == 2) {
+            const uint2 t = *reinterpret_cast<const uint2 *>(src);
+            k[0] = t.x;
+            k[1] = t.y;
+        } else {
+            k[0] = src[0];
         }
-        const unsigned empty = __ballot_sync(0xffffffffu, grid && k == 0u);
-        if (empty) {
+        float f[C];
+        bool hole[C], zero = false;
+#pragma unroll
+        for (int q = 0; q < C; ++q) {
+            const bool grid = row && c0 + C * lane + q < W;
+            f[q] = k[q] ? float_from_key(k[q]) : qnan;
+            hole[q] = grid && k[q] == 0u;
+            zero |= grid && f[q] == 0.0f;
+        }
+        if constexpr (C == 2) *reinterpret_cast<float2 *>(&fk[ly][2 * lane + 2]) = make_float2(f[0], f[1]);
+        else fk[ly][lane + 2] = f[0];
+        if (__any_sync(0xffffffffu, zero) && lane == 0) sm.specrow[ly] = 1;
+        const unsigned e0 = __ballot_sync(0xffffffffu, hole[0]), e1 = C == 2 ? __ballot_sync(0xffffffffu, hole[C - 1]) : 0u;
+        if (e0 | e1) {
             int slot = 0;
-            if (lane == __ffs(empty) - 1) slot = atomicAdd(&sm.n_holes, __popc(empty));
-            slot = __shfl_sync(0xffffffffu, slot, __ffs(empty) - 1);
-            if (grid && k == 0u) sm.u.e.holes[slot + __popc(empty & ((1u << lane) - 1u))] = static_cast<unsigned short>(idx);
+            if (lane == 0) slot = atomicAdd(&sm.n_holes, __popc(e0) + __popc(e1));
+            slot = __shfl_sync(0xffffffffu, slot, 0);
+            const unsigned below = (1u << lane) - 1u;
+            const int idx = ly * S::FW + C * lane + 1;
+            if (hole[0]) sm.u.e.holes[slot + __popc(e0 & below)] = static_cast<unsigned short>(idx);
+            if (C == 2 && hole[C - 1])
+                sm.u.e.holes[slot + __popc(e0) + __popc(e1 & below)] = static_cast<unsigned short>(idx + 1);
+        }
+    }
+    if (tid < 2 * S::FH) {                        // the halo columns 0 and OW + 1
+        const int ly = tid >> 1, lx = (tid & 1) ? OW + 1 : 0;
+        const unsigned k = sm.keys[(ly + 1) * S::KW + lx + 1];
+        const float f = k ? float_from_key(k) : qnan;
+        fk[ly][lx + 1] = f;
+        if (static_cast<unsigned>(r0 - 1 + ly) < static_cast<unsigned>(H) &&
+            static_cast<unsigned>(c0 - 1 + lx) < static_cast<unsigned>(W)) {
+            if (k == 0u) sm.u.e.holes[atomicAdd(&sm.n_holes, 1)] = static_cast<unsigned short>(ly * S::FW + lx);
+            else if (f == 0.0f) sm.specrow[ly] = 1;
         }
     }
     __syncthreads();
@@ -1385,59 +1421,104 @@ __device__ __forceinline__ void map_tile_finish(MapTileSmem<OW, OH> &sm, float *
                 if (dj != 1 || dk != 1) s8[m++] = sm.keys[(ly + dj) * S::KW + lx + dk];
         const unsigned any = s8[0] | s8[1] | s8[2] | s8[3] | s8[4] | s8[5] | s8[6] | s8[7];
         const float f = any ? median8_keys32(s8) : qnan;
-        sm.u.e.fk[ly][lx] = f;
+        fk[ly][lx + 1] = f;
         if (isnan(f) || f == 0.0f) sm.specrow[ly] = 1;
     }
     __syncthreads();
-    for (int i = tid; i < S::NK; i += kMapThreads) sm.keys[i] = 0u;   // dead until the next item
+    for (int i = tid; i < S::NK / 4; i += kMapThreads) reinterpret_cast<uint4 *>(sm.keys)[i] = make_uint4(0u, 0u, 0u, 0u);
+    // the replicated border, in the tiles that reach it: columns first, then whole rows
+    const int col_end = W - c0 + 1, row_end = H - r0 + 1;       // column / row just outside the image
+    if (c0 == 0 || col_end <= OW + 1) {
+        for (int ly = tid; ly < S::FH; ly += kMapThreads) {
+            if (c0 == 0) fk[ly][1] = fk[ly][2];
+            if (col_end <= OW + 1) fk[ly][col_end + 1] = fk[ly][col_end];
+        }
+        __syncthreads();
+    }
+    if (r0 == 0 || row_end <= OH + 1) {
+        for (int lx = tid; lx < OW + 3; lx += kMapThreads) {
+            if (r0 == 0) fk[0][lx] = fk[1][lx];
+            if (row_end <= OH + 1) fk[row_end][lx] = fk[row_end - 1][lx];
+        }
+        if (tid == 0) {
+            if (r0 == 0) sm.specrow[0] = sm.specrow[1];
+            if (row_end <= OH + 1) sm.specrow[row_end] = sm.specrow[row_end - 1];
+        }
+        __syncthreads();
+    }
     const bool line = H == 1 || W == 1;
-    constexpr int HALVES = OW / 32;
-    const float(&fk)[S::FH][S::FW] = sm.u.e.fk;
-    for (int p = tid >> 5; p < OH * HALVES; p += kMapThreads / 32) {
-        const int oy = p / HALVES, h = p - oy * HALVES;
-        const int r = r0 + oy, c = c0 + 32 * h + lane;
-        const int fx = 32 * h + lane + 1;
-        int ya = oy, yb = oy + 1, yc = oy + 2;
-        if (r == 0) ya = yb;
-        if (r == H - 1) yc = yb;
-        if (!line && !(sm.specrow[oy] | sm.specrow[oy + 1] | sm.specrow[oy + 2])) {
-            // sorted-column median: lane owns one column of a 32-column half row; lanes 0
-            // and 31 also sort the halo columns
-            const int xe = lane == 0 ? 32 * h : (lane == 31 ? 32 * h + 33 : fx);
-            float lo, mid, hi, elo, emid, ehi;
-            sort3f(fk[ya][fx], fk[yb][fx], fk[yc][fx], lo, mid, hi);
-            sort3f(fk[ya][xe], fk[yb][xe], fk[yc][xe], elo, emid, ehi);
-            float llo = __shfl_up_sync(0xffffffffu, lo, 1), lmid = __shfl_up_sync(0xffffffffu, mid, 1),
-                  lhi = __shfl_up_sync(0xffffffffu, hi, 1);
-            float rlo = __shfl_down_sync(0xffffffffu, lo, 1), rmid = __shfl_down_sync(0xffffffffu, mid, 1),
-                  rhi = __shfl_down_sync(0xffffffffu, hi, 1);
-            if (lane == 0) { llo = elo; lmid = emid; lhi = ehi; }
-            if (lane == 31) { rlo = elo; rmid = emid; rhi = ehi; }
-            if (c == 0) { llo = lo; lmid = mid; lhi = hi; }           // replicate border
-            if (c == W - 1) { rlo = lo; rmid = mid; rhi = hi; }
-            if (c < W && r < H)
-                out[static_cast<long long>(r) * W + c] =
-                    med3f(fmaxf(fmaxf(llo, lo), rlo), med3f(lmid, mid, rmid), fminf(fminf(lhi, hi), rhi));
-            continue;
-        }
-        if (r >= H || c >= W) continue;
-        int xa = fx - 1, xb = fx, xc = fx + 1;
-        if (c == 0) xa = xb;
-        if (c == W - 1) xc = xb;
-        float v;
-        if (H == 1) {
-            v = cv_median3_line(fk[yb][xa], fk[yb][xb], fk[yb][xc]);
-        } else if (W == 1) {
-            v = cv_median3_line(fk[ya][xb], fk[yb][xb], fk[yc][xb]);
+    const int y0 = warp * kRows, c = c0 + C * lane;
+    // lanes 0 and 31 also follow the halo columns
+    const int own = C * lane + 2, edge = lane == 0 ? 1 : (lane == 31 ? OW + 2 : own);
+    float u[C + 1], v[C + 1];
+    auto load = [&](int y, float (&x)[C + 1]) {
+        if constexpr (C == 2) {
+            const float2 t = *reinterpret_cast<const float2 *>(&fk[y][own]);
+            x[0] = t.x;
+            x[1] = t.y;
         } else {
-            const float p0 = fk[ya][xa], p1 = fk[ya][xb], p2 = fk[ya][xc], p3 = fk[yb][xa], p4 = fk[yb][xb],
-                        p5 = fk[yb][xc], p6 = fk[yc][xa], p7 = fk[yc][xb], p8 = fk[yc][xc];
-            // all nine NaN (the epilogue's own NaN): every exchange moves equal bits
-            const bool all_nan = isnan(p0) & isnan(p1) & isnan(p2) & isnan(p3) & isnan(p4) & isnan(p5) & isnan(p6) &
-                                 isnan(p7) & isnan(p8);
-            v = all_nan ? qnan : cv_median9(cv_vector_column(c, W), p0, p1, p2, p3, p4, p5, p6, p7, p8);
+            x[0] = fk[y][own];
         }
-        out[static_cast<long long>(r) * W + c] = v;
+        x[C] = fk[y][edge];
+    };
+    load(y0, u);
+    load(y0 + 1, v);
+    bool odd_u = sm.specrow[y0] != 0, odd_v = sm.specrow[y0 + 1] != 0;
+    float *dst = out + static_cast<long long>(r0 + y0) * W + c;
+#pragma unroll 2
+    for (int k = 0; k < kRows; ++k, dst += W) {
+        const int oy = y0 + k;
+        if (r0 + oy >= H) break;
+        float w[C + 1];
+        load(oy + 2, w);
+        const bool odd_w = sm.specrow[oy + 2] != 0;
+        float m[C];
+        if (!line && !(odd_u | odd_v | odd_w)) {
+            float lo[C + 1], mid[C + 1], hi[C + 1];
+#pragma unroll
+            for (int q = 0; q <= C; ++q) sort3f(u[q], v[q], w[q], lo[q], mid[q], hi[q]);
+            float llo = __shfl_up_sync(0xffffffffu, lo[C - 1], 1), lmid = __shfl_up_sync(0xffffffffu, mid[C - 1], 1),
+                  lhi = __shfl_up_sync(0xffffffffu, hi[C - 1], 1);
+            float rlo = __shfl_down_sync(0xffffffffu, lo[0], 1), rmid = __shfl_down_sync(0xffffffffu, mid[0], 1),
+                  rhi = __shfl_down_sync(0xffffffffu, hi[0], 1);
+            if (lane == 0) { llo = lo[C]; lmid = mid[C]; lhi = hi[C]; }
+            if (lane == 31) { rlo = lo[C]; rmid = mid[C]; rhi = hi[C]; }
+#pragma unroll
+            for (int q = 0; q < C; ++q) {
+                const float l0 = q ? lo[0] : llo, l1 = q ? mid[0] : lmid, l2 = q ? hi[0] : lhi;
+                const float q0 = q < C - 1 ? lo[C - 1] : rlo, q1 = q < C - 1 ? mid[C - 1] : rmid,
+                            q2 = q < C - 1 ? hi[C - 1] : rhi;
+                m[q] = med3f(fmaxf(fmaxf(l0, lo[q]), q0), med3f(l1, mid[q], q1), fminf(fminf(l2, hi[q]), q2));
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < C; ++q) {
+                const int x = own + q;
+                if (H == 1) {
+                    m[q] = cv_median3_line(fk[oy + 1][x - 1], fk[oy + 1][x], fk[oy + 1][x + 1]);
+                } else if (W == 1) {
+                    m[q] = cv_median3_line(fk[oy][x], fk[oy + 1][x], fk[oy + 2][x]);
+                } else {
+                    const float p0 = fk[oy][x - 1], p1 = fk[oy][x], p2 = fk[oy][x + 1], p3 = fk[oy + 1][x - 1],
+                                p4 = fk[oy + 1][x], p5 = fk[oy + 1][x + 1], p6 = fk[oy + 2][x - 1], p7 = fk[oy + 2][x],
+                                p8 = fk[oy + 2][x + 1];
+                    // all nine NaN (the epilogue's own NaN): every exchange moves equal bits
+                    const bool all_nan = isnan(p0) & isnan(p1) & isnan(p2) & isnan(p3) & isnan(p4) & isnan(p5) &
+                                         isnan(p6) & isnan(p7) & isnan(p8);
+                    m[q] = all_nan ? qnan : cv_median9(cv_vector_column(c + q, W), p0, p1, p2, p3, p4, p5, p6, p7, p8);
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < C; ++q)
+            if (c + q < W) dst[q] = m[q];
+#pragma unroll
+        for (int q = 0; q <= C; ++q) {
+            u[q] = v[q];
+            v[q] = w[q];
+        }
+        odd_u = odd_v;
+        odd_v = odd_w;
     }
 }
 
