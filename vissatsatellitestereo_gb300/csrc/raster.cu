@@ -659,81 +659,106 @@ int launch_blur(const T *in, float *out, long long h, long long w, long long n_i
 }
 
 // ---- fused produce_dsm epilogue: keys -> nanmax -> hole fill -> float32 -> blur ---------
-// One 32x32 output tile per CTA of 32x8 threads (4 outputs per thread, rows ty + 8j).  The
-// key tile carries a 2-cell halo (hole fill needs the 3x3 neighbourhood of each blurred
-// cell's 3x3 neighbourhood); the hole-filled float32 values are staged for the blur;
-// 32-bit indexing (grid dimensions < 2^31).
-constexpr int TX = 32, TY = 8, TILE_Y = 32;
-constexpr int RAW_W = TX + 4, RAW_H = TILE_Y + 4, FK_W = TX + 2, FK_H = TILE_Y + 2;
+// One 64 x 32 output tile per CTA of 8 warps.  The key tile carries a 2-cell halo (hole fill needs
+// the 3x3 neighbourhood of each blurred cell's 3x3 neighbourhood); the hole-filled float32 values
+// are staged for the blur; 32-bit indexing (grid dimensions < 2^31).
+//
+// Issue-bound: an earlier form with 32 x 32 tiles and one cell per thread spent 198 instructions per cell
+// on two-dimensional indices, border tests and three loads per column and output.  A warp walks
+// rows, two columns per lane, with all of its keys loaded before the first is used (the ballots order
+// the steps); the blur takes four consecutive rows, each of which loads one new row; the image's
+// border is copied around the tile in the tiles that have one: 120 instructions.  Ten views of 1503 x 1409 cells, with their binning: 516 us,
+// 487 us (five CTAs per SM; four 490, six with spills 511, 64 x 16 tiles 494).
+constexpr int TX = 32, TY = 8;                          // the CTA: a warp per threadIdx.y
+constexpr int kTileW = 64, kTileH = 32;
+constexpr int RAW_W = kTileW + 4, RAW_H = kTileH + 4, FK_W = kTileW + 2, FK_H = kTileH + 2;
 
-// Shared-memory working set of one epilogue tile.
-struct EpilogueSmem {
-    unsigned long long raw[RAW_H * RAW_W];   // 0: empty cell or outside the image
-    float fk[FK_H][FK_W];                    // hole-filled cells as float32 (the blur's input)
+// Shared-memory working set of one epilogue tile.  Column f of the blur input (0: the halo) is at
+// fk[][f + 1] and raw[][f + 1], so that a lane's columns 2l + 1 and 2l + 2 are one access.
+struct __align__(16) EpilogueSmem {
+    unsigned long long raw[RAW_H][RAW_W];    // 0: empty cell or outside the image
+    float fk[FK_H][RAW_W];                   // hole-filled cells as float32 (the blur's input)
     unsigned short holes[FK_H * FK_W];
     int n_holes;
+    unsigned char special[FK_H];             // a NaN or a zero in this row of the blur input
 };
 
-// One 32 x 32 output tile: keys (decoded by `dec(key, cell)`, which resolves zero keys to
-// their signed value) -> nanmax values -> hole fill -> float32 -> 3x3 median blur.
-// Threads are TX x TY; the caller synchronises before reusing `sm`.  With `next_keys` it
-// also clears this tile of the idle key grid (the next view's), which nobody reads
-// concurrently, so no per-view memset is needed.  Empty cells (a few percent) are
-// collected in a shared list and filled by consecutive threads, so the hole-fill work does
-// not diverge every warp that happens to hold one.
-// AHEAD: all of a thread's keys are loaded before the first is used -- the ballots order the steps,
-// and one load per step makes a tile wait for L2 six times (1503 x 1409 cells: 21.5 us,
-// 19.5 us; needs 40 registers, which raster_pipe_kernel's tiles do not have).
-template <bool AHEAD, class Dec>
+// One tile: keys (decoded by `dec(key, cell)`, which resolves zero keys to their signed value)
+// -> nanmax values -> hole fill -> float32 -> 3x3 median blur.  Threads are TX x TY; the caller
+// synchronises before reusing `sm`.  With `next_keys` it also clears this tile of the idle key
+// grid (the next view's), which nobody reads concurrently, so no per-view memset is needed.
+// Empty cells (a few percent) are collected in a shared list and filled by consecutive
+// threads, so the hole-fill work does not diverge every warp that happens to hold one.
+template <class Dec>
 __device__ __forceinline__ void epilogue_tile(const unsigned long long *__restrict__ vk, const Dec &dec,
                                               float *__restrict__ out, unsigned long long *__restrict__ next_keys,
                                               int H, int W, int r0, int c0, EpilogueSmem &sm) {
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx, lane = tid & 31;
-    bool special = false;          // this thread staged a NaN or a zero
-    if (tid == 0) sm.n_holes = 0;
-    // one pass over the key block: stage the keys (the hole fill reads the neighbours) and,
-    // for the blur input's cells, the float32 values and the list of empty cells
-    constexpr int kSteps = (RAW_H * RAW_W + TX * TY - 1) / (TX * TY), kGroup = AHEAD ? kSteps : 1;
-    unsigned long long key[kGroup];
-#pragma unroll(kGroup)
-    for (int q = 0; q < kSteps; ++q) {
-        const int i = q * (TX * TY) + tid;
-        const bool in = i < RAW_H * RAW_W;
-        const int ly = i / RAW_W, lx = i - ly * RAW_W;
-        if (q % kGroup == 0) {
+    constexpr int kSteps = (RAW_H + TY - 1) / TY, kRows = kTileH / TY;
+    const int lane = threadIdx.x, warp = threadIdx.y, tid = warp * TX + lane;
+    const float qnan = __uint_as_float(0x7fffffffu);
+    const int c = c0 + 2 * lane;                       // the lane's columns c and c + 1
+    const bool in_a = c < W, in_b = c + 1 < W;
+    unsigned long long key[kSteps][2], halo = kEmptyKey;
 #pragma unroll
-            for (int g = 0; g < kGroup; ++g) {
-                const int j = (q + g) * (TX * TY) + tid, jy = j / RAW_W, jx = j - jy * RAW_W;
-                const int r = r0 + jy - 2, c = c0 + jx - 2;
-                key[g] = kEmptyKey;
-                if (j < RAW_H * RAW_W && static_cast<unsigned>(r) < static_cast<unsigned>(H) &&
-                    static_cast<unsigned>(c) < static_cast<unsigned>(W))
-                    key[g] = vk[static_cast<long long>(r) * W + c];
-            }
-            if (q == 0) __syncthreads();             // n_holes
+    for (int q = 0; q < kSteps; ++q) {
+        const int i = warp + q * TY, r = r0 - 2 + i;
+        key[q][0] = key[q][1] = kEmptyKey;
+        if (i < RAW_H && static_cast<unsigned>(r) < static_cast<unsigned>(H)) {
+            const unsigned long long *p = vk + static_cast<long long>(r) * W + c;
+            if (in_a) key[q][0] = __ldg(p);
+            if (in_b) key[q][1] = __ldg(p + 1);
         }
-        unsigned long long k = key[q % kGroup];
-        if (k == kZeroKey) k = dec(k, static_cast<long long>(r0 + ly - 2) * W + (c0 + lx - 2));
-        if (in) sm.raw[i] = k;
-        const bool inner = in && ly >= 1 && ly <= RAW_H - 2 && lx >= 1 && lx <= RAW_W - 2;
-        if (inner && k != kEmptyKey) {
-            // the conversion instruction (IEEE round-to-nearest, like f64_to_f32): one issue
-            // slot on the narrow FP64 pipe instead of a dozen integer instructions -- here,
-            // at ~1.3 conversions per cell, the issue slots are the scarcer resource
-            const float f = __double2float_rn(double_from_key(k));
-            sm.fk[ly - 1][lx - 1] = f;
-            special |= isnan(f) || f == 0.0f;
+    }
+    const int hi = tid >> 2, hj = (tid & 2) ? kTileW + (tid & 3) : (tid & 3);   // raw columns 0, 1, 66, 67
+    const int hr = r0 - 2 + hi, hc = c0 - 2 + hj;
+    const bool halo_in = tid < 4 * RAW_H && static_cast<unsigned>(hr) < static_cast<unsigned>(H) &&
+                         static_cast<unsigned>(hc) < static_cast<unsigned>(W);
+    if (halo_in) halo = __ldg(vk + static_cast<long long>(hr) * W + hc);
+    if (tid == 0) sm.n_holes = 0;
+    if (tid < FK_H) sm.special[tid] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kSteps; ++q) {
+        const int i = warp + q * TY, r = r0 - 2 + i;
+        if (i >= RAW_H) break;
+        unsigned long long ka = key[q][0], kb = key[q][1];
+        const bool row = static_cast<unsigned>(r) < static_cast<unsigned>(H);
+        if (ka == kZeroKey || kb == kZeroKey) {
+            const long long cell = static_cast<long long>(r) * W + c;
+            ka = dec(ka, cell);
+            kb = dec(kb, cell + 1);
         }
-        // warp-aggregated append of the empty cells to the hole list
-        const bool hole = inner && k == kEmptyKey;
-        const unsigned empty = __ballot_sync(0xffffffffu, hole);
-        if (empty) {
+        *reinterpret_cast<ulonglong2 *>(&sm.raw[i][2 * lane + 2]) = make_ulonglong2(ka, kb);
+        if (i < 1 || i > FK_H) continue;
+        // the conversion instruction (IEEE round-to-nearest, like f64_to_f32): one issue slot on the
+        // narrow FP64 pipe instead of a dozen integer instructions -- here the issue slots are the
+        // scarcer resource (an empty cell's key decodes to a NaN)
+        const float fa = __double2float_rn(double_from_key(ka)), fb = __double2float_rn(double_from_key(kb));
+        *reinterpret_cast<float2 *>(&sm.fk[i - 1][2 * lane + 2]) = make_float2(fa, fb);
+        if (__all_sync(0xffffffffu, fabsf(fa) > 0.0f && fabsf(fb) > 0.0f) || !row) continue;
+        const bool ha = in_a && ka == kEmptyKey, hb = in_b && kb == kEmptyKey;
+        if (__any_sync(0xffffffffu, fa == 0.0f || fb == 0.0f) && lane == 0) sm.special[i - 1] = 1;
+        const unsigned ea = __ballot_sync(0xffffffffu, ha), eb = __ballot_sync(0xffffffffu, hb);
+        if (ea | eb) {
             int slot = 0;
-            if (lane == __ffs(empty) - 1) slot = atomicAdd(&sm.n_holes, __popc(empty));
-            slot = __shfl_sync(0xffffffffu, slot, __ffs(empty) - 1);
-            if (hole)
-                sm.holes[slot + __popc(empty & ((1u << lane) - 1u))] =
-                    static_cast<unsigned short>((ly - 1) * FK_W + (lx - 1));
+            if (lane == 0) slot = atomicAdd(&sm.n_holes, __popc(ea) + __popc(eb));
+            slot = __shfl_sync(0xffffffffu, slot, 0);
+            const unsigned below = (1u << lane) - 1u;
+            const int idx = (i - 1) * FK_W + 2 * lane + 1;
+            if (ha) sm.holes[slot + __popc(ea & below)] = static_cast<unsigned short>(idx);
+            if (hb) sm.holes[slot + __popc(ea) + __popc(eb & below)] = static_cast<unsigned short>(idx + 1);
+        }
+    }
+    if (tid < 4 * RAW_H) {
+        if (halo == kZeroKey) halo = dec(halo, static_cast<long long>(hr) * W + hc);
+        sm.raw[hi][hj] = halo;
+        if (hi >= 1 && hi <= FK_H && (hj == 1 || hj == FK_W)) {      // columns 0 and FK_W - 1 of the blur input
+            const float f = __double2float_rn(double_from_key(halo));
+            sm.fk[hi - 1][hj] = f;
+            if (halo_in && halo == kEmptyKey)
+                sm.holes[atomicAdd(&sm.n_holes, 1)] = static_cast<unsigned short>((hi - 1) * FK_W + hj - 1);
+            else if (halo_in && f == 0.0f)
+                sm.special[hi - 1] = 1;
         }
     }
     __syncthreads();
@@ -742,71 +767,109 @@ __device__ __forceinline__ void epilogue_tile(const unsigned long long *__restri
         const int ly = i / FK_W, lx = i - ly * FK_W;
         unsigned long long s8[8];
         int m = 0;
+        bool any = false;
 #pragma unroll
         for (int dj = 0; dj < 3; ++dj)
 #pragma unroll
             for (int dk = 0; dk < 3; ++dk)
-                if (dj != 1 || dk != 1) s8[m++] = sm.raw[(ly + dj) * RAW_W + lx + dk];
-        bool any = false;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) any |= s8[q] != kEmptyKey;
-        const float f = any ? f64_to_f32(median8_keys(s8)) : __uint_as_float(0x7fffffffu);
-        sm.fk[ly][lx] = f;
-        special |= isnan(f) || f == 0.0f;
+                if (dj != 1 || dk != 1) {
+                    s8[m] = sm.raw[ly + dj][lx + dk];
+                    any |= s8[m++] != kEmptyKey;
+                }
+        float f = qnan;
+        if (any) f = f64_to_f32(median8_keys(s8));
+        sm.fk[ly][lx + 1] = f;
+        if (isnan(f) || f == 0.0f) sm.special[ly] = 1;
     }
-    // A tile whose staged values hold no NaN and no zero takes the sorted-column median:
-    // with no NaN and no -0/+0 pair every compare-exchange order yields the same value, so
-    // OpenCV's network and the column form agree bit for bit.
-    const bool exact_net = __syncthreads_or(special) != 0 || H == 1 || W == 1;
-    const int c = c0 + tx;
-    int xa = tx, xb = tx + 1, xc = tx + 2;
-    if (c == 0) xa = xb;                 // replicate border: clamp the neighbours into the image
-    if (c == W - 1) xc = xb;
-    if (!exact_net) {
-        // lane tx owns fk column tx + 1; lanes 0 and 31 also sort the halo columns 0 and 33
-        const int xe = tx == 0 ? 0 : (tx == TX - 1 ? TX + 1 : tx + 1);
-#pragma unroll
-        for (int j = 0; j < TILE_Y / TY; ++j) {
-            const int oy = ty + TY * j, r = r0 + oy;
-            int ya = oy, yb = oy + 1, yc = oy + 2;
-            if (r == 0) ya = yb;
-            if (r == H - 1) yc = yb;
-            float lo, mid, hi, elo, emid, ehi;
-            sort3f(sm.fk[ya][tx + 1], sm.fk[yb][tx + 1], sm.fk[yc][tx + 1], lo, mid, hi);
-            sort3f(sm.fk[ya][xe], sm.fk[yb][xe], sm.fk[yc][xe], elo, emid, ehi);
-            float llo = __shfl_up_sync(0xffffffffu, lo, 1), lmid = __shfl_up_sync(0xffffffffu, mid, 1),
-                  lhi = __shfl_up_sync(0xffffffffu, hi, 1);
-            float rlo = __shfl_down_sync(0xffffffffu, lo, 1), rmid = __shfl_down_sync(0xffffffffu, mid, 1),
-                  rhi = __shfl_down_sync(0xffffffffu, hi, 1);
-            if (tx == 0) { llo = elo; lmid = emid; lhi = ehi; }
-            if (tx == TX - 1) { rlo = elo; rmid = emid; rhi = ehi; }
-            if (c == 0) { llo = lo; lmid = mid; lhi = hi; }           // replicate border
-            if (c == W - 1) { rlo = lo; rmid = mid; rhi = hi; }
-            if (c >= W || r >= H) continue;
-            const long long cell = static_cast<long long>(r) * W + c;
-            if (next_keys) next_keys[cell] = kEmptyKey;
-            out[cell] = med3f(fmaxf(fmaxf(llo, lo), rlo), med3f(lmid, mid, rmid), fminf(fminf(lhi, hi), rhi));
+    __syncthreads();
+    // the replicated border, in the tiles that reach it: columns first, then whole rows
+    const int col_end = W - c0 + 1, row_end = H - r0 + 1;       // column / row just outside the image
+    if (c0 == 0 || col_end < FK_W) {
+        if (tid < FK_H) {
+            if (c0 == 0) sm.fk[tid][1] = sm.fk[tid][2];
+            if (col_end < FK_W) sm.fk[tid][col_end + 1] = sm.fk[tid][col_end];
         }
-        return;
+        __syncthreads();
     }
-    if (c >= W) return;
-    const bool vec = cv_vector_column(c, W);
+    if (r0 == 0 || row_end < FK_H) {
+        if (tid < RAW_W - 1) {
+            if (r0 == 0) sm.fk[0][tid] = sm.fk[1][tid];
+            if (row_end < FK_H) sm.fk[row_end][tid] = sm.fk[row_end - 1][tid];
+        }
+        if (tid == 0) {
+            if (r0 == 0) sm.special[0] = sm.special[1];
+            if (row_end < FK_H) sm.special[row_end] = sm.special[row_end - 1];
+        }
+        __syncthreads();
+    }
+    // Rows whose three-row window holds no NaN and no zero take the sorted-column median: with no NaN and
+    // no -0/+0 pair every compare-exchange order yields the same value, so OpenCV's network and the
+    // column form agree bit for bit.
+    const bool line = H == 1 || W == 1;
+    const int y0 = warp * kRows, own = 2 * lane + 2, edge = lane == 0 ? 1 : (lane == 31 ? FK_W : own);
+    float u[3], v[3];                                    // the lane's columns and, for lanes 0 and 31, the halo's
+    auto load = [&](int y, float (&x)[3]) {
+        const float2 t = *reinterpret_cast<const float2 *>(&sm.fk[y][own]);
+        x[0] = t.x;
+        x[1] = t.y;
+        x[2] = sm.fk[y][edge];
+    };
+    load(y0, u);
+    load(y0 + 1, v);
+    bool odd_u = sm.special[y0] != 0, odd_v = sm.special[y0 + 1] != 0;
+    float *dst = out + static_cast<long long>(r0 + y0) * W + c;
+    unsigned long long *clear = next_keys ? next_keys + static_cast<long long>(r0 + y0) * W + c : nullptr;
+#pragma unroll 2
+    for (int k = 0; k < kRows; ++k, dst += W) {
+        const int oy = y0 + k;
+        if (r0 + oy >= H) break;
+        float w[3];
+        load(oy + 2, w);
+        const bool odd_w = sm.special[oy + 2] != 0;
+        float m0, m1;
+        if (!line && !(odd_u | odd_v | odd_w)) {
+            float lo[3], mid[3], hi3[3];
 #pragma unroll
-    for (int j = 0; j < TILE_Y / TY; ++j) {
-        const int oy = ty + TY * j, r = r0 + oy;
-        if (r >= H) break;
-        int ya = oy, yb = oy + 1, yc = oy + 2;
-        if (r == 0) ya = yb;
-        if (r == H - 1) yc = yb;
-        const long long cell = static_cast<long long>(r) * W + c;
-        if (next_keys) next_keys[cell] = kEmptyKey;
-        if (H == 1)
-            out[cell] = cv_median3_line(sm.fk[yb][xa], sm.fk[yb][xb], sm.fk[yb][xc]);
-        else if (W == 1)
-            out[cell] = cv_median3_line(sm.fk[ya][xb], sm.fk[yb][xb], sm.fk[yc][xb]);
-        else
-            out[cell] = cv_median9(vec, sm.fk[ya][xa], sm.fk[ya][xb], sm.fk[ya][xc], sm.fk[yb][xa], sm.fk[yb][xb],
-                                   sm.fk[yb][xc], sm.fk[yc][xa], sm.fk[yc][xb], sm.fk[yc][xc]);
+            for (int q = 0; q < 3; ++q) sort3f(u[q], v[q], w[q], lo[q], mid[q], hi3[q]);
+            float llo = __shfl_up_sync(0xffffffffu, lo[1], 1), lmid = __shfl_up_sync(0xffffffffu, mid[1], 1),
+                  lhi = __shfl_up_sync(0xffffffffu, hi3[1], 1);
+            float rlo = __shfl_down_sync(0xffffffffu, lo[0], 1), rmid = __shfl_down_sync(0xffffffffu, mid[0], 1),
+                  rhi = __shfl_down_sync(0xffffffffu, hi3[0], 1);
+            if (lane == 0) { llo = lo[2]; lmid = mid[2]; lhi = hi3[2]; }
+            if (lane == 31) { rlo = lo[2]; rmid = mid[2]; rhi = hi3[2]; }
+            m0 = med3f(fmaxf(fmaxf(llo, lo[0]), lo[1]), med3f(lmid, mid[0], mid[1]), fminf(fminf(lhi, hi3[0]), hi3[1]));
+            m1 = med3f(fmaxf(fmaxf(lo[0], lo[1]), rlo), med3f(mid[0], mid[1], rmid), fminf(fminf(hi3[0], hi3[1]), rhi));
+        } else {
+            float m[2];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int x = own + q;
+                const float p0 = sm.fk[oy][x - 1], p1 = sm.fk[oy][x], p2 = sm.fk[oy][x + 1], p3 = sm.fk[oy + 1][x - 1],
+                            p4 = sm.fk[oy + 1][x], p5 = sm.fk[oy + 1][x + 1], p6 = sm.fk[oy + 2][x - 1],
+                            p7 = sm.fk[oy + 2][x], p8 = sm.fk[oy + 2][x + 1];
+                const bool all_nan = isnan(p0) & isnan(p1) & isnan(p2) & isnan(p3) & isnan(p4) & isnan(p5) & isnan(p6) &
+                                     isnan(p7) & isnan(p8);
+                if (H == 1) m[q] = cv_median3_line(p3, p4, p5);
+                else if (W == 1) m[q] = cv_median3_line(p1, p4, p7);
+                else m[q] = all_nan ? qnan : cv_median9(cv_vector_column(c + q, W), p0, p1, p2, p3, p4, p5, p6, p7, p8);
+            }
+            m0 = m[0];
+            m1 = m[1];
+        }
+        if (in_a) dst[0] = m0;
+        if (in_b) dst[1] = m1;
+        if (next_keys) {
+            if (in_a) clear[0] = kEmptyKey;
+            if (in_b) clear[1] = kEmptyKey;
+            clear += W;
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            u[q] = v[q];
+            v[q] = w[q];
+        }
+        odd_u = odd_v;
+        odd_v = odd_w;
     }
 }
 
@@ -819,20 +882,20 @@ struct PointsZeroDecoder {
     }
 };
 
-__global__ void __launch_bounds__(TX *TY) dsm_epilogue_kernel(
+__global__ void __launch_bounds__(TX *TY, 5) dsm_epilogue_kernel(
     const unsigned long long *__restrict__ vk, const unsigned long long *__restrict__ first,
     const double *__restrict__ pts, float *__restrict__ out, unsigned long long *__restrict__ next_keys, int H,
     int W) {
     chain_wait();
     __shared__ EpilogueSmem sm;
-    epilogue_tile<true>(vk, PointsZeroDecoder{first, pts}, out, next_keys, H, W, blockIdx.y * TILE_Y, blockIdx.x * TX, sm);
+    epilogue_tile(vk, PointsZeroDecoder{first, pts}, out, next_keys, H, W, blockIdx.y * kTileH, blockIdx.x * kTileW, sm);
 }
 
 // ---- pipelined rasterisation: view v's binning and view v-1's epilogue in one launch -----
 // The binning streams the points from HBM and waits on loads; the epilogue works on an
 // L2-resident key grid and is issue-bound.  Launched one after the other they barely
 // overlap (the binning's resident wave fills every SM until its tail), so one launch
-// carries both: its work items -- chunks of view v's points and 32x32 tiles of view v-1's
+// carries both: its work items -- chunks of view v's points and tiles of view v-1's
 // epilogue, interleaved evenly -- are handed out by a device counter, so every SM runs a
 // mix of both kinds until the launch drains.  The epilogue's inputs (view v-1's key grid
 // and first-zero words) were completed by the previous launch on the same stream; nothing
@@ -855,9 +918,10 @@ struct PipeEpi {          // view v-1's epilogue (n_tiles = 0: none)
     long long n_tiles;
 };
 
-// MINB: resident CTAs per SM the registers are budgeted for (6: 40 registers, 5: 48).
-template <bool FLIP_ROW, bool FLIP_COL, int MINB>
-__global__ void __launch_bounds__(TX *TY, MINB) raster_pipe_kernel(const double *__restrict__ pts, PipeBin bin,
+// Registers for five CTAs per SM (48; with six, 40 and spills: ten views of 1503 x 1409 cells 660 us
+// against 508).
+template <bool FLIP_ROW, bool FLIP_COL>
+__global__ void __launch_bounds__(TX *TY, 5) raster_pipe_kernel(const double *__restrict__ pts, PipeBin bin,
                                                                     PipeEpi epi, unsigned *__restrict__ counter) {
     chain_wait();
     __shared__ EpilogueSmem sm;
@@ -890,8 +954,8 @@ __global__ void __launch_bounds__(TX *TY, MINB) raster_pipe_kernel(const double 
         if (code >= total) break;
         if (code >= 0) {
             const int ty = static_cast<int>(code / epi.tiles_x), tx = static_cast<int>(code - static_cast<long long>(ty) * epi.tiles_x);
-            epilogue_tile<false>(epi.keys, PointsZeroDecoder{epi.first, pts}, epi.out, epi.clear, epi.H, epi.W, ty * TILE_Y,
-                          tx * TX, sm);
+            epilogue_tile(epi.keys, PointsZeroDecoder{epi.first, pts}, epi.out, epi.clear, epi.H, epi.W, ty * kTileH,
+                          tx * kTileW, sm);
         } else {
             const long long c0 = begin + (-1 - code) * kChunkPoints;
 #pragma unroll 1
@@ -1690,7 +1754,7 @@ extern "C" int vs_dsm_from_points(const double *points, const int64_t *offsets, 
     if (s != VS_OK) return s;
     // per-view counts live on the device: launch for a full GPU and let the grid stride
     const long long launch_points = static_cast<long long>(sm_count()) * 8 * 256 * kPts;
-    const dim3 egrid(static_cast<unsigned>(ceil_div(xsize, TX)), static_cast<unsigned>(ceil_div(ysize, TILE_Y)));
+    const dim3 egrid(static_cast<unsigned>(ceil_div(xsize, kTileW)), static_cast<unsigned>(ceil_div(ysize, kTileH)));
     for (int v = 0; v < n_views; ++v) {
         unsigned long long *cur = w.keys[v & 1], *nxt = (v + 1 < n_views) ? w.keys[(v + 1) & 1] : nullptr;
         s = bin_launch(points, reinterpret_cast<const long long *>(offsets), v, 0, launch_points, tb, cur, w.first, st);
@@ -1821,7 +1885,7 @@ extern "C" int vs_dsm_from_points_host(const double *host_points, const int64_t 
         set_error("vs_dsm_from_points_host: cudaEventCreate failed");
         return VS_ERR_CUDA;
     }
-    const dim3 egrid(static_cast<unsigned>(ceil_div(xsize, TX)), static_cast<unsigned>(ceil_div(ysize, TILE_Y)));
+    const dim3 egrid(static_cast<unsigned>(ceil_div(xsize, kTileW)), static_cast<unsigned>(ceil_div(ysize, kTileH)));
     // the copy stream starts after the work already queued on `stream` (tables, clears)
     if (cudaEventRecord(freed[0], st) != cudaSuccess || cudaStreamWaitEvent(cs, freed[0], 0) != cudaSuccess)
         s = VS_ERR_CUDA;
@@ -1891,7 +1955,7 @@ extern "C" int vs_dsm_from_points_overlap(const double *points, const int64_t *o
     if (s == VS_OK) s = clear(w.keys[0], w.cleared, st);
     if (s != VS_OK) return s;
     const long long launch_points = static_cast<long long>(sm_count()) * 8 * 256 * kPts;
-    const dim3 egrid(static_cast<unsigned>(ceil_div(xsize, TX)), static_cast<unsigned>(ceil_div(ysize, TILE_Y)));
+    const dim3 egrid(static_cast<unsigned>(ceil_div(xsize, kTileW)), static_cast<unsigned>(ceil_div(ysize, kTileH)));
     auto cuda_ok = [](cudaError_t e) {
         if (e == cudaSuccess) return true;
         set_error("stream ordering failed: %s", cudaGetErrorString(e));
@@ -1929,12 +1993,11 @@ extern "C" int vs_dsm_from_points_overlap(const double *points, const int64_t *o
 // bin(v) fills K[v%3]; epilogue(v-1) reads K[(v-1)%3] and clears K[(v+1)%3], which
 // epilogue(v-2) finished reading in the previous launch; the first-zero words alternate.
 // One counter per launch (cleared once per call) hands out the work items.
-template <int MINB>
 static void launch_pipe(bool flip_row, bool flip_col, unsigned gx, cudaStream_t st, const double *points,
                         const vs::PipeBin &b, const vs::PipeEpi &e, unsigned *counter, size_t key_bytes) {
     using namespace vs;
-    auto kern = flip_row ? (flip_col ? raster_pipe_kernel<true, true, MINB> : raster_pipe_kernel<true, false, MINB>)
-                         : (flip_col ? raster_pipe_kernel<false, true, MINB> : raster_pipe_kernel<false, false, MINB>);
+    auto kern = flip_row ? (flip_col ? raster_pipe_kernel<true, true> : raster_pipe_kernel<true, false>)
+                         : (flip_col ? raster_pipe_kernel<false, true> : raster_pipe_kernel<false, false>);
     launch_with_key_window(kern, dim3(gx), dim3(TX, TY), st, b.keys, b.active ? key_bytes : 0, points, b, e, counter);
 }
 
@@ -1974,13 +2037,13 @@ extern "C" int vs_dsm_from_points_pipelined(const double *points, const int64_t 
     if (s == VS_OK) s = clear(w.keys[0], w.cleared, st);
     if (s == VS_OK) s = clear(counters, sizeof(unsigned) * (static_cast<size_t>(n_views) + 1), st);
     if (s != VS_OK) return s;
-    const int tiles_x = static_cast<int>(ceil_div(xsize, TX));
-    const long long n_tiles = static_cast<long long>(tiles_x) * ceil_div(ysize, TILE_Y);
+    const int tiles_x = static_cast<int>(ceil_div(xsize, kTileW));
+    const long long n_tiles = static_cast<long long>(tiles_x) * ceil_div(ysize, kTileH);
     if (!fast_binning(tb)) {
         // points outside the fast path's precondition: the literal FP64 binning, then the
         // epilogue, view by view (same results)
         const long long launch_points = static_cast<long long>(sm_count()) * 8 * 256 * kPts;
-        const dim3 egrid(static_cast<unsigned>(tiles_x), static_cast<unsigned>(ceil_div(ysize, TILE_Y)));
+        const dim3 egrid(static_cast<unsigned>(tiles_x), static_cast<unsigned>(ceil_div(ysize, kTileH)));
         for (int v = 0; v < n_views; ++v) {
             s = bin_launch(points, reinterpret_cast<const long long *>(offsets), v, 0, launch_points, tb, w.keys[v % 3],
                            w.first[v & 1], st);
@@ -1996,18 +2059,15 @@ extern "C" int vs_dsm_from_points_pipelined(const double *points, const int64_t 
     FastAxis fa[2];
     fast_axes(tb, fa);
     const bool flip_row = !tb.row.neg, flip_col = tb.col.neg != 0;
-    // a cap of 5 or fewer CTAs per SM takes the 48-register build, which spills nothing
-    const bool narrow = g_bin_ctas_per_sm > 0 && g_bin_ctas_per_sm <= 5;
-    static int resident[2] = {0, 0};
-    if (!resident[narrow]) {
+    static int resident = 0;
+    if (!resident) {
         int per_sm = 0;
-        const cudaError_t e = narrow ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                                           &per_sm, raster_pipe_kernel<true, false, 5>, TX * TY, 0)
-                                     : cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                                           &per_sm, raster_pipe_kernel<true, false, 6>, TX * TY, 0);
-        resident[narrow] = (e == cudaSuccess && per_sm > 0) ? per_sm : 4;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, raster_pipe_kernel<true, false>, TX * TY, 0) !=
+                cudaSuccess || per_sm <= 0)
+            per_sm = 4;
+        resident = per_sm;
     }
-    const int per_sm = g_bin_ctas_per_sm > 0 ? std::min(g_bin_ctas_per_sm, resident[narrow]) : resident[narrow];
+    const int per_sm = g_bin_ctas_per_sm > 0 ? std::min(g_bin_ctas_per_sm, resident) : resident;
     // the views' point counts stay on the device: every launch is one resident wave, and
     // its CTAs derive the chunk count from the offsets
     const unsigned gx = static_cast<unsigned>(sm_count() * per_sm);
@@ -2038,10 +2098,7 @@ extern "C" int vs_dsm_from_points_pipelined(const double *points, const int64_t 
             return VS_ERR_CUDA;
         }
         const size_t key_bytes = sizeof(unsigned long long) * static_cast<size_t>(cells);
-        if (narrow)
-            launch_pipe<5>(flip_row, flip_col, gx, st, points, b, e, counters + v, key_bytes);
-        else
-            launch_pipe<6>(flip_row, flip_col, gx, st, points, b, e, counters + v, key_bytes);
+        launch_pipe(flip_row, flip_col, gx, st, points, b, e, counters + v, key_bytes);
         VS_LAUNCH_CHECK("raster_pipe_kernel");
         if (launch_events && cudaEventRecord(static_cast<cudaEvent_t>(launch_events[2 * v + 1]), st) != cudaSuccess) {
             set_error("vs_dsm_from_points_pipelined: cudaEventRecord failed");
@@ -2523,14 +2580,14 @@ __global__ void __launch_bounds__(256, 3) depth_bin_kernel(const float *__restri
     }
 }
 
-__global__ void __launch_bounds__(TX *TY) depth_epilogue_kernel(const unsigned long long *__restrict__ vk,
+__global__ void __launch_bounds__(TX *TY, 5) depth_epilogue_kernel(const unsigned long long *__restrict__ vk,
                                                                const unsigned long long *__restrict__ first,
                                                                float *__restrict__ out,
                                                                unsigned long long *__restrict__ next_keys, int H,
                                                                int W) {
     chain_wait();
     __shared__ EpilogueSmem sm;
-    epilogue_tile<true>(vk, SignZeroDecoder{first}, out, next_keys, H, W, blockIdx.y * TILE_Y, blockIdx.x * TX, sm);
+    epilogue_tile(vk, SignZeroDecoder{first}, out, next_keys, H, W, blockIdx.y * kTileH, blockIdx.x * kTileW, sm);
 }
 
 }  // namespace
@@ -2575,7 +2632,7 @@ extern "C" int vs_dsm_from_depth_maps(const float *const *depths, const int64_t 
     const GeoFast &gf = geo_plan_fast(plan);
     const GeoFrame *gfr = geo_plan_frame(plan);
     const int south = geo_plan_south(plan);
-    const dim3 egrid(static_cast<unsigned>(ceil_div(xsize, TX)), static_cast<unsigned>(ceil_div(ysize, TILE_Y)));
+    const dim3 egrid(static_cast<unsigned>(ceil_div(xsize, kTileW)), static_cast<unsigned>(ceil_div(ysize, kTileH)));
     int *fl = reinterpret_cast<int *>(flags);
     for (int v = 0; v < n_views; ++v) {
         DepthView dv;
