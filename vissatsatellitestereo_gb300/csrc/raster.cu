@@ -1200,7 +1200,6 @@ struct MapViewDev {
     int ej, ei, nj, ni;
     int W, H;
     int aoi;
-    int vec;                  // rows are 16-byte aligned: float4 loads
     long long off;            // cell offset of the view's DSM in the run's buffer
     float *out;               // the view's DSM, or null: the run's buffer at `off`
     // the axes' differences from the grid origin (in ulps of the origin's binade) are
@@ -1235,6 +1234,17 @@ constexpr int kMapThreads = 256;
 constexpr unsigned kMapKeyZero = 0x80000000u;   // key of +0.0f; any zero while binning
 constexpr int kMapUnitPx = 8;                   // consecutive pixels of a row per thread step
 
+// The per-pixel constants of one work item, kept in shared memory (the loop over the pixels has no
+// registers for them), columns then rows: d = d0 + di * i + dj * j of pixel (i, j); the step of the
+// estimate's product per pixel; the tile's part of the grid, [lo, lo + count) cells; the estimate's parameters.
+struct __align__(16) MapItem {
+    long long d0[2], di[2], dj[2];
+    unsigned long long step[2], wide[2];
+    int lo[2];
+    unsigned count[2], mul[2], fmask[2], fsure[2];
+    int shift[2], fbits[2];
+};
+
 // Shared-memory tile of one work item: an OW x OH block of one view's DSM.  The key tile
 // carries a 2-cell halo (the hole fill of the blur's 1-cell halo needs its neighbours);
 // its keys are 32-bit order keys of the float32 heights (0: no point), enough for the
@@ -1253,8 +1263,9 @@ struct __align__(16) MapTileSmem {
             unsigned short holes[NF];       // empty in-grid cells of the blur input
         } e;
     } u;
+    MapItem it;
     long long item;
-    int view, r0, c0, ia, ib, ja, jb;
+    int view, r0, c0, box[4];               // rows [0], [1], columns [2], [3] of the pixel box
     int n_holes, has_zero;
     unsigned char specrow[FH];              // a NaN or a zero in this row of the blur input
 };
@@ -1270,99 +1281,183 @@ __device__ __forceinline__ bool axis_tile(const FastAxis &a, long long d, int &r
     return ok;
 }
 
-// One pass over the item's pixel box [ia, ib] x [ja, jb] (ja a multiple of 4 for float4
-// rows).  Every pixel is binned exactly as the per-view path bins its FP64 point (the
-// integer/FP32 axis test and the threshold correction); pixels whose cell lies outside
-// the key tile are dropped.  ZERO = false: the nanmax keys, zeros as kMapKeyZero;
-// ZERO = true: for cells whose maximum is a zero, the first zero pixel and its sign.
+// Exact cell index along one axis of a difference inside the grid.
+__device__ __forceinline__ int axis_exact(const FastAxis &a, long long d) {
+    int r;
+    bool sure;
+    axis_tile(a, d, r, sure);
+    return sure ? r : axis_correct(a.thr, min(max(r, 0), a.nm1), d);
+}
+
+// (step * mul) >> shift, 0 < shift < 64: the step of the estimate's product per pixel, where it fits 64 bits.
+__device__ __forceinline__ long long estimate_step(long long step, unsigned mul, int shift) {
+    const long long hi = __mul64hi(step, static_cast<long long>(mul));
+    const unsigned long long lo = static_cast<unsigned long long>(step) * mul;
+    return static_cast<long long>((lo >> shift) | (static_cast<unsigned long long>(hi) << (64 - shift)));
+}
+
+// Bins pixels [k0, k1) of map row i one by one (any map, any place; the exact index of every one
+// inside the grid).  ZERO = false: the nanmax keys, zeros as kMapKeyZero; true returned: one
+// was a zero.  ZERO = true: for cells whose maximum is a zero, the first zero pixel and its sign.
 template <int OW, int OH, bool ZERO>
-__device__ __forceinline__ void map_tile_pass(const MapViewDev &mv, const FastAxis &R, const FastAxis &C, int rbase,
-                                              int cbase, int ia, int ib, int ja, int jb, MapTileSmem<OW, OH> &sm) {
+__device__ __noinline__ bool map_pixels(const MapViewDev &mv, const AoiDev &ad, int rbase, int cbase, int i, int k0, int k1,
+                                        MapTileSmem<OW, OH> &sm) {
+    using S = MapTileSmem<OW, OH>;
+    const FastAxis &R = ad.row, &C = ad.col;
+    const int di2 = 2 * i + 1 - mv.H, dj0 = 2 * k0 + 1 - mv.W;
+    long long dcol = mv.dc0 + mv.dc_di * di2 + mv.dc_dj * dj0;
+    long long drow = mv.dr0 + mv.dr_di * di2 + mv.dr_dj * dj0;
+    const float *src = mv.map + static_cast<long long>(i) * mv.stride;
+    bool zero_seen = false;
+#pragma unroll 1
+    for (int j = k0; j < k1; ++j, dcol += 2 * mv.dc_dj, drow += 2 * mv.dr_dj) {
+        const unsigned hb = __float_as_uint(__ldg(src + j)), mag = hb & 0x7fffffffu;
+        if (!(ZERO ? mag == 0u : mag <= 0x7f800000u)) continue;           // not NaN
+        if (static_cast<unsigned long long>(dcol) >= static_cast<unsigned long long>(C.tmax) ||
+            static_cast<unsigned long long>(drow) >= static_cast<unsigned long long>(R.tmax))
+            continue;
+        const unsigned lc = static_cast<unsigned>(axis_exact(C, dcol) - cbase),
+                       lr = static_cast<unsigned>(axis_exact(R, drow) - rbase);
+        if (lr >= static_cast<unsigned>(S::KH) || lc >= static_cast<unsigned>(S::KW)) continue;
+        const int cell = static_cast<int>(lr) * S::KW + static_cast<int>(lc);
+        if (ZERO) {
+            const unsigned idx = static_cast<unsigned>(i) * static_cast<unsigned>(mv.W) + static_cast<unsigned>(j);
+            if (sm.keys[cell] == kMapKeyZero)
+                atomicMax(&sm.u.zw[cell], ((static_cast<unsigned>(kMapIdxLimit) - 1u - idx) << 1) | (hb >> 31));
+        } else {
+            zero_seen |= mag == 0u;
+            atomicMax(&sm.keys[cell], mag == 0u ? kMapKeyZero : hb ^ (static_cast<unsigned>(static_cast<int>(hb) >> 31) | 0x80000000u));
+        }
+    }
+    return zero_seen;
+}
+
+// One axis of an item's constants: cells [base, base + cells) of the key tile, n in the grid.
+__device__ __forceinline__ void set_item_axis(MapItem &it, int k, const FastAxis &a, long long d0, long long di, long long dj,
+                                              int W, int H, int base, int cells) {
+    it.d0[k] = d0 + di * (1 - H) + dj * (1 - W);
+    it.di[k] = 2 * di;
+    it.dj[k] = 2 * dj;
+    it.shift[k] = a.shift + 2;
+    it.step[k] = static_cast<unsigned long long>(estimate_step(2 * dj, a.mul, a.shift + 2));
+    it.wide[k] = 1ull << (a.shift + 33);
+    it.lo[k] = max(base, 0);
+    it.count[k] = static_cast<unsigned>(max(min(base + cells, a.nm1 + 1) - it.lo[k], 0));
+    it.mul[k] = a.mul;
+    it.fbits[k] = a.fbits - 2;
+    it.fmask[k] = a.fmask >> 2;
+    it.fsure[k] = max(a.fmask >> 2, 7u) - 7u;
+}
+
+// One pass over the item's pixel box [ia, ib] x [ja, jb].  Every pixel is binned exactly as the
+// per-view path bins its FP64 point (the integer/FP32 axis test and the threshold correction);
+// pixels whose cell lies outside the key tile are dropped.
+//
+// Issue-bound, with two pixels per cell the larger part of the kernel.  The differences of a unit's
+// pixels are affine in the pixel, so axis_estimate's product advances by a constant: the first
+// product and k steps are below the product of the exact difference by no more than the floors of the
+// shifted difference and of the steps (together under 1 + 8 * 2^-32 units of the high word), as axis_estimate's
+// own is, so the same four units of margin prove the index.  With two bits fewer the product is signed and
+// holds differences of up to twice the estimate's range on either side of the origin: units that cross rows,
+// or the grid's border, as those of a third of the tiles do, are no case of their own, and the cell index
+// alone tells whether a pixel is inside.  Two 32-bit additions, a shift and a test per axis and pixel;
+// unproven pixels (8 units in 2^(fbits - 2)) take the exact index, units further away map_pixels.  A row's
+// units start on 16-byte boundaries, whatever its own alignment.  107 M cells, 226 M pixels: the
+// kernel 1.19 ms with 64-bit tests, a case per row change and one for each border unit, 0.98 ms so.
+template <int OW, int OH>
+__device__ __forceinline__ void map_tile_pass(const MapViewDev &mv, const AoiDev &ad, int rbase, int cbase, int ia, int ib,
+                                              int ja, int jb, MapTileSmem<OW, OH> &sm) {
     using S = MapTileSmem<OW, OH>;
     constexpr int P = kMapUnitPx;
-    const int G = (jb - ja) / P + 1;                    // P-pixel groups per box row
+    const MapItem &it = sm.it;
+    const int W = mv.W;
+    const long long stride = mv.stride;
+    const float *const map = mv.map;
+    const int G = (jb - ja + 3) / P + 1;                // P-pixel groups per box row
     const int units = (ib - ia + 1) * G;
     int row = threadIdx.x / G, g = threadIdx.x - row * G;
     const int rstep = kMapThreads / G, gstep = kMapThreads - rstep * G;
-    const long long scol = 2 * mv.dc_dj, srow = 2 * mv.dr_dj;   // per pixel along a row
     bool zero_seen = false;
     for (int unit = threadIdx.x; unit < units; unit += kMapThreads) {
-        const int i = ia + row, j0 = ja + g * P;
-        const float *src = mv.map + static_cast<long long>(i) * mv.stride + j0;
-        unsigned hb[P];
-        if (mv.vec && j0 + P <= mv.W) {
-#pragma unroll
-            for (int q = 0; q < P / 4; ++q) {
-                const float4 v4 = __ldg(reinterpret_cast<const float4 *>(src) + q);
-                hb[4 * q] = __float_as_uint(v4.x); hb[4 * q + 1] = __float_as_uint(v4.y);
-                hb[4 * q + 2] = __float_as_uint(v4.z); hb[4 * q + 3] = __float_as_uint(v4.w);
-            }
-        } else {
-#pragma unroll
-            for (int k = 0; k < P; ++k) hb[k] = j0 + k < mv.W ? __float_as_uint(__ldg(src + k)) : 0x7fc00000u;
-        }
-        const int di2 = 2 * i + 1 - mv.H, dj0 = 2 * j0 + 1 - mv.W;
-        long long dcol = mv.dc0 + mv.dc_di * di2 + mv.dc_dj * dj0;
-        long long drow = mv.dr0 + mv.dr_di * di2 + mv.dr_dj * dj0;
-        // rows: d is affine along the unit, and the exact row monotone in d, so when the
-        // first and the last pixel fall in the same row with sure estimates, all do
-        int ra, rb;
-        bool sa, sb;
-        const bool oka = axis_tile(R, drow, ra, sa), okb = axis_tile(R, drow + (P - 1) * srow, rb, sb);
-        const bool row_fixed = oka & okb & sa & sb & (ra == rb);
-        const unsigned lr_fixed = static_cast<unsigned>(ra - rbase);
-        int cell[P];
-        unsigned key[P];
-#pragma unroll
-        for (int k = 0; k < P; ++k, dcol += scol, drow += srow) {
-            const unsigned mag = hb[k] & 0x7fffffffu;
-            int c;
-            bool sc;
-            bool ok = ZERO ? mag == 0u : mag <= 0x7f800000u;    // not NaN
-            unsigned lr = lr_fixed;
-            if (!row_fixed) {
-                int r;
-                bool sr;
-                ok &= axis_tile(R, drow, r, sr);
-                if (ok && !sr) r = axis_correct(R.thr, min(max(r, 0), R.nm1), drow);
-                lr = static_cast<unsigned>(r - rbase);
-            }
-            ok &= axis_tile(C, dcol, c, sc);
-            if (ok && !sc) c = axis_correct(C.thr, min(max(c, 0), C.nm1), dcol);
-            const unsigned lc = static_cast<unsigned>(c - cbase);
-            ok &= (lr < static_cast<unsigned>(S::KH)) & (lc < static_cast<unsigned>(S::KW));
-            cell[k] = ok ? static_cast<int>(lr) * S::KW + static_cast<int>(lc) : -1;
-            if (ZERO) {
-                const unsigned idx = static_cast<unsigned>(i) * static_cast<unsigned>(mv.W) + static_cast<unsigned>(j0 + k);
-                key[k] = ((static_cast<unsigned>(kMapIdxLimit) - 1u - idx) << 1) | (hb[k] >> 31);
-            } else {
-                zero_seen |= ok & (mag == 0u);
-                key[k] = mag == 0u ? kMapKeyZero : ((hb[k] >> 31) ? ~hb[k] : (hb[k] | 0x80000000u));
-            }
-        }
-        if (ZERO) {
-#pragma unroll
-            for (int k = 0; k < P; ++k)
-                if (cell[k] >= 0 && sm.keys[cell[k]] == kMapKeyZero) atomicMax(&sm.u.zw[cell[k]], key[k]);
-        } else {
-#pragma unroll
-            for (int k = 1; k < P; ++k) {     // merge runs of consecutive pixels in one cell
-                const bool same = (cell[k] >= 0) & (cell[k] == cell[k - 1]);
-                key[k] = same ? max(key[k], key[k - 1]) : key[k];
-                cell[k - 1] = same ? -1 : cell[k - 1];
-            }
-#pragma unroll
-            for (int k = 0; k < P; ++k)
-                if (cell[k] >= 0) atomicMax(&sm.keys[cell[k]], key[k]);
-        }
+        const int i = ia + row;
+        const float *const line = map + i * stride;
+        const int j0 = ja + g * P - static_cast<int>((reinterpret_cast<unsigned long long>(line + ja) >> 2) & 3);
         g += gstep;
         row += rstep;
         if (g >= G) {
             g -= G;
             ++row;
         }
+        const long long dc = it.d0[0] + it.di[0] * i + it.dj[0] * j0, dr = it.d0[1] + it.di[1] * i + it.dj[1] * j0;
+        {
+            const unsigned long long wc = it.wide[0], wr = it.wide[1];
+            const bool near = (dc + wc < 2 * wc) & (dr + wr < 2 * wr) & (dc + (P - 1) * it.dj[0] + wc < 2 * wc) &
+                              (dr + (P - 1) * it.dj[1] + wr < 2 * wr);
+            if (!near) {
+                zero_seen |= map_pixels<OW, OH, false>(mv, ad, rbase, cbase, i, max(j0, 0), min(j0 + P, W), sm);
+                continue;
+            }
+        }
+        float h[P];
+        if (j0 >= 0 && j0 + P <= W) {
+#pragma unroll
+            for (int q = 0; q < P / 4; ++q) {
+                const float4 v4 = __ldg(reinterpret_cast<const float4 *>(line + j0) + q);
+                h[4 * q] = v4.x; h[4 * q + 1] = v4.y; h[4 * q + 2] = v4.z; h[4 * q + 3] = v4.w;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < P; ++k)
+                h[k] = static_cast<unsigned>(j0 + k) < static_cast<unsigned>(W) ? __ldg(line + j0 + k) : __uint_as_float(0x7fffffffu);
+        }
+        // four units below the estimate: an index is proven by its fraction alone
+        unsigned long long ac = static_cast<unsigned long long>(static_cast<long long>(static_cast<int>(dc >> it.shift[0])) * it.mul[0]) - (4ull << 32);
+        unsigned long long ar = static_cast<unsigned long long>(static_cast<long long>(static_cast<int>(dr >> it.shift[1])) * it.mul[1]) - (4ull << 32);
+        const unsigned long long sc = it.step[0], sr = it.step[1];
+        const unsigned fmc = it.fmask[0], fsc = it.fsure[0], fmr = it.fmask[1], fsr = it.fsure[1];
+        const unsigned nc = it.count[0], nr = it.count[1];
+        const int fbc = it.fbits[0], fbr = it.fbits[1], lo_c = it.lo[0], lo_r = it.lo[1];
+        const int first = (lo_r - rbase) * S::KW + (lo_c - cbase);
+        int cell[P];
+        bool unsure = false;
+#pragma unroll
+        for (int k = 0; k < P; ++k, ac += sc, ar += sr) {
+            const int hc = static_cast<int>(ac >> 32), hr = static_cast<int>(ar >> 32);
+            unsure |= ((hc & fmc) >= fsc) | ((hr & fmr) >= fsr);
+            const int lc = (hc >> fbc) - lo_c, lr = (hr >> fbr) - lo_r;
+            const bool ok = !isnan(h[k]) & (static_cast<unsigned>(lr) < nr) & (static_cast<unsigned>(lc) < nc);
+            cell[k] = ok ? lr * S::KW + lc + first : -1;
+        }
+        if (unsure) {
+#pragma unroll
+            for (int k = 0; k < P; ++k) {
+                const long long ec = dc + k * it.dj[0], er = dr + k * it.dj[1];
+                cell[k] = -1;
+                if (isnan(h[k]) || static_cast<unsigned long long>(ec) >= static_cast<unsigned long long>(ad.col.tmax) ||
+                    static_cast<unsigned long long>(er) >= static_cast<unsigned long long>(ad.row.tmax))
+                    continue;
+                const int lc = axis_exact(ad.col, ec) - lo_c, lr = axis_exact(ad.row, er) - lo_r;
+                if (static_cast<unsigned>(lr) < nr && static_cast<unsigned>(lc) < nc) cell[k] = lr * S::KW + lc + first;
+            }
+        }
+        unsigned key[P];
+#pragma unroll
+        for (int k = 0; k < P; ++k) {
+            const unsigned hb = __float_as_uint(__fadd_rn(h[k], 0.0f));      // a zero: +0
+            zero_seen |= (cell[k] >= 0) & (hb == 0u);
+            key[k] = hb ^ (static_cast<unsigned>(static_cast<int>(hb) >> 31) | 0x80000000u);
+        }
+#pragma unroll
+        for (int k = 1; k < P; ++k) {     // merge runs of consecutive pixels in one cell
+            const bool same = (cell[k] >= 0) & (cell[k] == cell[k - 1]);
+            key[k] = same ? max(key[k], key[k - 1]) : key[k];
+            cell[k - 1] = same ? -1 : cell[k - 1];
+        }
+#pragma unroll
+        for (int k = 0; k < P; ++k)
+            if (cell[k] >= 0) atomicMax(&sm.keys[cell[k]], key[k]);
     }
-    if (!ZERO && zero_seen) sm.has_zero = 1;
+    if (zero_seen) sm.has_zero = 1;
 }
 
 // cswap on 32-bit keys.
@@ -1403,6 +1498,11 @@ __device__ __forceinline__ float median8_keys32(unsigned (&s)[8]) {
     cswap32(s[1], s[2]); cswap32(s[3], s[4]); cswap32(s[5], s[6]);
     const unsigned lo = select8_32(s, (n - 1) >> 1), hi = select8_32(s, n >> 1);
     if (n & 1) return float_from_key(hi == 0x7fffffffu ? kMapKeyZero : hi);   // -0 + 0 = +0
+    // FP64's sum of two floats is exact when their exponents differ by at most 28, and its half is then
+    // rounded once: the FP32 sum's half, away from overflow and subnormals
+    const float a = float_from_key(lo), b = float_from_key(hi);
+    const unsigned ea = (__float_as_uint(a) >> 23) & 0xffu, eb = (__float_as_uint(b) >> 23) & 0xffu;
+    if (ea - 64u < 128u && eb - 64u < 128u && ea - eb + 28u <= 56u) return __fmul_rn(__fadd_rn(a, b), 0.5f);
     return f64_to_f32(median_from_middle(key64_of_key32(lo), key64_of_key32(hi), n));
 }
 
@@ -1417,7 +1517,8 @@ __device__ __forceinline__ float median8_keys32(unsigned (&s)[8]) {
 // output.  A warp now walks rows with OW / 32 columns per lane -- staging them with the indices of a
 // row, blurring eight consecutive rows that each load one new row -- and the image's border is
 // copied around the tile once, in the tiles that have one: 416 -> 305 instructions per cell, 107 M cells and
-// 226 M pixels 1.53 -> 1.19 ms.
+// 226 M pixels 1.53 -> 1.19 ms.  (The mean of a hole's two middle neighbours in FP32, where that is exact, and
+// map_tile_pass's product brought it to 0.98 ms; asking for the next item ahead, its box by lanes, to 0.93 ms.)
 template <int OW, int OH>
 __device__ __forceinline__ void map_tile_finish(MapTileSmem<OW, OH> &sm, float *__restrict__ out, int H, int W,
                                                 int r0, int c0) {
@@ -1589,31 +1690,21 @@ __device__ __forceinline__ void map_tile_finish(MapTileSmem<OW, OH> &sm, float *
 // Pixel box [ia, ib] x [ja, jb] of the pixels whose cells can fall in rows [rlo, rhi) and
 // columns [clo, chi) of the grid: the affine pixel <- cell map at the region's corners,
 // widened by a quarter cell and by bmarg pixels (one pixel plus a bound of the FP64
-// rounding of the map), clipped to the map.  ja is rounded down to a multiple of 4 for float4 rows.
-__device__ __forceinline__ void map_pixel_box(const MapViewDev &mv, int rlo, int rhi, int clo, int chi, int &ia, int &ib,
-                                              int &ja, int &jb) {
-    if (mv.box_all) {
-        ia = 0; ib = mv.H - 1; ja = 0; jb = mv.W - 1;
-    } else {
-        const double sr[2] = {rlo - 0.25, rhi + 0.25}, sc[2] = {clo - 0.25, chi + 0.25};
-        double imin = 1e300, imax = -1e300, jmin = 1e300, jmax = -1e300;
-#pragma unroll
-        for (int a = 0; a < 2; ++a)
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                const double pi = __fma_rn(mv.bir, sr[a], __fma_rn(mv.bic, sc[b], mv.bi0));
-                const double pj = __fma_rn(mv.bjr, sr[a], __fma_rn(mv.bjc, sc[b], mv.bj0));
-                imin = fmin(imin, pi); imax = fmax(imax, pi);
-                jmin = fmin(jmin, pj); jmax = fmax(jmax, pj);
-            }
-        // clamp before converting (a far-away tile maps far outside the map)
-        ia = static_cast<int>(fmin(fmax(floor(imin - mv.bmarg), 0.0), mv.H));
-        ib = static_cast<int>(fmax(fmin(ceil(imax + mv.bmarg), mv.H - 1.0), -1.0));
-        ja = static_cast<int>(fmin(fmax(floor(jmin - mv.bmarg), 0.0), mv.W));
-        jb = static_cast<int>(fmax(fmin(ceil(jmax + mv.bmarg), mv.W - 1.0), -1.0));
-        if (!(imin <= imax && jmin <= jmax)) { ia = 1; ib = 0; }    // NaN: nothing
-    }
-    if (mv.vec) ja &= ~3;      // float4 rows: groups start 16-byte aligned
+// rounding of the map), clipped to the map.  Lane q < 4 of a warp returns ia, ib, ja, jb: an extreme of the
+// map lies at the corner that its coefficients' signs choose, so a lane evaluates one corner in
+// 8 FP64 operations of 59 cycles, where one thread took about 40 while the block waited.
+__device__ __forceinline__ int map_pixel_box(const MapViewDev &mv, int rlo, int rhi, int clo, int chi, int q) {
+    const bool top = q & 1, cols = q & 2;
+    const int last = (cols ? mv.W : mv.H) - 1;
+    if (mv.box_all) return top ? last : 0;
+    const double cr = cols ? mv.bjr : mv.bir, cc = cols ? mv.bjc : mv.bic, c0 = cols ? mv.bj0 : mv.bi0;
+    const bool up_r = (__double2hiint(cr) >= 0) == top, up_c = (__double2hiint(cc) >= 0) == top;
+    const double r = __int2double_rn(up_r ? rhi : rlo), c = __int2double_rn(up_c ? chi : clo);
+    const double quarter_r = up_r ? 0.25 : -0.25, quarter_c = up_c ? 0.25 : -0.25;
+    const double p = __fma_rn(cr, __dadd_rn(r, quarter_r), __fma_rn(cc, __dadd_rn(c, quarter_c), c0));
+    // the upper end as the negated floor of the negated value; the conversion saturates
+    const int t = __double2int_rd(__dadd_rn(top ? -p : p, -mv.bmarg));
+    return top ? min(max(t, -last), 1) * -1 : min(max(t, 0), last + 1);
 }
 
 // The batched rasterisation of many views, one fused kernel: a CTA takes work items (one
@@ -1629,13 +1720,18 @@ __global__ void __launch_bounds__(kMapThreads, 4) map_tile_kernel(
     using S = MapTileSmem<OW, OH>;
     __shared__ S sm;
     for (int i = threadIdx.x; i < S::NK; i += kMapThreads) sm.keys[i] = 0u;
-    int vlast = v_lo;      // thread 0: the view of this CTA's previous item (items only grow)
+    int vlast = v_lo;      // first warp: the view of this CTA's previous item (items only grow)
+    unsigned long long next = 0;      // thread 0: the next item, requested before the epilogue of the one at hand
+    if (threadIdx.x == 0) next = atomicAdd(counter, 1ull);
     for (;;) {
-        if (threadIdx.x == 0) {
-            const long long it = item_begin + static_cast<long long>(atomicAdd(counter, 1ull));
-            sm.item = it;
-            sm.n_holes = 0;
-            sm.has_zero = 0;
+        if (threadIdx.x < 32) {
+            const int lane = threadIdx.x;
+            const long long it = item_begin + static_cast<long long>(__shfl_sync(0xffffffffu, next, 0));
+            if (lane == 0) {
+                sm.item = it;
+                sm.n_holes = 0;
+                sm.has_zero = 0;
+            }
             if (it < item_end) {
                 int v = vlast;
                 for (int step = 0; step < 8 && v < v_hi && __ldg(tile_start + v + 1) <= it; ++step) ++v;
@@ -1647,31 +1743,39 @@ __global__ void __launch_bounds__(kMapThreads, 4) map_tile_kernel(
                 const int local = static_cast<int>(it - __ldg(tile_start + v));
                 const int ty = local / tiles_x, tx = local - ty * tiles_x;
                 const int r0 = ty * OH, c0 = tx * OW;
-                int ia, ib, ja, jb;
-                map_pixel_box(mv, max(r0 - 2, 0), min(r0 + OH + 2, ad.ysize), max(c0 - 2, 0),
-                              min(c0 + OW + 2, ad.xsize), ia, ib, ja, jb);
-                sm.view = v; sm.r0 = r0; sm.c0 = c0;
-                sm.ia = ia; sm.ib = ib; sm.ja = ja; sm.jb = jb;
+                const int end = map_pixel_box(mv, max(r0 - 2, 0), min(r0 + OH + 2, ad.ysize), max(c0 - 2, 0),
+                                              min(c0 + OW + 2, ad.xsize), lane);
+                if (lane < 4) sm.box[lane] = end;
+                if (lane == 0) {
+                    sm.view = v; sm.r0 = r0; sm.c0 = c0;
+                    set_item_axis(sm.it, 0, ad.col, mv.dc0, mv.dc_di, mv.dc_dj, mv.W, mv.H, c0 - 2, S::KW);
+                } else if (lane == 1) {
+                    set_item_axis(sm.it, 1, ad.row, mv.dr0, mv.dr_di, mv.dr_dj, mv.W, mv.H, r0 - 2, S::KH);
+                }
             }
         }
         __syncthreads();
         if (sm.item >= item_end) return;
-        const int v = sm.view, r0 = sm.r0, c0 = sm.c0, ia = sm.ia, ib = sm.ib, ja = sm.ja, jb = sm.jb;
+        const int v = sm.view, r0 = sm.r0, c0 = sm.c0, ia = sm.box[0], ib = sm.box[1], ja = sm.box[2], jb = sm.box[3];
         for (int i = threadIdx.x; i < S::FH; i += kMapThreads) sm.specrow[i] = 0;
         const MapViewDev &mv = views[v];
         const AoiDev &ad = aois[mv.aoi];
-        const FastAxis R = ad.row, C = ad.col;
-        if (ia <= ib && ja <= jb) map_tile_pass<OW, OH, false>(mv, R, C, r0 - 2, c0 - 2, ia, ib, ja, jb, sm);
+        if (ia <= ib && ja <= jb) map_tile_pass<OW, OH>(mv, ad, r0 - 2, c0 - 2, ia, ib, ja, jb, sm);
         __syncthreads();
         if (sm.has_zero) {       // rare: resolve the sign of cells whose maximum is a zero
             for (int i = threadIdx.x; i < S::NK; i += kMapThreads) sm.u.zw[i] = 0u;
             __syncthreads();
-            map_tile_pass<OW, OH, true>(mv, R, C, r0 - 2, c0 - 2, ia, ib, ja, jb, sm);
+            const int groups = (jb - ja) / kMapUnitPx + 1;
+            for (int u = threadIdx.x; u < (ib - ia + 1) * groups; u += kMapThreads) {
+                const int j = ja + u % groups * kMapUnitPx;
+                map_pixels<OW, OH, true>(mv, ad, r0 - 2, c0 - 2, ia + u / groups, j, min(j + kMapUnitPx, mv.W), sm);
+            }
             __syncthreads();
             for (int i = threadIdx.x; i < S::NK; i += kMapThreads)
                 if (sm.keys[i] == kMapKeyZero) sm.keys[i] = (sm.u.zw[i] & 1u) ? 0x7fffffffu : kMapKeyZero;
             __syncthreads();
         }
+        if (threadIdx.x == 0) next = atomicAdd(counter, 1ull);
         map_tile_finish<OW, OH>(sm, mv.out ? mv.out : dsm + mv.off, ad.ysize, ad.xsize, r0, c0);
     }
 }
@@ -2298,7 +2402,6 @@ extern "C" int vs_aoi_batch_plan(const VsAoi *aois, int n_aois, const VsMapView 
         d.W = V.width;
         d.H = V.height;
         d.aoi = V.aoi;
-        d.vec = ((reinterpret_cast<uintptr_t>(V.heights) & 15) == 0) && (V.row_stride % 4 == 0);
         d.off = p->view_off[v];
         d.out = V.dsm;
         // d = bits(x) - bits(xoff) = (bx - bits(xoff)) + (x_fx << shx), x_fx affine in the
