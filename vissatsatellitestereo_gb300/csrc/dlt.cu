@@ -296,8 +296,9 @@ __device__ __forceinline__ void prefetch_l2(const void *p, long long bytes) {
 // Latency-bound: 40 bytes and 200 instructions per point, and 80 accumulators and inputs per thread
 // leave 20 warps per SM.  So one thread sends the block's 80 KB on its way to L2 at the start, and
 // each thread loads its next two points before it adds the current two.  50 x 800,000 points (1.6 GB,
-// 240 us of HBM time): 400 us with the loads at the head of each group, 354 us with the prefetch,
-// 324 us with both; one point ahead and six blocks per SM 330 us.
+// 240 us of HBM time): 400 us with the loads at the head of each group, 336 us so.  (Of the whole fit's
+// 1996 us the prefetch alone takes off 46, two points ahead alone 43, both 67; one point ahead at six
+// blocks per SM, with the prefetch, 61.)
 __global__ void __launch_bounds__(kMomThreads, 5) moments_kernel(
     const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ z, long long xyz_stride,
     const double *__restrict__ col, const double *__restrict__ row, const float4 *__restrict__ colrow,
