@@ -456,6 +456,14 @@ __device__ __forceinline__ double median8_keys(unsigned long long (&s)[8]) {
     return median_from_middle(select8(s, (n - 1) >> 1), select8(s, n >> 1), n);
 }
 
+// A launch over rows of tiles: gridDim.y holds 65,535 of them, the rest go to gridDim.z.
+dim3 tile_grid(long long tiles_x, long long tiles_y) {
+    const long long rows = std::min<long long>(tiles_y, 65535);
+    return dim3(static_cast<unsigned>(tiles_x), static_cast<unsigned>(rows), static_cast<unsigned>(ceil_div(tiles_y, rows)));
+}
+// The tile row of a block; past the last one in the last layer of gridDim.z.
+__device__ __forceinline__ int tile_row() { return static_cast<int>(blockIdx.z * gridDim.y + blockIdx.y); }
+
 // The FP64 grid from the keys: nanmax values and the non-propagating hole fill
 // (lib/proj_to_grid.py:64-79) in one pass over 32 x 32 tiles.  The keys and a 1-cell halo are
 // loaded at once (six loads in flight per thread, one trip to L2) and staged; empty cells go
@@ -472,7 +480,8 @@ __global__ void __launch_bounds__(kGridThreads) grid_f64_kernel(const unsigned l
     __shared__ int n_holes;
     chain_wait();
     constexpr int kLoads = (kGridRaw * kGridRaw + kGridThreads - 1) / kGridThreads;
-    const int tid = threadIdx.x, r0 = blockIdx.y * kGridTile, c0 = blockIdx.x * kGridTile;
+    if (tile_row() > (H - 1) / kGridTile) return;
+    const int tid = threadIdx.x, r0 = tile_row() * kGridTile, c0 = blockIdx.x * kGridTile;
     if (tid == 0) n_holes = 0;
     unsigned long long k[kLoads];
 #pragma unroll
@@ -1825,9 +1834,9 @@ extern "C" int vs_proj_to_grid(const double *points, int64_t n, double xoff, dou
     if (s == VS_OK) s = make_tables(xoff, yoff, xresolution, yresolution, xsize, ysize, w, tb, st);
     if (s == VS_OK) s = bin_launch(points, nullptr, 0, n, n, tb, w.keys[0], w.first, st);
     if (s != VS_OK) return s;
-    const dim3 grid(static_cast<unsigned>(ceil_div(xsize, kGridTile)), static_cast<unsigned>(ceil_div(ysize, kGridTile)));
+    const dim3 grid = tile_grid(ceil_div(xsize, kGridTile), ceil_div(ysize, kGridTile));
     launch_chained(grid_f64_kernel, grid, kGridThreads, 0, st, w.keys[0], w.first, points, dsm, static_cast<int>(ysize),
-                                                   static_cast<int>(xsize));
+                   static_cast<int>(xsize));
     VS_LAUNCH_CHECK("grid_f64_kernel");
     return VS_OK;
 }
