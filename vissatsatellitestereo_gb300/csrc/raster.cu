@@ -897,7 +897,8 @@ __global__ void __launch_bounds__(TX *TY, 5) dsm_epilogue_kernel(
     int W) {
     chain_wait();
     __shared__ EpilogueSmem sm;
-    epilogue_tile(vk, PointsZeroDecoder{first, pts}, out, next_keys, H, W, blockIdx.y * kTileH, blockIdx.x * kTileW, sm);
+    if (tile_row() > (H - 1) / kTileH) return;
+    epilogue_tile(vk, PointsZeroDecoder{first, pts}, out, next_keys, H, W, tile_row() * kTileH, blockIdx.x * kTileW, sm);
 }
 
 // ---- pipelined rasterisation: view v's binning and view v-1's epilogue in one launch -----
@@ -1867,7 +1868,7 @@ extern "C" int vs_dsm_from_points(const double *points, const int64_t *offsets, 
     if (s != VS_OK) return s;
     // per-view counts live on the device: launch for a full GPU and let the grid stride
     const long long launch_points = static_cast<long long>(sm_count()) * 8 * 256 * kPts;
-    const dim3 egrid(static_cast<unsigned>(ceil_div(xsize, kTileW)), static_cast<unsigned>(ceil_div(ysize, kTileH)));
+    const dim3 egrid = tile_grid(ceil_div(xsize, kTileW), ceil_div(ysize, kTileH));
     for (int v = 0; v < n_views; ++v) {
         unsigned long long *cur = w.keys[v & 1], *nxt = (v + 1 < n_views) ? w.keys[(v + 1) & 1] : nullptr;
         s = bin_launch(points, reinterpret_cast<const long long *>(offsets), v, 0, launch_points, tb, cur, w.first, st);
@@ -1998,7 +1999,7 @@ extern "C" int vs_dsm_from_points_host(const double *host_points, const int64_t 
         set_error("vs_dsm_from_points_host: cudaEventCreate failed");
         return VS_ERR_CUDA;
     }
-    const dim3 egrid(static_cast<unsigned>(ceil_div(xsize, kTileW)), static_cast<unsigned>(ceil_div(ysize, kTileH)));
+    const dim3 egrid = tile_grid(ceil_div(xsize, kTileW), ceil_div(ysize, kTileH));
     // the copy stream starts after the work already queued on `stream` (tables, clears)
     if (cudaEventRecord(freed[0], st) != cudaSuccess || cudaStreamWaitEvent(cs, freed[0], 0) != cudaSuccess)
         s = VS_ERR_CUDA;
@@ -2068,7 +2069,7 @@ extern "C" int vs_dsm_from_points_overlap(const double *points, const int64_t *o
     if (s == VS_OK) s = clear(w.keys[0], w.cleared, st);
     if (s != VS_OK) return s;
     const long long launch_points = static_cast<long long>(sm_count()) * 8 * 256 * kPts;
-    const dim3 egrid(static_cast<unsigned>(ceil_div(xsize, kTileW)), static_cast<unsigned>(ceil_div(ysize, kTileH)));
+    const dim3 egrid = tile_grid(ceil_div(xsize, kTileW), ceil_div(ysize, kTileH));
     auto cuda_ok = [](cudaError_t e) {
         if (e == cudaSuccess) return true;
         set_error("stream ordering failed: %s", cudaGetErrorString(e));
@@ -2156,7 +2157,7 @@ extern "C" int vs_dsm_from_points_pipelined(const double *points, const int64_t 
         // points outside the fast path's precondition: the literal FP64 binning, then the
         // epilogue, view by view (same results)
         const long long launch_points = static_cast<long long>(sm_count()) * 8 * 256 * kPts;
-        const dim3 egrid(static_cast<unsigned>(tiles_x), static_cast<unsigned>(ceil_div(ysize, kTileH)));
+        const dim3 egrid = tile_grid(tiles_x, ceil_div(ysize, kTileH));
         for (int v = 0; v < n_views; ++v) {
             s = bin_launch(points, reinterpret_cast<const long long *>(offsets), v, 0, launch_points, tb, w.keys[v % 3],
                            w.first[v & 1], st);
@@ -2699,7 +2700,8 @@ __global__ void __launch_bounds__(TX *TY, 5) depth_epilogue_kernel(const unsigne
                                                                int W) {
     chain_wait();
     __shared__ EpilogueSmem sm;
-    epilogue_tile(vk, SignZeroDecoder{first}, out, next_keys, H, W, blockIdx.y * kTileH, blockIdx.x * kTileW, sm);
+    if (tile_row() > (H - 1) / kTileH) return;
+    epilogue_tile(vk, SignZeroDecoder{first}, out, next_keys, H, W, tile_row() * kTileH, blockIdx.x * kTileW, sm);
 }
 
 }  // namespace
@@ -2744,7 +2746,7 @@ extern "C" int vs_dsm_from_depth_maps(const float *const *depths, const int64_t 
     const GeoFast &gf = geo_plan_fast(plan);
     const GeoFrame *gfr = geo_plan_frame(plan);
     const int south = geo_plan_south(plan);
-    const dim3 egrid(static_cast<unsigned>(ceil_div(xsize, kTileW)), static_cast<unsigned>(ceil_div(ysize, kTileH)));
+    const dim3 egrid = tile_grid(ceil_div(xsize, kTileW), ceil_div(ysize, kTileH));
     int *fl = reinterpret_cast<int *>(flags);
     for (int v = 0; v < n_views; ++v) {
         DepthView dv;
