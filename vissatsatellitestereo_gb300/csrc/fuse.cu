@@ -472,18 +472,20 @@ __global__ void __launch_bounds__(kTileCells, 3) fuse_wide_kernel(const float *_
     }
 }
 
+// Lets a kernel take `bytes` of dynamic shared memory on the current device.  Asked for by every launch:
+// the grant is the device's, so a flag kept per process left the second device without it.  The same
+// value for every caller of a kernel, so that threads do not undo one another's.
+template <typename Kernel>
+bool allow_smem(Kernel kernel, size_t bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)) == cudaSuccess;
+}
+
 size_t fuse_tile_smem(int V, int N) { return sizeof(float) * static_cast<size_t>(V + N) * kTileCells; }
 
 template <int N>
 bool launch_fuse_v64(const float *dsm, int layout, int V, long long cells, float *out, bool aligned, cudaStream_t st) {
     const size_t sh = fuse_tile_smem(V, N);
-    static bool configured = false;     // per instantiation: room for the largest tile (V = N)
-    if (!configured) {
-        if (cudaFuncSetAttribute(fuse_tile_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(fuse_tile_smem(N, N))) != cudaSuccess)
-            return false;
-        configured = true;
-    }
+    if (!allow_smem(fuse_tile_kernel<N>, fuse_tile_smem(N, N))) return false;     // the largest tile: V = N
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fuse_tile_kernel<N>, kTileCells, sh) != cudaSuccess ||
         per_sm <= 0)
@@ -500,14 +502,8 @@ bool launch_fuse_wide_n(const float *dsm, int layout, int V, long long cells, fl
     using T = WideTile<L>;
     const size_t base = (static_cast<size_t>(T::kSorted) + 3) & ~size_t(3);
     const size_t sh = sizeof(float) * (base + T::floats(layout, V));
-    static bool configured = false;     // per instantiation: room for the largest tile (V = 64 L)
-    if (!configured) {
-        const size_t most = sizeof(float) * (base + std::max<size_t>(64 * L * T::TS, T::CS * (64 * L + 32)));
-        if (cudaFuncSetAttribute(fuse_wide_kernel<N, L>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(most)) != cudaSuccess)
-            return false;
-        configured = true;
-    }
+    const size_t most = sizeof(float) * (base + std::max<size_t>(64 * L * T::TS, T::CS * (64 * L + 32)));    // V = 64 L
+    if (!allow_smem(fuse_wide_kernel<N, L>, most)) return false;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fuse_wide_kernel<N, L>, kTileCells, sh) != cudaSuccess ||
         per_sm <= 0)
