@@ -11,10 +11,12 @@
 // largest over the points of the first iteration at which that point has converged, so
 //   1. inverse_first_kernel iterates each warp's points, in registers, until every one of them has
 //      converged once, keeps their state and posts that iteration (a maximum per camera);
-//   2. inverse_advance_kernel takes every point on to the posted maximum, writes the results
-//      and counts the points that have left convergence again.
+//   2. inverse_advance_kernel takes every point on to the posted maximum and counts the points
+//      that have left convergence again;
+//   3. inverse_result_kernel writes the results, unless a point of the call was found unconverged: a
+//      call that fails leaves its outputs as they were.
 // No such point: done, with one host synchronisation.  Otherwise the camera goes on one iteration at
-// a time (inverse_advance_kernel, target + 1).  Every point runs each iteration once either way.
+// a time (2 and 3, target + 1).  Every point runs each iteration once either way.
 #include <algorithm>
 #include <vector>
 
@@ -150,12 +152,17 @@ __device__ __forceinline__ void save_point(const InvState &st, long long s, cons
     st.k[s] = k;
 }
 
-// grid (points, cameras).  target[c]: the largest posted iteration; failed[c]: a point of the
-// camera has not converged within max_iter iterations.
+// Per camera: the largest posted iteration, whether a point has not converged within max_iter
+// iterations, the points that do not reproject within the bound at the posted iteration, and whether the
+// camera goes on.  open: set if there is any such point in the call.
+struct InvCounters {
+    int *target, *failed, *count, *open, *run;
+};
+
+// grid (points, cameras).
 __global__ void __launch_bounds__(kInvThreads, 12) inverse_first_kernel(
     const VsRpcCamera *__restrict__ cams, const double *__restrict__ col, const double *__restrict__ row,
-    const double *__restrict__ alt, long long n, long long stride, int max_iter, InvState st, int *__restrict__ target,
-    int *__restrict__ failed) {
+    const double *__restrict__ alt, long long n, long long stride, int max_iter, InvState st, InvCounters ct) {
     __shared__ RpcExact cam;
     const int c = blockIdx.y;
     load_exact(cams + c, cam);
@@ -178,21 +185,21 @@ __global__ void __launch_bounds__(kInvThreads, 12) inverse_first_kernel(
         done |= converged(p.o[0], p.o[1], p.cc, p.cr);
     }
     if (in) save_point(st, c * n + i, p, k);
-    if ((threadIdx.x & 31) == 0) atomicMax(target + c, k);
-    if (!done) atomicOr(failed + c, 1);
+    if ((threadIdx.x & 31) == 0) atomicMax(ct.target + c, k);
+    if (!done) ct.failed[c] = *ct.open = 1;
 }
 
-// Takes the points of the cameras with run[c] != 0 on to iteration target[c], writes their
-// results and counts those that do not reproject within the bound there.
-__global__ void __launch_bounds__(kInvThreads, 12) inverse_advance_kernel(
-    const VsRpcCamera *__restrict__ cams, const double *__restrict__ alt, long long n, long long stride, int normalized,
-    InvState st, const int *__restrict__ target, const int *__restrict__ run, double *__restrict__ lon_out,
-    double *__restrict__ lat_out, double *__restrict__ alt_out, int *__restrict__ count) {
+// Takes the points of the cameras that go on (at first: that have not failed) to iteration target[c] and
+// counts those that do not reproject within the bound there.
+__global__ void __launch_bounds__(kInvThreads, 12) inverse_advance_kernel(const VsRpcCamera *__restrict__ cams,
+                                                                          long long n, InvState st, InvCounters ct,
+                                                                          int first) {
     __shared__ RpcExact cam;
     const int c = blockIdx.y;
-    if (run && !run[c]) return;
+    chain_wait();
+    if (first ? ct.failed[c] : !ct.run[c]) return;
     load_exact(cams + c, cam);
-    const int to = target[c];
+    const int to = ct.target[c];
     const long long i = blockIdx.x * static_cast<long long>(kInvThreads) + threadIdx.x;
     bool unconverged = false;
     if (i < n) {
@@ -209,31 +216,46 @@ __global__ void __launch_bounds__(kInvThreads, 12) inverse_advance_kernel(
         for (int k = from; k < to; ++k) inverse_iteration(cam, k, p);
         if (from < to) save_point(st, s, p, to);
         unconverged = !converged(p.o[0], p.o[1], p.cc, p.cr);
-        if (normalized) {
-            lon_out[s] = p.lon;
-            lat_out[s] = p.lat;
-            if (alt_out) alt_out[s] = p.ca;
-        } else {
-            lon_out[s] = __dadd_rn(__dmul_rn(p.lon, cam.cam.lon_scale), cam.cam.lon_off);
-            lat_out[s] = __dadd_rn(__dmul_rn(p.lat, cam.cam.lat_scale), cam.cam.lat_off);
-            if (alt_out) alt_out[s] = alt[c * stride + i];
-        }
     }
     const unsigned b = __ballot_sync(0xffffffffu, unconverged);
-    if ((threadIdx.x & 31) == 0 && b) atomicAdd(count + c, __popc(b));
+    if ((threadIdx.x & 31) == 0 && b) {
+        atomicAdd(ct.count + c, __popc(b));
+        *ct.open = 1;
+    }
 }
 
-// Per camera: targets, failure flags, unconverged counts, and which cameras go on.
-struct InvCounters {
-    int *target, *failed, *count, *run;
-};
+// The results of a call whose points have all converged.
+__global__ void __launch_bounds__(256) inverse_result_kernel(const VsRpcCamera *__restrict__ cams,
+                                                             const double *__restrict__ alt, long long n,
+                                                             long long stride, int normalized, InvState st,
+                                                             InvCounters ct, double *__restrict__ lon_out,
+                                                             double *__restrict__ lat_out,
+                                                             double *__restrict__ alt_out) {
+    chain_wait();
+    const long long i = blockIdx.x * 256ll + threadIdx.x;
+    if (*ct.open || i >= n) return;
+    const int c = blockIdx.y;
+    const VsRpcCamera &cam = cams[c];
+    const long long s = c * n + i;
+    const double lon = st.f[0][s], lat = st.f[1][s];
+    if (normalized) {
+        lon_out[s] = lon;
+        lat_out[s] = lat;
+        if (alt_out) alt_out[s] = st.f[10][s];
+    } else {
+        lon_out[s] = __dadd_rn(__dmul_rn(lon, cam.lon_scale), cam.lon_off);
+        lat_out[s] = __dadd_rn(__dmul_rn(lat, cam.lat_scale), cam.lat_off);
+        if (alt_out) alt_out[s] = alt[c * stride + i];
+    }
+}
 
 InvState carve_inverse(Carver &cv, int n_cams, long long n, InvCounters &k) {
     InvState st;
     for (auto &f : st.f) f = cv.take<double>(static_cast<size_t>(n_cams) * n);
     st.k = cv.take<int>(static_cast<size_t>(n_cams) * n);
-    int *base = cv.take<int>(4 * static_cast<size_t>(n_cams));
-    k = {base, base + n_cams, base + 2 * static_cast<size_t>(n_cams), base + 3 * static_cast<size_t>(n_cams)};
+    const size_t m = n_cams;
+    int *base = cv.take<int>(4 * m + 1);
+    k = {base, base + m, base + 2 * m, base + 3 * m, base + 3 * m + 1};      // the first four: cleared together
     return st;
 }
 
@@ -279,16 +301,17 @@ extern "C" int vs_rpc_inverse_project(const VsRpcCamera *cams, int n_cams, const
         if (e != cudaSuccess) set_error("vs_rpc_inverse_project: %s", cudaGetErrorString(e));
         return e == cudaSuccess;
     };
-    if (!cuda_ok(cudaMemsetAsync(d.target, 0, 3 * bytes, st))) return VS_ERR_CUDA;
-    inverse_first_kernel<<<grid, kInvThreads, 0, st>>>(cams, col, row, alt, n, point_stride, max_iter, state, d.target,
-                                                       d.failed);
+    if (!cuda_ok(cudaMemsetAsync(d.target, 0, 3 * bytes + sizeof(int), st))) return VS_ERR_CUDA;
+    inverse_first_kernel<<<grid, kInvThreads, 0, st>>>(cams, col, row, alt, n, point_stride, max_iter, state, d);
     VS_LAUNCH_CHECK("inverse_first_kernel");
-    const int *run = nullptr;
+    const dim3 wide(static_cast<unsigned>(ceil_div(n, 256)), static_cast<unsigned>(n_cams));
     std::vector<int> go(n_cams);
-    for (;;) {
-        inverse_advance_kernel<<<grid, kInvThreads, 0, st>>>(cams, alt, n, point_stride, normalized, state, d.target, run,
-                                                             lon, lat, alt_out, d.count);
+    for (int first = 1;; first = 0) {
+        launch_chained(inverse_advance_kernel, grid, kInvThreads, 0, st, cams, n, state, d, first);
         VS_LAUNCH_CHECK("inverse_advance_kernel");
+        launch_chained(inverse_result_kernel, wide, 256, 0, st, cams, alt, n, point_stride, normalized, state, d, lon, lat,
+                       alt_out);
+        VS_LAUNCH_CHECK("inverse_result_kernel");
         if (!cuda_ok(cudaMemcpyAsync(h.data(), d.target, 3 * bytes, cudaMemcpyDeviceToHost, st)) ||
             !cuda_ok(cudaStreamSynchronize(st)))
             return VS_ERR_CUDA;
@@ -307,9 +330,8 @@ extern "C" int vs_rpc_inverse_project(const VsRpcCamera *cams, int n_cams, const
         for (int c = 0; c < n_cams; ++c) h[c] += go[c];
         if (!cuda_ok(cudaMemcpyAsync(d.target, h.data(), bytes, cudaMemcpyHostToDevice, st)) ||
             !cuda_ok(cudaMemcpyAsync(d.run, go.data(), bytes, cudaMemcpyHostToDevice, st)) ||
-            !cuda_ok(cudaMemsetAsync(d.count, 0, bytes, st)))
+            !cuda_ok(cudaMemsetAsync(d.count, 0, bytes + sizeof(int), st)))
             return VS_ERR_CUDA;
-        run = d.run;
     }
     if (iterations)
         for (int c = 0; c < n_cams; ++c) iterations[c] = h[c];
