@@ -138,8 +138,9 @@ int vs_set_l2_persisting(size_t bytes);
  * return_normalized=True); alt_out (nullable): the input altitudes, or the normalised ones.
  * iterations (nullable, HOST int32 [n_cams]): the iteration counts.  The reference loops
  * without a bound; here a camera exceeding max_iter fails with VS_ERR_DEGENERATE.  The
- * call synchronises `stream` once, and once more for every iteration that points which had
- * reached the bound leave it again at the common count. */
+ * call synchronises `stream` once, once more for every further 32 iterations, and for every
+ * iteration that points which had reached the bound leave it again at the common count.  A
+ * call that fails writes no output. */
 size_t vs_rpc_inverse_project_workspace_size(int n_cams, int64_t n);
 int vs_rpc_inverse_project(const VsRpcCamera *cams, int n_cams, const double *col, const double *row,
                            const double *alt, int64_t n, int64_t point_stride, int normalized, double *lon,

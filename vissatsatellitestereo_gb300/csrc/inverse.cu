@@ -16,7 +16,8 @@
 //   3. inverse_result_kernel writes the results, unless a point of the call was found unconverged: a
 //      call that fails leaves its outputs as they were.
 // No such point: done, with one host synchronisation.  Otherwise the camera goes on one iteration at
-// a time (2 and 3, target + 1).  Every point runs each iteration once either way.
+// a time (2 and 3, target + 1).  Every point runs each iteration once either way.  A launch does 32
+// iterations at most; cameras that need more go on from the saved state.
 #include <algorithm>
 #include <vector>
 
@@ -141,6 +142,18 @@ __device__ __forceinline__ void inverse_iteration(const RpcExact &s, int k, InvP
     frames(s, p.lat, p.lon, p.ca, 0.1, p.o);
 }
 
+__device__ __forceinline__ InvPoint load_point(const InvState &st, long long s) {
+    InvPoint p;
+    p.lon = st.f[0][s];
+    p.lat = st.f[1][s];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) p.o[q] = st.f[2 + q][s];
+    p.cc = st.f[8][s];
+    p.cr = st.f[9][s];
+    p.ca = st.f[10][s];
+    return p;
+}
+
 __device__ __forceinline__ void save_point(const InvState &st, long long s, const InvPoint &p, int k) {
     st.f[0][s] = p.lon;
     st.f[1][s] = p.lat;
@@ -152,74 +165,90 @@ __device__ __forceinline__ void save_point(const InvState &st, long long s, cons
     st.k[s] = k;
 }
 
-// Per camera: the largest posted iteration, whether a point has not converged within max_iter
-// iterations, the points that do not reproject within the bound at the posted iteration, and whether the
-// camera goes on.  open: set if there is any such point in the call.
+// Iterations of a point in one launch.  A launch's time is then bounded whatever the caller's
+// max_iter is (a point that never converges, a NaN, runs to max_iter); image points take 5 to 13.
+constexpr int kInvBurst = 32;
+constexpr int kUnfinished = 1, kBehind = 2;      // flags of InvCounters::state
+constexpr int kAdvance = 1, kResume = 2;         // values of InvCounters::run
+
+// Per camera: the largest posted iteration; whether a point has not converged yet (kUnfinished) or has
+// not come to the posted iteration (kBehind); the points that do not reproject within the bound at the
+// posted iteration; and whether the camera goes on.  open: set if there is any such point in the call.
 struct InvCounters {
-    int *target, *failed, *count, *open, *run;
+    int *target, *state, *count, *open, *run;
 };
 
-// grid (points, cameras).
+// Iterations up to `limit` of a warp's points (RESUME: of cameras with unfinished points, from the saved
+// state), until every one of them has converged once.  The points of a warp share their count, which is
+// saved complemented for a point that has not converged yet.  grid (points, cameras).
+template <bool RESUME>
 __global__ void __launch_bounds__(kInvThreads, 12) inverse_first_kernel(
     const VsRpcCamera *__restrict__ cams, const double *__restrict__ col, const double *__restrict__ row,
-    const double *__restrict__ alt, long long n, long long stride, int max_iter, InvState st, InvCounters ct) {
+    const double *__restrict__ alt, long long n, long long stride, int limit, InvState st, InvCounters ct) {
     __shared__ RpcExact cam;
     const int c = blockIdx.y;
+    if (RESUME && ct.run[c] != kResume) return;
     load_exact(cams + c, cam);
     const long long i = blockIdx.x * static_cast<long long>(kInvThreads) + threadIdx.x;
     const bool in = i < n;
     InvPoint p;
-    {
+    bool done;
+    int k = 0;
+    if (RESUME) {
+        const int saved = in ? st.k[c * n + i] : 0;
+        p = load_point(st, c * n + (in ? i : n - 1));           // idle lanes: any point, done
+        done = saved >= 0;
+        k = __shfl_sync(0xffffffffu, done ? saved : ~saved, 0);
+    } else {
         const long long g = c * stride + (in ? i : n - 1);      // idle lanes follow the last point
         p.cc = __ddiv_rn(__dsub_rn(col[g], cam.cam.col_off), cam.cam.col_scale);
         p.cr = __ddiv_rn(__dsub_rn(row[g], cam.cam.row_off), cam.cam.row_scale);
         p.ca = __ddiv_rn(__dsub_rn(alt[g], cam.cam.alt_off), cam.cam.alt_scale);
+        p.lon = p.lat = -1.0;
+        frames(cam, -1.0, -1.0, p.ca, 2.0, p.o);
+        done = converged(p.o[0], p.o[1], p.cc, p.cr);
     }
-    p.lon = p.lat = -1.0;
-    frames(cam, -1.0, -1.0, p.ca, 2.0, p.o);
-    bool done = converged(p.o[0], p.o[1], p.cc, p.cr);
-    int k = 0;
-    while (k < max_iter && !__all_sync(0xffffffffu, done)) {
+    while (k < limit && !__all_sync(0xffffffffu, done)) {
         inverse_iteration(cam, k, p);
         ++k;
         done |= converged(p.o[0], p.o[1], p.cc, p.cr);
     }
-    if (in) save_point(st, c * n + i, p, k);
+    if (in) save_point(st, c * n + i, p, done ? k : ~k);
     if ((threadIdx.x & 31) == 0) atomicMax(ct.target + c, k);
-    if (!done) ct.failed[c] = *ct.open = 1;
+    if (!done) {
+        atomicOr(ct.state + c, kUnfinished);
+        *ct.open = 1;
+    }
 }
 
-// Takes the points of the cameras that go on (at first: that have not failed) to iteration target[c] and
-// counts those that do not reproject within the bound there.
+// Takes the points of the cameras that go on (at first: all) and have no unfinished point towards
+// iteration target[c], and counts those that do not reproject within the bound there.
 __global__ void __launch_bounds__(kInvThreads, 12) inverse_advance_kernel(const VsRpcCamera *__restrict__ cams,
                                                                           long long n, InvState st, InvCounters ct,
                                                                           int first) {
     __shared__ RpcExact cam;
     const int c = blockIdx.y;
     chain_wait();
-    if (first ? ct.failed[c] : !ct.run[c]) return;
+    // the same for a whole block: other blocks may set kBehind meanwhile, never kUnfinished
+    if ((ct.state[c] & kUnfinished) || !(first || ct.run[c])) return;
     load_exact(cams + c, cam);
     const int to = ct.target[c];
     const long long i = blockIdx.x * static_cast<long long>(kInvThreads) + threadIdx.x;
-    bool unconverged = false;
+    bool unconverged = false, behind = false;
     if (i < n) {
         const long long s = c * n + i;
-        InvPoint p;
-        p.lon = st.f[0][s];
-        p.lat = st.f[1][s];
-#pragma unroll
-        for (int q = 0; q < 6; ++q) p.o[q] = st.f[2 + q][s];
-        p.cc = st.f[8][s];
-        p.cr = st.f[9][s];
-        p.ca = st.f[10][s];
-        const int from = st.k[s];
-        for (int k = from; k < to; ++k) inverse_iteration(cam, k, p);
-        if (from < to) save_point(st, s, p, to);
-        unconverged = !converged(p.o[0], p.o[1], p.cc, p.cr);
+        InvPoint p = load_point(st, s);
+        const int from = st.k[s], end = min(to, from + kInvBurst);
+        for (int k = from; k < end; ++k) inverse_iteration(cam, k, p);
+        if (from < end) save_point(st, s, p, end);
+        behind = end < to;
+        unconverged = !behind && !converged(p.o[0], p.o[1], p.cc, p.cr);
     }
     const unsigned b = __ballot_sync(0xffffffffu, unconverged);
-    if ((threadIdx.x & 31) == 0 && b) {
-        atomicAdd(ct.count + c, __popc(b));
+    const bool any_behind = __any_sync(0xffffffffu, behind);
+    if ((threadIdx.x & 31) == 0 && (b || any_behind)) {
+        if (b) atomicAdd(ct.count + c, __popc(b));
+        if (any_behind) atomicOr(ct.state + c, kBehind);
         *ct.open = 1;
     }
 }
@@ -295,43 +324,61 @@ extern "C" int vs_rpc_inverse_project(const VsRpcCamera *cams, int n_cams, const
     InvCounters d;
     const InvState state = carve_inverse(cv, n_cams, n, d);
     const dim3 grid(static_cast<unsigned>(ceil_div(n, kInvThreads)), static_cast<unsigned>(n_cams));
-    std::vector<int> h(3 * static_cast<size_t>(n_cams));      // targets, failures, counts
+    std::vector<int> h(3 * static_cast<size_t>(n_cams));      // targets, flags, counts
     const size_t bytes = sizeof(int) * n_cams;
     auto cuda_ok = [](cudaError_t e) {
         if (e != cudaSuccess) set_error("vs_rpc_inverse_project: %s", cudaGetErrorString(e));
         return e == cudaSuccess;
     };
+    int limit = std::min(max_iter, kInvBurst);
     if (!cuda_ok(cudaMemsetAsync(d.target, 0, 3 * bytes + sizeof(int), st))) return VS_ERR_CUDA;
-    inverse_first_kernel<<<grid, kInvThreads, 0, st>>>(cams, col, row, alt, n, point_stride, max_iter, state, d);
+    inverse_first_kernel<false><<<grid, kInvThreads, 0, st>>>(cams, col, row, alt, n, point_stride, limit, state, d);
     VS_LAUNCH_CHECK("inverse_first_kernel");
     const dim3 wide(static_cast<unsigned>(ceil_div(n, 256)), static_cast<unsigned>(n_cams));
-    std::vector<int> go(n_cams);
+    std::vector<int> run(n_cams);
+    std::vector<char> failed(n_cams, 0);
+    int worst = n_cams;                       // the first camera that has failed
     for (int first = 1;; first = 0) {
         launch_chained(inverse_advance_kernel, grid, kInvThreads, 0, st, cams, n, state, d, first);
         VS_LAUNCH_CHECK("inverse_advance_kernel");
-        launch_chained(inverse_result_kernel, wide, 256, 0, st, cams, alt, n, point_stride, normalized, state, d, lon, lat,
-                       alt_out);
-        VS_LAUNCH_CHECK("inverse_result_kernel");
+        if (worst == n_cams) {
+            launch_chained(inverse_result_kernel, wide, 256, 0, st, cams, alt, n, point_stride, normalized, state, d, lon,
+                           lat, alt_out);
+            VS_LAUNCH_CHECK("inverse_result_kernel");
+        }
         if (!cuda_ok(cudaMemcpyAsync(h.data(), d.target, 3 * bytes, cudaMemcpyDeviceToHost, st)) ||
             !cuda_ok(cudaStreamSynchronize(st)))
             return VS_ERR_CUDA;
-        const int *target = h.data(), *failed = target + n_cams, *count = failed + n_cams;
-        bool any = false;
+        const int *target = h.data(), *flags = target + n_cams, *count = flags + n_cams;
+        bool resume = false, any = false;
+        const int reached = limit;
         for (int c = 0; c < n_cams; ++c) {
-            go[c] = count[c] > 0;
-            any |= go[c] != 0;
-            if (failed[c] || (go[c] && target[c] >= max_iter)) {
-                set_error("vs_rpc_inverse_project: camera %d did not converge in %d iterations", c, max_iter);
-                return VS_ERR_DEGENERATE;
+            const bool unfinished = flags[c] & kUnfinished, behind = flags[c] & kBehind;
+            const bool open = unfinished || behind || count[c] > 0;
+            if (open && !behind && (unfinished ? reached : target[c]) >= max_iter) {
+                failed[c] = 1;
+                worst = std::min(worst, c);
             }
+            run[c] = !open || failed[c] ? 0 : (unfinished ? kResume : kAdvance);
+            any |= run[c] != 0;
+            resume |= run[c] == kResume;
+            // points that left the bound again at the common iteration: their camera goes on by one
+            if (run[c] == kAdvance && !behind) ++h[c];
         }
         if (!any) break;
-        // points that left the bound again at the common iteration: their cameras go on by one
-        for (int c = 0; c < n_cams; ++c) h[c] += go[c];
         if (!cuda_ok(cudaMemcpyAsync(d.target, h.data(), bytes, cudaMemcpyHostToDevice, st)) ||
-            !cuda_ok(cudaMemcpyAsync(d.run, go.data(), bytes, cudaMemcpyHostToDevice, st)) ||
-            !cuda_ok(cudaMemsetAsync(d.count, 0, bytes + sizeof(int), st)))
+            !cuda_ok(cudaMemcpyAsync(d.run, run.data(), bytes, cudaMemcpyHostToDevice, st)) ||
+            !cuda_ok(cudaMemsetAsync(d.state, 0, 2 * bytes + sizeof(int), st)))
             return VS_ERR_CUDA;
+        if (resume) {
+            limit = max_iter - limit > kInvBurst ? limit + kInvBurst : max_iter;
+            inverse_first_kernel<true><<<grid, kInvThreads, 0, st>>>(cams, col, row, alt, n, point_stride, limit, state, d);
+            VS_LAUNCH_CHECK("inverse_first_kernel");
+        }
+    }
+    if (worst < n_cams) {
+        set_error("vs_rpc_inverse_project: camera %d did not converge in %d iterations", worst, max_iter);
+        return VS_ERR_DEGENERATE;
     }
     if (iterations)
         for (int c = 0; c < n_cams; ++c) iterations[c] = h[c];
