@@ -601,6 +601,11 @@ __device__ __forceinline__ float as_f32<double>(double v) { return f64_to_f32(v)
 // 2000 x 2000 float32: 35.5 us with nine loads and a 64-bit division per cell, 13 us;
 // 1025 x 1025 FP64: 20 us, 9 us.
 constexpr int kBlurRows = 8, kBlurCols = 30;
+// Percent of the warps' rows and columns that lie in the image below which a thread per cell is faster: narrow
+// images and stacks of tiny ones.  Float32 / FP64 input, warps against cells: 1,000,000 x 1 57 / 80 us, 10 / 10 us;
+// 500,000 x 3 38 / 50, 14 / 24; 300,000 x 5 (17 %) 24 / 31, 14 / 24; 100,000 images of 3 x 3 39 / 58, 19 / 19;
+// the other way 300,000 x 6 (20 %) 24 / 31, 20 / 32; 200,000 x 7 16 / 21, 16 / 26; 2 x 500,000 (25 %) 10 / 11, 10 / 16.
+constexpr int kBlurFill = 18;
 
 // I: the index type, 32 bits unless a side or the number of warps needs more (a 64-bit division
 // costs as much as a row).
@@ -654,9 +659,40 @@ __global__ void __launch_bounds__(256) median_blur3x3_kernel(const T *__restrict
     }
 }
 
+// One cell per thread: nine loads and two divisions, but no idle lanes on images of a few columns or rows.
+template <typename T>
+__global__ void __launch_bounds__(256) median_blur3x3_cell_kernel(const T *__restrict__ in, float *__restrict__ out,
+                                                                  long long H, long long W, long long total) {
+    chain_wait();
+    for (long long i = blockIdx.x * 256ll + threadIdx.x; i < total; i += gridDim.x * 256ll) {
+        const long long plane = i / (H * W), rc = i - plane * (H * W), r = rc / W, c = rc - r * W;
+        const T *img = in + plane * (H * W);
+        const long long rows[3] = {max(r - 1, 0ll), r, min(r + 1, H - 1)}, cols[3] = {max(c - 1, 0ll), c, min(c + 1, W - 1)};
+        if (H == 1 || W == 1) {
+            float p[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) p[a] = as_f32(__ldg(img + (H == 1 ? cols[a] : rows[a])));
+            out[i] = cv_median3_line(p[0], p[1], p[2]);
+            continue;
+        }
+        float p[9];
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int b = 0; b < 3; ++b) p[3 * a + b] = as_f32(__ldg(img + rows[a] * W + cols[b]));
+        out[i] = cv_median9(cv_vector_column(c, W), p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], p[8]);
+    }
+}
+
 template <typename T>
 int launch_blur(const T *in, float *out, long long h, long long w, long long n_img, cudaStream_t st) {
     const long long strips = ceil_div(h, kBlurRows), groups = ceil_div(w, kBlurCols), warps = n_img * strips * groups;
+    const long long cells = n_img * h * w;
+    if (100 * cells < kBlurFill * kBlurRows * kBlurCols * warps) {
+        launch_chained(median_blur3x3_cell_kernel<T>, static_cast<unsigned>(std::min<long long>(ceil_div(cells, 256), sm_count() * 16LL)),
+                       256, 0, st, in, out, h, w, cells);
+        return check_launch("median_blur3x3_cell_kernel");
+    }
     const unsigned blocks = static_cast<unsigned>(ceil_div(warps, 8));
     const long long small = (1LL << 31) - 64;
     if (h < small && w < small && warps < small)
