@@ -1,10 +1,10 @@
-"""Images of a few columns or rows, alone and in stacks, on both sides of the rule that gives them a thread per
-cell, against the oracle (bit-exact)."""
+"""Images and grids of a few columns or rows, alone and in stacks, on both sides of the rules that give them a
+thread per cell or long tiles, against the oracle (bit-exact)."""
 import numpy as np
 import pytest
 
 from conftest import same_bits
-from oracle import blur
+from oracle import blur, raster
 
 pytestmark = pytest.mark.gpu
 
@@ -22,3 +22,15 @@ def test_blur_of_narrow_images(n, H, W):
         got = median_blur3x3(a)
         for b in range(n):
             assert same_bits(got[b], blur.median_blur3x3(a[b].astype(np.float32))), b
+
+
+@pytest.mark.parametrize('xsize,ysize', [(1, 700), (2, 1025), (4, 256), (5, 257), (8, 511), (9, 300), (700, 1), (1025, 2),
+                                         (256, 4), (257, 5), (511, 8), (300, 9)])
+def test_grid_of_few_columns_or_rows(xsize, ysize):
+    from vissatsatellitestereo_gb300.proj_to_grid import proj_to_grid
+    rng = np.random.default_rng(xsize * 100 + ysize)
+    n = int(0.7 * xsize * ysize) + 1                     # sparse: holes with 0 to 8 valid neighbours
+    args = (354052.25, 6182702.5, 0.5, 0.5, xsize, ysize)
+    p = np.stack([354052.25 + rng.uniform(-0.5, xsize * 0.5 + 0.5, n), 6182702.5 - rng.uniform(-0.5, ysize * 0.5 + 0.5, n),
+                  rng.choice([0.0, -0.0, 3.25, -7.5, np.nan, 12.125], n)], axis=1)
+    assert same_bits(proj_to_grid(p, *args), raster.proj_to_grid(p, *args))

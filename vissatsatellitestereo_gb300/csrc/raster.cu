@@ -465,51 +465,53 @@ dim3 tile_grid(long long tiles_x, long long tiles_y) {
 __device__ __forceinline__ int tile_row() { return static_cast<int>(blockIdx.z * gridDim.y + blockIdx.y); }
 
 // The FP64 grid from the keys: nanmax values and the non-propagating hole fill
-// (lib/proj_to_grid.py:64-79) in one pass over 32 x 32 tiles.  The keys and a 1-cell halo are
+// (lib/proj_to_grid.py:64-79) in one pass over tiles of 1024 cells.  The keys and a 1-cell halo are
 // loaded at once (six loads in flight per thread, one trip to L2) and staged; empty cells go
 // to a list that consecutive threads fill, so that a warp with one hole does not run the
 // median for 32 cells.  1025 x 1025 cells: 32 us as a decode and a per-cell fill, 11 us.
-constexpr int kGridTile = 32, kGridRaw = kGridTile + 2, kGridThreads = 256;
+constexpr int kGridThreads = 256;
 
+template <int TW, int TH>
 __global__ void __launch_bounds__(kGridThreads) grid_f64_kernel(const unsigned long long *__restrict__ keys,
                                                                 const unsigned long long *__restrict__ first,
                                                                 const double *__restrict__ pts,
                                                                 double *__restrict__ out, int H, int W) {
-    __shared__ unsigned long long raw[kGridRaw * kGridRaw];
-    __shared__ unsigned short holes[kGridTile * kGridTile];
+    constexpr int kW = TW + 2, kRaw = kW * (TH + 2);
+    __shared__ unsigned long long raw[kRaw];
+    __shared__ unsigned short holes[TW * TH];
     __shared__ int n_holes;
     chain_wait();
-    constexpr int kLoads = (kGridRaw * kGridRaw + kGridThreads - 1) / kGridThreads;
-    if (tile_row() > (H - 1) / kGridTile) return;
-    const int tid = threadIdx.x, r0 = tile_row() * kGridTile, c0 = blockIdx.x * kGridTile;
+    constexpr int kLoads = (kRaw + kGridThreads - 1) / kGridThreads;
+    if (tile_row() > (H - 1) / TH) return;
+    const int tid = threadIdx.x, r0 = tile_row() * TH, c0 = blockIdx.x * TW;
     if (tid == 0) n_holes = 0;
     unsigned long long k[kLoads];
 #pragma unroll
     for (int q = 0; q < kLoads; ++q) {
-        const int i = q * kGridThreads + tid, ly = i / kGridRaw, lx = i - ly * kGridRaw;
+        const int i = q * kGridThreads + tid, ly = i / kW, lx = i - ly * kW;
         const int r = r0 + ly - 1, c = c0 + lx - 1;
         k[q] = kEmptyKey;
-        if (i < kGridRaw * kGridRaw && static_cast<unsigned>(r) < static_cast<unsigned>(H) &&
+        if (i < kRaw && static_cast<unsigned>(r) < static_cast<unsigned>(H) &&
             static_cast<unsigned>(c) < static_cast<unsigned>(W))
             k[q] = keys[static_cast<long long>(r) * W + c];
     }
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < kLoads; ++q) {
-        const int i = q * kGridThreads + tid, ly = i / kGridRaw, lx = i - ly * kGridRaw;
-        if (i >= kGridRaw * kGridRaw) break;
+        const int i = q * kGridThreads + tid, ly = i / kW, lx = i - ly * kW;
+        if (i >= kRaw) break;
         const int r = r0 + ly - 1, c = c0 + lx - 1;
         const long long cell = static_cast<long long>(r) * W + c;
         k[q] = cell_key(k[q], cell, first, pts);
         raw[i] = k[q];
-        if (ly >= 1 && ly <= kGridTile && lx >= 1 && lx <= kGridTile && r < H && c < W) {
+        if (ly >= 1 && ly <= TH && lx >= 1 && lx <= TW && r < H && c < W) {
             if (k[q] != kEmptyKey) out[cell] = double_from_key(k[q]);
             else holes[atomicAdd(&n_holes, 1)] = static_cast<unsigned short>(i);
         }
     }
     __syncthreads();
     for (int h = tid; h < n_holes; h += kGridThreads) {
-        const int i = holes[h], ly = i / kGridRaw, lx = i - ly * kGridRaw;
+        const int i = holes[h], ly = i / kW, lx = i - ly * kW;
         unsigned long long s[8];
         int m = 0;
         bool any = false;
@@ -518,7 +520,7 @@ __global__ void __launch_bounds__(kGridThreads) grid_f64_kernel(const unsigned l
 #pragma unroll
             for (int dk = -1; dk <= 1; ++dk)
                 if (dj != 0 || dk != 0) {
-                    s[m] = raw[i + dj * kGridRaw + dk];
+                    s[m] = raw[i + dj * kW + dk];
                     any |= s[m++] != kEmptyKey;
                 }
         out[static_cast<long long>(r0 + ly - 1) * W + (c0 + lx - 1)] =
@@ -1853,6 +1855,14 @@ static bool grid_ok(int64_t xsize, int64_t ysize) {
     return xsize > 0 && ysize > 0 && xsize < (1LL << 31) && ysize < (1LL << 31);
 }
 
+template <int TW, int TH>
+static int launch_grid_f64(const vs::RasterWs &w, const double *points, double *dsm, int64_t xsize, int64_t ysize,
+                           cudaStream_t st) {
+    launch_chained(grid_f64_kernel<TW, TH>, tile_grid(ceil_div(xsize, TW), ceil_div(ysize, TH)), kGridThreads, 0, st,
+                   w.keys[0], w.first, points, dsm, static_cast<int>(ysize), static_cast<int>(xsize));
+    return check_launch("grid_f64_kernel");
+}
+
 extern "C" int vs_proj_to_grid(const double *points, int64_t n, double xoff, double yoff,
                                double xresolution, double yresolution, int64_t xsize, int64_t ysize,
                                double *dsm, void *workspace, size_t workspace_bytes, void *stream) {
@@ -1871,11 +1881,12 @@ extern "C" int vs_proj_to_grid(const double *points, int64_t n, double xoff, dou
     if (s == VS_OK) s = make_tables(xoff, yoff, xresolution, yresolution, xsize, ysize, w, tb, st);
     if (s == VS_OK) s = bin_launch(points, nullptr, 0, n, n, tb, w.keys[0], w.first, st);
     if (s != VS_OK) return s;
-    const dim3 grid = tile_grid(ceil_div(xsize, kGridTile), ceil_div(ysize, kGridTile));
-    launch_chained(grid_f64_kernel, grid, kGridThreads, 0, st, w.keys[0], w.first, points, dsm, static_cast<int>(ysize),
-                   static_cast<int>(xsize));
-    VS_LAUNCH_CHECK("grid_f64_kernel");
-    return VS_OK;
+    // grids of a few columns or rows take long tiles, of which they fill more.  The whole call with 32 x 32 and with
+    // long tiles: 1 x 1,000,000 cells 167 and 103 us, 4 x 500,000 115 and 78 us, 8 x 300,000 91 and 74 us, 16 x 100,000
+    // 48 and 47 us, 31 x 30,000 27 and 29 us; 1,000,000 x 1 150 and 95 us, 300,000 x 8 81 and 70 us
+    if (xsize <= 8) return launch_grid_f64<4, 256>(w, points, dsm, xsize, ysize, st);
+    if (ysize <= 8) return launch_grid_f64<256, 4>(w, points, dsm, xsize, ysize, st);
+    return launch_grid_f64<32, 32>(w, points, dsm, xsize, ysize, st);
 }
 
 extern "C" size_t vs_dsm_from_points_workspace_size(int n_views, int64_t xsize, int64_t ysize) {
