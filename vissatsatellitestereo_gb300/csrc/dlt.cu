@@ -1285,9 +1285,13 @@ extern "C" int vs_rpc_project(const VsRpcCamera *cams, int n_cams, const double 
     VS_REQUIRE(cams && lat && lon && alt && col && row, "vs_rpc_project: null pointer");
     // The exact form is bound by each SM's FP64 pipe, so few points are spread over all SMs:
     // 1999 points in blocks of 256 took 26 us on 8 SMs, in blocks of 32 on 63 SMs 14 us.
+    // The fast form is bound by each block's preparation of its camera, which the threads share: 100 points 6.5 us
+    // in a block of 256, 8.3 in blocks of 32; 2000 points 6.9 and 8.3, 10,000 8.1 and 8.4.  Above 128 points
+    // per SM blocks of 64 spread them better: 20,000 points 8.3 us with 256, 7.4 with 64.
     const int sms = sm_count();
     const long long points = n * n_cams;
-    const int threads = points >= 512LL * sms ? 256 : (points >= 128LL * sms ? 64 : 32);
+    const int few = mode == VS_PROJ_EXACT ? 32 : 256;
+    const int threads = points >= 512LL * sms ? 256 : (points >= 128LL * sms ? 64 : few);
     const long long want = ceil_div(n, threads);
     const long long cap = std::max(1LL, sms * (2048LL / threads) / n_cams + 1);
     // even shares: every thread of a full grid takes as many points as any other, +-1
