@@ -514,7 +514,10 @@ bool launch_fuse_wide_n(const float *dsm, int layout, int V, long long cells, fl
     return true;
 }
 
-// The fewest lanes that hold the views, each with the smallest of three networks that takes its share.
+// The fewest lanes that hold the views, each with the smallest of three networks that takes its share.  40 million
+// values in all, networks of 44, 52 and 64: 72 views (2 lanes, 36 values each) 187, 202 and 232 us, 97 views (49) 151 us with 52,
+// 175 with 64; 140 views (4 lanes, 35) 255, 288 and 320 us, 177 views (45) 219 and 247 us; 300 views (8 lanes, 38)
+// 335, 346 and 383 us, 353 views (45) 299 and 327 us.  Each further network is three more kernels to compile.
 template <int L>
 bool launch_fuse_wide_l(const float *dsm, int layout, int V, long long cells, float *out, bool aligned,
                         cudaStream_t st) {
