@@ -100,16 +100,6 @@ __device__ __forceinline__ double rare_ddiv(double a, double b) {
     asm volatile("div.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
     return r;
 }
-__device__ __forceinline__ float rare_d2f(double a) {
-    float r;
-    asm volatile("cvt.rn.f32.f64 %0, %1;" : "=f"(r) : "d"(a));
-    return r;
-}
-__device__ __forceinline__ double rare_f2d(float a) {
-    double r;
-    asm volatile("cvt.f64.f32 %0, %1;" : "=d"(r) : "f"(a));
-    return r;
-}
 
 // ---- double-float arithmetic ---------------------------------------------------------
 // A value hi + lo with |lo| <= ulp(hi)/2 carried in two floats (about 48 significant
@@ -132,14 +122,6 @@ __device__ __forceinline__ df fast_two_sum(float a, float b) {  // |a| >= |b|
 __device__ __forceinline__ df two_prod(float a, float b) {
     float p = a * b;
     return {p, __fmaf_rn(a, b, -p)};
-}
-__device__ __forceinline__ df df_add(df a, df b) {
-    df s = two_sum(a.hi, b.hi);
-    df t = two_sum(a.lo, b.lo);
-    s.lo += t.hi;
-    s = fast_two_sum(s.hi, s.lo);
-    s.lo += t.lo;
-    return fast_two_sum(s.hi, s.lo);
 }
 __device__ __forceinline__ df df_add_f(df a, float b) {
     df s = two_sum(a.hi, b);
@@ -309,10 +291,6 @@ __device__ __forceinline__ unsigned long long key_from_double(double v) {
 __device__ __forceinline__ double double_from_key(unsigned long long k) {
     unsigned long long b = (k >> 63) ? (k & 0x7fffffffffffffffull) : ~k;
     return __longlong_as_double(static_cast<long long>(b));
-}
-__device__ __forceinline__ unsigned key_from_float(float v) {
-    unsigned b = __float_as_uint(v);
-    return (b >> 31) ? ~b : (b | 0x80000000u);
 }
 __device__ __forceinline__ float float_from_key(unsigned k) {
     unsigned b = (k >> 31) ? (k & 0x7fffffffu) : ~k;

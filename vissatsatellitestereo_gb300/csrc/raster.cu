@@ -230,9 +230,7 @@ __global__ void __launch_bounds__(256) bin_max_kernel(const double *__restrict__
 struct FastAxis {
     long long off_bits, tmax;
     const long long *thr;
-    unsigned top12;
     int shift, nm1;
-    float scale, err_abs, err_rel;
     unsigned mul, fmask, fsure;
     int fbits;
 };
@@ -242,12 +240,8 @@ FastAxis fast_axis_of(const Axis &ax) {
     memcpy(&fa.off_bits, &ax.off, sizeof(long long));
     fa.tmax = ax.tmax;
     fa.thr = ax.thr;
-    fa.top12 = ax.top12;
     fa.shift = ax.shift;
     fa.nm1 = static_cast<int>(ax.n - 1);
-    fa.scale = ax.scale;
-    fa.err_abs = ax.err_abs;
-    fa.err_rel = ax.err_rel;
     fa.mul = ax.mul;
     fa.fmask = ax.fmask;
     fa.fsure = ax.fsure;
@@ -266,21 +260,6 @@ __device__ __forceinline__ void axis_estimate(const FastAxis &a, unsigned u, int
     sure = ((hi & a.fmask) - 4u) < a.fsure;
 }
 
-template <bool FLIP>   // FLIP: d = off - v (rows of a positive origin, columns of a negative one)
-__device__ __forceinline__ bool axis_fast(const FastAxis &a, long long bv, int &r, long long &d, bool &sure) {
-    const unsigned hi = static_cast<unsigned>(static_cast<unsigned long long>(bv) >> 32);
-    d = FLIP ? (a.off_bits - bv) : (bv - a.off_bits);
-    const bool ok = ((hi >> 20) == a.top12) & (d >= 0) & (d < a.tmax);
-    const unsigned u = static_cast<unsigned>(static_cast<unsigned long long>(d) >> a.shift);
-    const float q = __fmul_rn(__uint2float_rn(u), a.scale);
-    const float big = __fadd_rn(q, 12582912.0f);
-    const float fr = __fsub_rn(q, __fsub_rn(big, 12582912.0f));
-    const int rn = static_cast<int>(static_cast<unsigned>(__float_as_int(big)) - 0x4b400000u);
-    r = min(max(rn - (fr < 0.0f ? 1 : 0), 0), a.nm1);
-    sure = fabsf(fr) > __fmaf_rn(a.err_rel, q, a.err_abs);
-    return ok;
-}
-
 __device__ __noinline__ int axis_correct(const long long *thr, int r, long long d) {
     for (int it = 0; it < 8 && __ldg(thr + r) > d; ++it) --r;
     for (int it = 0; it < 8 && __ldg(thr + r + 1) <= d; ++it) ++r;
@@ -292,7 +271,7 @@ __device__ __noinline__ int axis_correct(const long long *thr, int r, long long 
 // coordinate off the grid, including those of the other sign or another binade (their
 // wrapped difference is at least the origin's bit pattern, far above tmax, because the
 // grid +-2 cells lies inside the origin's binade) and NaN/inf.
-template <bool FLIP>
+template <bool FLIP>   // FLIP: d = off - v (rows of a positive origin, columns of a negative one)
 __device__ __forceinline__ bool axis_contained(const FastAxis &a, long long bv, int &r, long long &d, bool &sure) {
     const unsigned long long ud = FLIP ? static_cast<unsigned long long>(a.off_bits) - static_cast<unsigned long long>(bv)
                                        : static_cast<unsigned long long>(bv) - static_cast<unsigned long long>(a.off_bits);
