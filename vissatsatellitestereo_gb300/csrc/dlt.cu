@@ -465,8 +465,8 @@ __global__ void __launch_bounds__(256) project_view_kernel(const VsRpcCamera *__
 // vectors (component i = l mod 4 of row b = l / 4) and row l of the factor, and the divisions,
 // which were one after the other in one lane, run side by side; those by a pivot or a scale, which
 // repeat each iteration, use its reciprocal (div_known: 4 operations, the same bits).  Every
-// element sees the operations of the serial form in its order.  One view: 175 us, 96 us, of which about
-// 50 us are FP64 latency (59 cycles an operation, 600 a division or square root).
+// element sees the operations of the serial form in its order.  One view: 175 us, 95 us, most of it
+// FP64 latency (59 cycles an operation, 600 a division or square root).
 
 // A divisor and whether its quotients may take the reciprocal form.
 struct LaneDivisor {

@@ -30,9 +30,9 @@ namespace {
 // The kernels are bound by the FP64 pipe (19 sums and a share of the quotients per polynomial),
 // which every SM has its own of: small blocks spread the points evenly over the SMs (90,001
 // points: blocks of 64 hold every SM to within 8% of the mean load, blocks of 256 to 30%), and
-// registers for 12 of them on an SM (90,001 points, 7 iterations: 511 us; for 8 or fewer
-// 600 us, for 16 520 us).  The whole call took 1088 us with the products on the FP64 pipe and a
-// host synchronisation per iteration, 485 us now.
+// registers for 12 of them on an SM (whole calls, for 8, 10, 12 and 16: 90,001 points 560, 462, 471 and 477 us; four
+// cameras of 30,000 points 681, 687, 664 and 639 us, of 300,000 points 5.73, 5.37, 5.40 and 5.62 ms).
+// 90,001 points with the products on the FP64 pipe and a host synchronisation per iteration took 1111 us.
 constexpr int kInvThreads = 64;
 constexpr int kStateFields = 11;   // lon lat x0 y0 x1 y1 x2 y2 c_col c_row c_alt
 
